@@ -1,0 +1,59 @@
+"""The prompt pass of the plain decoder (all prompt positions of a chunk in one read of the weights) against the CPU
+restatement of the one-token step: tokens, the last step's logits and the residual stream, bit for bit, at the edges of
+its tiles (8 / 16 / 32 tokens, 32 / 64 rows, blocks that do not fill 32 lanes, the chunk of 512 positions)."""
+import numpy as np
+import pytest
+
+import oracle_lib as ol
+from test_y_dense_decoder import _oracle_for
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def wd():
+    import warpdecode_b200 as w
+    w.lib()
+    return w
+
+
+#            hidden heads kv  hd   ffn  layers prompt gen  style
+CASES = [(256, 4, 2, 64, 512, 2, 2, 3, "q4"),
+         (256, 4, 2, 64, 512, 2, 9, 1, "q4"),
+         (512, 3, 1, 96, 928, 2, 17, 4, "q4"),           # 29 blocks per ffn row: lanes without a block
+         (256, 2, 1, 128, 1056, 2, 33, 0, "q4"),         # 33 blocks: one lane with two; nothing generated
+         (1024, 8, 8, 32, 2816, 1, 40, 5, "file"),       # Q8_0 matrices, biases, head norms
+         (2048, 32, 8, 64, 8192, 1, 70, 2, "q4"),        # the benchmark width: the wide row tile
+         (256, 4, 1, 64, 256, 1, 530, 3, "q4")]          # two chunks
+
+
+@pytest.mark.parametrize("H,nh,nkv,hd,F,L,P,G,style", CASES)
+def test_prompt_pass_equals_the_one_token_steps(wd, oracle, H, nh, nkv, hd, F, L, P, G, style):
+    V = 1000
+    cfg = dict(hidden=H, n_heads=nh, n_kv_heads=nkv, head_dim=hd, ffn=F, vocab=V, n_layers=L, max_ctx=P + G + 1, rms_eps=1e-5)
+    dec = wd.DenseDecoder(H, nh, nkv, hd, F, V, L, P + G + 1, 1e-5, 500000.0)
+    dec.synth(7, 0.05)
+    rng = np.random.Generator(np.random.PCG64(P))
+    for l in range(L):
+        for which in (wd.DT_ATTN_NORM, wd.DT_FFN_NORM):
+            dec.set_tensor(l, which, (1.0 + 0.1 * rng.standard_normal(H)).astype(np.float32))
+        if style == "file":
+            from warpdecode_b200 import synth
+            for which in (wd.DT_WQKV, wd.DT_W_DOWN):
+                shp = dec.shape(which)
+                w = (rng.standard_normal(shp) * 0.05).astype(np.float32)
+                dec.set_tensor(l, which, synth.quantize_q8_0(w).reshape(-1), wd.TYPE_Q8_0)
+            dec.set_tensor(l, wd.DT_BQKV, (0.2 * rng.standard_normal(dec.vector_len(wd.DT_BQKV))).astype(np.float32))
+            for which in (wd.DT_Q_NORM, wd.DT_K_NORM):
+                dec.set_tensor(l, which, (1.0 + 0.2 * rng.standard_normal(hd)).astype(np.float32))
+    prompt = rng.integers(0, V, P)
+    got, _ = dec.decode(prompt, G)
+    logits, hidden = dec.read()
+    ref = _oracle_for(wd, oracle, dec, cfg, 500000.0)
+    want = ref.decode(prompt, G)
+    assert np.array_equal(got, want)
+    assert np.array_equal(ol.fbits(logits), ol.fbits(ref.logits))
+    assert np.array_equal(ol.fbits(hidden), ol.fbits(ref.hidden))
+    again, _ = dec.decode(prompt[:max(2, P // 2)], 1)          # a shorter prompt on the used caches and workspace
+    assert np.array_equal(again, ref.decode(prompt[:max(2, P // 2)], 1))
+    dec.close()

@@ -24,6 +24,7 @@
 #include "wd_dense.cuh"
 #include "wd_dense_decoder.cuh"
 #include "wd_dense_token.cuh"
+#include "wd_dense_prefill.cuh"
 #include "wd_plain_moe.cuh"
 #include "wd_grids.h"
 
