@@ -24,7 +24,8 @@ CASES = [(256, 4, 2, 64, 512, 2, 2, 3, "q4"),
          (256, 2, 1, 128, 1056, 2, 33, 0, "q4"),         # 33 blocks: one lane with two; nothing generated
          (1024, 8, 8, 32, 2816, 1, 40, 5, "file"),       # Q8_0 matrices, biases, head norms
          (2048, 32, 8, 64, 8192, 1, 70, 2, "q4"),        # the benchmark width: the wide row tile
-         (256, 4, 1, 64, 256, 1, 530, 3, "q4")]          # two chunks
+         (512, 4, 2, 128, 512, 1, 300, 4, "q4"),         # more positions than the value ring of the decode attention holds
+         (256, 4, 1, 64, 256, 1, 530, 3, "q4")]          # two chunks; likewise
 
 
 @pytest.mark.parametrize("H,nh,nkv,hd,F,L,P,G,style", CASES)

@@ -454,43 +454,128 @@ __device__ __forceinline__ float dense_attention_core(const float *qs, const flo
     return 0.0f;
 }
 
-// Rotary embedding + cache store + decode attention + Q8_0 of the head's output, one CTA (128 threads) per query head
-// (rope_store_kernel :1855 and attention_decode_kernel :1902 of src/warodecode.cu, the latter as two passes; orders in
-// the header and in the oracle). The rotary embedding pairs element p with p + head_dim / 2 (GPT-NeoX) and takes
-// cos/sin from the table row of *pos. Every CTA rotates its own q head and, for itself, the new k head of its KV
-// group; the first CTA of a group also stores the rotated k and the v into the caches [max_ctx][kv_dim]. Cache
-// position pos itself is taken from the CTA's own copy, so no CTA waits for another's store.
-// head_dim a multiple of 32, at most 128; dynamic shared memory: max_ctx + 32 * head_dim floats.
+// The dot q . k of the one-token order - lane l runs fmaf over d = l, l + 32, ..., then the butterfly - by ONE thread, four
+// lanes at a time: quads of lanes meet in the butterfly's own pairs (16 apart, 8 apart, 4, 2, 1), so nothing is shuffled.
+template <int HD>
+__device__ __forceinline__ float lane_order_dot(const float *q, const float4 (&k)[HD / 4]) {
+    auto quad = [&](int b, float (&a)[4]) {         // lanes 4 b .. 4 b + 3
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = 0.0f;
+#pragma unroll
+        for (int r = 0; r < HD / 32; ++r) {
+            const float4 qv = *reinterpret_cast<const float4 *>(q + r * 32 + b * 4);
+            const float4 kv = k[r * 8 + b];
+            a[0] = __fmaf_rn(qv.x, kv.x, a[0]);
+            a[1] = __fmaf_rn(qv.y, kv.y, a[1]);
+            a[2] = __fmaf_rn(qv.z, kv.z, a[2]);
+            a[3] = __fmaf_rn(qv.w, kv.w, a[3]);
+        }
+    };
+    float s8[2][4];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {                   // lanes 4 p .. 4 p + 3 with those 16, 8 and 24 above
+        float a[4], b[4], c[4], d[4];
+        quad(p, a);
+        quad(p + 4, b);
+        asm volatile("" ::: "memory");              // the loads of q stay behind this point: registers belong to the key
+        quad(p + 2, c);
+        quad(p + 6, d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s8[p][i] = __fadd_rn(__fadd_rn(a[i], b[i]), __fadd_rn(c[i], d[i]));
+        asm volatile("" ::: "memory");
+    }
+    float s4[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s4[i] = __fadd_rn(s8[0][i], s8[1][i]);
+    return __fadd_rn(__fadd_rn(s4[0], s4[2]), __fadd_rn(s4[1], s4[3]));
+}
+
+// Asynchronous 16-byte copy global -> shared; !live fills the destination with zeros.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool live) {
+    const int bytes = live ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Geometry of the decode attention for a head dimension: threads, and the ring of value chunks (64 positions each).
+template <int HD>
+struct DecodeAttn {
+    static constexpr int kThreads = HD <= 64 ? 512 : 256;       // a thread keeps a whole key in registers
+    static constexpr int kChunk = 64, kRing = HD <= 64 ? 8 : 4; // values in flight: 128 KB at most
+};
+
+// Rotary embedding + cache store + decode attention + Q8_0 of the head's output, one CTA per query head (rope_store_kernel
+// :1855 and attention_decode_kernel :1902 of src/warodecode.cu, the latter as two passes; orders in the header and in the
+// oracle). The rotary embedding pairs element p with p + head_dim / 2 (GPT-NeoX) and takes cos/sin from the table row of
+// *pos. Every CTA rotates its own q head and, for itself, the new k head of its KV group; the first CTA of a group also
+// stores the rotated k and the v into the caches [max_ctx][kv_dim]. Cache position pos itself is taken from the CTA's own
+// copy, so no CTA waits for another's store.
+//
+// Bound: latency. The sums over positions run ascending (one fmaf per position and element, four cycles each), so the
+// keys and values must be there when they are needed: the cache below pos was written by earlier graph launches, and
+// its first 256 or 512 keys (one per thread, in registers) and the first chunks of the values (shared memory) are
+// requested BEFORE the wait for the QKV product; a score is one thread's work, without shuffles.
+// Measured on the 16-layer model (32 heads of 64): 512 positions 1.8 ms -> see the design table, 72 positions likewise.
+//
 // EXTRAS: the layer has q/k/v biases (Qwen2-style files: added to the QKV product's rows) and / or RMSNorm weights for
 // the q and k heads (Qwen3-style: qk_norm_kernel, src/warodecode.cu:1836), applied in that order before the rotary
 // embedding (emit_step :2069-2075). Layers without them run the instantiation that has none of that code.
-template <bool EXTRAS>
-__global__ void __launch_bounds__(128) dense_attention_kernel(const float *qkv, const float *table, float *kcache, float *vcache,
-                                                              const int *pos_ptr, int heads, int kv_heads, int head_dim, int max_ctx,
-                                                              float inv_sqrt, int8_t *oq, float *od, const float *bqkv,
-                                                              const float *q_norm, const float *k_norm, float eps) {
-    extern __shared__ __align__(16) float sc[];        // [max_ctx] scores, then [32][head_dim] value staging
-    __shared__ float qs[128], kn[128], vn[128], outv[128];
-    float *vbuf = sc + max_ctx;
+// Dynamic shared memory: `ring` value chunks, then max_ctx scores.
+template <int HD, bool EXTRAS>
+__global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kernel(const float *qkv, const float *table, float *kcache,
+                                                                                 float *vcache, const int *pos_ptr, int heads,
+                                                                                 int kv_heads, int ring, float inv_sqrt, int8_t *oq,
+                                                                                 float *od, const float *bqkv, const float *q_norm,
+                                                                                 const float *k_norm, float eps) {
+    using A = DecodeAttn<HD>;
+    constexpr int kNt = A::kThreads, kChunk = A::kChunk, kHalf = HD / 2, kRow16 = HD / 4;
+    extern __shared__ __align__(16) float vring[];
+    __shared__ __align__(16) float qs[HD], kn[HD];
+    __shared__ float vn[HD], outv[HD], wmax[kNt / 32];
+    float *sc = vring + static_cast<size_t>(ring) * kChunk * HD;
     grid_dep_launch();
-    grid_dep_wait();
     const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int pos = *pos_ptr, kv_dim = kv_heads * head_dim, kvh = (h * kv_heads) / heads, half = head_dim / 2;
-    const float *q_raw = qkv + static_cast<size_t>(h) * head_dim;
-    const float *k_raw = qkv + static_cast<size_t>(heads + kvh) * head_dim;
-    const float *v_raw = qkv + static_cast<size_t>(heads + kv_heads + kvh) * head_dim;
+    const int pos = *pos_ptr, kv_dim = kv_heads * HD, kvh = (h * kv_heads) / heads;
+    float *kc = kcache + static_cast<size_t>(kvh) * HD, *vc = vcache + static_cast<size_t>(kvh) * HD;
+    const int n_chunks = (pos + kChunk - 1) / kChunk;           // positions 0 .. pos - 1
+    auto request = [&](int c) {
+        float *dst = vring + static_cast<size_t>(c % ring) * kChunk * HD;
+        for (int i = tid; i < kChunk * kRow16; i += kNt) {
+            const int r = i / kRow16, e = i - r * kRow16, t = c * kChunk + r;
+            if (t < pos) cp_async16(dst + r * HD + e * 4, vc + static_cast<size_t>(t) * kv_dim + e * 4, true);
+        }
+    };
+    for (int c = 0; c < min(ring, n_chunks); ++c) request(c);
+    cp_async_commit();
+    float4 k[HD / 4];
+    auto load_key = [&](int t) {
+#pragma unroll
+        for (int i = 0; i < HD / 4; ++i) k[i] = *reinterpret_cast<const float4 *>(kc + static_cast<size_t>(t) * kv_dim + i * 4);
+    };
+    if (tid < pos) load_key(tid);
+    float cs = 0.0f, sn = 0.0f;
+    if (tid < kHalf) {
+        cs = table[(static_cast<size_t>(pos) * kHalf + tid) * 2];
+        sn = table[(static_cast<size_t>(pos) * kHalf + tid) * 2 + 1];
+    }
+    grid_dep_wait();
+    const float *q_raw = qkv + static_cast<size_t>(h) * HD;
+    const float *k_raw = qkv + static_cast<size_t>(heads + kvh) * HD;
+    const float *v_raw = qkv + static_cast<size_t>(heads + kv_heads + kvh) * HD;
     if constexpr (EXTRAS) {
-        __shared__ float qn[128], kn_in[128], vn_in[128];
+        __shared__ float qn[HD], kn_in[HD], vn_in[HD];
         __shared__ double nred[2][4];
         float xq_ = 0.0f, xk_ = 0.0f, xv_ = 0.0f;
-        if (tid < head_dim) {
+        if (tid < HD) {
             xq_ = q_raw[tid];
             xk_ = k_raw[tid];
             xv_ = v_raw[tid];
             if (bqkv != nullptr) {
-                xq_ = __fadd_rn(xq_, bqkv[static_cast<size_t>(h) * head_dim + tid]);
-                xk_ = __fadd_rn(xk_, bqkv[static_cast<size_t>(heads + kvh) * head_dim + tid]);
-                xv_ = __fadd_rn(xv_, bqkv[static_cast<size_t>(heads + kv_heads + kvh) * head_dim + tid]);
+                xq_ = __fadd_rn(xq_, bqkv[static_cast<size_t>(h) * HD + tid]);
+                xk_ = __fadd_rn(xk_, bqkv[static_cast<size_t>(heads + kvh) * HD + tid]);
+                xv_ = __fadd_rn(xv_, bqkv[static_cast<size_t>(heads + kv_heads + kvh) * HD + tid]);
             }
         }
         if (q_norm != nullptr || k_norm != nullptr) {
@@ -503,22 +588,22 @@ __global__ void __launch_bounds__(128) dense_attention_kernel(const float *qkv, 
                 sq_ = __dadd_rn(sq_, __shfl_xor_sync(0xffffffffu, sq_, s));
                 sk_ = __dadd_rn(sk_, __shfl_xor_sync(0xffffffffu, sk_, s));
             }
-            if (lane == 0) {
+            if (lane == 0 && warp < 4) {
                 nred[0][warp] = sq_;
                 nred[1][warp] = sk_;
             }
             __syncthreads();
             const double tq = __dadd_rn(__dadd_rn(nred[0][0], nred[0][1]), __dadd_rn(nred[0][2], nred[0][3]));
             const double tk = __dadd_rn(__dadd_rn(nred[1][0], nred[1][1]), __dadd_rn(nred[1][2], nred[1][3]));
-            const double hd = static_cast<double>(head_dim), ep = static_cast<double>(eps);
+            const double hd = static_cast<double>(HD), ep = static_cast<double>(eps);
             const float scq = __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__ddiv_rn(tq, hd), ep))));
             const float sck = __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__ddiv_rn(tk, hd), ep))));
-            if (tid < head_dim) {
+            if (tid < HD) {
                 if (q_norm != nullptr) xq_ = __fmul_rn(__fmul_rn(xq_, scq), q_norm[tid]);
                 if (k_norm != nullptr) xk_ = __fmul_rn(__fmul_rn(xk_, sck), k_norm[tid]);
             }
         }
-        if (tid < head_dim) {
+        if (tid < HD) {
             qn[tid] = xq_;
             kn_in[tid] = xk_;
             vn_in[tid] = xv_;
@@ -528,36 +613,78 @@ __global__ void __launch_bounds__(128) dense_attention_kernel(const float *qkv, 
         k_raw = kn_in;
         v_raw = vn_in;
     }
-    float *kc = kcache + static_cast<size_t>(kvh) * head_dim, *vc = vcache + static_cast<size_t>(kvh) * head_dim;
     const bool writer = h % (heads / kv_heads) == 0;        // the first head of its KV group
-    if (tid < half) {
-        const float cs = table[(static_cast<size_t>(pos) * half + tid) * 2], sn = table[(static_cast<size_t>(pos) * half + tid) * 2 + 1];
-        {
-            const float a = q_raw[tid], b = q_raw[tid + half];
-            qs[tid] = __fadd_rn(__fmul_rn(a, cs), -__fmul_rn(b, sn));
-            qs[tid + half] = __fadd_rn(__fmul_rn(a, sn), __fmul_rn(b, cs));
-        }
-        const float a = k_raw[tid], b = k_raw[tid + half];
-        const float k0 = __fadd_rn(__fmul_rn(a, cs), -__fmul_rn(b, sn)), k1 = __fadd_rn(__fmul_rn(a, sn), __fmul_rn(b, cs));
+    if (tid < kHalf) {
+        const float a = q_raw[tid], b = q_raw[tid + kHalf], c = k_raw[tid], d = k_raw[tid + kHalf];
+        const float v0 = v_raw[tid], v1 = v_raw[tid + kHalf];
+        qs[tid] = __fadd_rn(__fmul_rn(a, cs), -__fmul_rn(b, sn));
+        qs[tid + kHalf] = __fadd_rn(__fmul_rn(a, sn), __fmul_rn(b, cs));
+        const float k0 = __fadd_rn(__fmul_rn(c, cs), -__fmul_rn(d, sn)), k1 = __fadd_rn(__fmul_rn(c, sn), __fmul_rn(d, cs));
         kn[tid] = k0;
-        kn[tid + half] = k1;
-        const float v0 = v_raw[tid], v1 = v_raw[tid + half];
+        kn[tid + kHalf] = k1;
         vn[tid] = v0;
-        vn[tid + half] = v1;
+        vn[tid + kHalf] = v1;
         if (writer) {
             const size_t off = static_cast<size_t>(pos) * kv_dim;
             kc[off + tid] = k0;
-            kc[off + tid + half] = k1;
+            kc[off + tid + kHalf] = k1;
             vc[off + tid] = v0;
-            vc[off + tid + half] = v1;
+            vc[off + tid + kHalf] = v1;
         }
     }
     __syncthreads();
-    const float o = dense_attention_core(qs, kn, vn, kc, vc, pos, kv_dim, head_dim, inv_sqrt, sc, vbuf, 128);
-    if (tid < head_dim) outv[tid] = o;
+    float m = -INFINITY;
+    for (int t = tid; t <= pos; t += kNt) {
+        if (t == pos) {
+#pragma unroll
+            for (int i = 0; i < HD / 4; ++i) k[i] = *reinterpret_cast<const float4 *>(kn + i * 4);
+        } else if (t != tid) {
+            load_key(t);
+        }
+        const float v = __fmul_rn(lane_order_dot<HD>(qs, k), inv_sqrt);
+        sc[t] = v;
+        m = v > m ? v : m;          // a NaN score never becomes the maximum
+    }
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+    if (lane == 0) wmax[warp] = m;
     __syncthreads();
-    if (warp < head_dim / 32) {
-        const int b = (h * head_dim) / 32 + warp;
+    m = wmax[lane & (kNt / 32 - 1)];
+#pragma unroll
+    for (int s = kNt / 64; s >= 1; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+    for (int t = tid; t <= pos; t += kNt) sc[t] = exp_ggml(__fadd_rn(sc[t], -m));
+    cp_async_wait<0>();
+    __syncthreads();
+    float l = 0.0f, acc = 0.0f;
+#pragma unroll 1
+    for (int c = 0; c < n_chunks; ++c) {
+        if (tid < HD) {
+            const float *v = vring + static_cast<size_t>(c % ring) * kChunk * HD + tid, *p = sc + c * kChunk;
+            const int n = min(kChunk, pos - c * kChunk);
+#pragma unroll 8
+            for (int r = 0; r < n; ++r) {
+                l = __fadd_rn(l, p[r]);
+                acc = __fmaf_rn(p[r], v[r * HD], acc);
+            }
+        }
+        if (n_chunks > ring) {      // longer than the ring: refill the slot, and wait when the next one was refilled too
+            __syncthreads();
+            if (c + ring < n_chunks) request(c + ring);
+            cp_async_commit();
+            if (c + 1 >= ring) {
+                cp_async_wait<A::kRing - 1>();
+                __syncthreads();
+            }
+        }
+    }
+    if (tid < HD) {
+        l = __fadd_rn(l, sc[pos]);
+        acc = __fmaf_rn(sc[pos], vn[tid], acc);
+        outv[tid] = __fdiv_rn(acc, l);
+    }
+    __syncthreads();
+    if (warp < HD / 32) {
+        const int b = (h * HD) / 32 + warp;
         q8_0_block_warp(outv[warp * 32 + lane], lane, oq + static_cast<size_t>(b) * 32, od + b);
     }
 }

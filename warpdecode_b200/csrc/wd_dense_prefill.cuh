@@ -47,18 +47,10 @@ __global__ void __launch_bounds__(kDecThreads) prefill_norm_quant_kernel(float *
 // so it walks the lanes l = 4 x + c with x in bit-reversed order and folds the finished lane sums with a three-deep stack;
 // the four residues meet in shared memory at the end ((c0 + c2) + (c1 + c3)). A stage of the copy pipeline holds, for
 // every row and token, the four neighbouring blocks 32 t + 4 x + {0..3} of two values of t.
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool live) {
-    const int bytes = live ? 16 : 0;        // 0: the destination is filled with zeros
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void cp_async4(void *dst, const void *src, bool live) {
     const int bytes = live ? 4 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 __device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
                  : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
@@ -306,40 +298,6 @@ __global__ void __launch_bounds__(128) prefill_rope_kernel(const float *qkv, con
 }
 
 // ---- attention of the chunk ----------------------------------------------------------------------------------------------
-// The dot q . k of the one-token order - lane l runs fmaf over d = l, l + 32, ..., then the butterfly - by ONE thread, four
-// lanes at a time: quads of lanes meet in the butterfly's own pairs (16 apart, 8 apart, 4, 2, 1), so nothing is shuffled.
-template <int HD>
-__device__ __forceinline__ float lane_order_dot(const float *q, const float4 (&k)[HD / 4]) {
-    auto quad = [&](int b, float (&a)[4]) {         // lanes 4 b .. 4 b + 3
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = 0.0f;
-#pragma unroll
-        for (int r = 0; r < HD / 32; ++r) {
-            const float4 qv = *reinterpret_cast<const float4 *>(q + r * 32 + b * 4);
-            const float4 kv = k[r * 8 + b];
-            a[0] = __fmaf_rn(qv.x, kv.x, a[0]);
-            a[1] = __fmaf_rn(qv.y, kv.y, a[1]);
-            a[2] = __fmaf_rn(qv.z, kv.z, a[2]);
-            a[3] = __fmaf_rn(qv.w, kv.w, a[3]);
-        }
-    };
-    float s8[2][4];
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {                   // lanes 4 p .. 4 p + 3 with those 16, 8 and 24 above
-        float a[4], b[4], c[4], d[4];
-        quad(p, a);
-        quad(p + 4, b);
-        quad(p + 2, c);
-        quad(p + 6, d);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) s8[p][i] = __fadd_rn(__fadd_rn(a[i], b[i]), __fadd_rn(c[i], d[i]));
-    }
-    float s4[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) s4[i] = __fadd_rn(s8[0][i], s8[1][i]);
-    return __fadd_rn(__fadd_rn(s4[0], s4[2]), __fadd_rn(s4[1], s4[3]));
-}
-
 constexpr int kPrefillAttnThreads = 288;    // eight warps on scores and values, one on the sums of the weights
 
 // One CTA per (head, QT consecutive tokens). Scores, weights and the sums over positions keep the one-token order: maximum,
