@@ -20,13 +20,18 @@ namespace wd {
 
 constexpr int kDecThreads = 256;
 
-// ggml Q4_0 blocks [rows][nb][18 B] -> [rows][nb][16 B] quants, then [rows][nb] f16 scales.
-__global__ void repack_q4_0_rows_kernel(const uint8_t *src, uint8_t *dst, long long nblocks) {
+// Blocks per row in the packed layouts: rounded up, so that a row's scales start on 8 bytes (the prompt pass copies four).
+// The blocks behind a row's end are never read.
+__host__ __device__ inline int dense_row_stride(int nb) { return (nb + 3) & ~3; }
+
+// ggml Q4_0 blocks [rows][nb][18 B] -> [rows][stride][16 B] quants, then [rows][stride] f16 scales.
+__global__ void repack_q4_0_rows_kernel(const uint8_t *src, uint8_t *dst, long long nblocks, int nb) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (i >= nblocks) return;
+    const long long row = i / nb, stride = dense_row_stride(nb), o = row * stride + (i - row * nb);
     const uint8_t *s = src + i * 18;
-    uint8_t *q = dst + i * 16;
-    uint16_t *d = reinterpret_cast<uint16_t *>(dst + nblocks * 16) + i;
+    uint8_t *q = dst + o * 16;
+    uint16_t *d = reinterpret_cast<uint16_t *>(dst + nblocks / nb * stride * 16) + o;
     *d = static_cast<uint16_t>(s[0] | (s[1] << 8));
     for (int j = 0; j < 16; ++j) q[j] = s[2 + j];
 }
@@ -70,8 +75,18 @@ __global__ void synth_q4_0_kernel(uint8_t *dst, long long nblocks, float sigma, 
     }
 }
 
+// A quant in the order the prompt pass multiplies with: lane q of an MMA reads values 4 q .. 4 q + 3 and 16 + 4 q .. of a
+// block as one 8-byte word (wd_dense_prefill.cuh).
+struct PairedQuant {
+    int8_t v;
+};
+__device__ __forceinline__ int paired_place(int v) { return ((v >> 2) & 3) * 8 + (v >> 4) * 4 + (v & 3); }
+__device__ __forceinline__ void store_quant(int8_t *out, int e, int q) { out[e] = static_cast<int8_t>(q); }
+__device__ __forceinline__ void store_quant(PairedQuant *out, int e, int q) { out[(e & ~31) + paired_place(e & 31)].v = static_cast<int8_t>(q); }
+
 // Q8_0 of 32 floats held one per lane: quant byte and the f16-rounded scale (ggml's rule, as quantize_q8_0_cta).
-__device__ __forceinline__ void q8_0_block_warp(float v, int lane, int8_t *q_out, float *d_out) {
+template <class Quant>
+__device__ __forceinline__ void q8_0_block_warp(float v, int lane, Quant *q_out, float *d_out) {
     float amax = fabsf(v);
 #pragma unroll
     for (int s = 16; s >= 1; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
@@ -80,7 +95,7 @@ __device__ __forceinline__ void q8_0_block_warp(float v, int lane, int8_t *q_out
         q = __float2int_rn(__fmul_rn(v, __fdiv_rn(127.0f, amax)));
         q = max(-128, min(127, q));
     }
-    q_out[lane] = static_cast<int8_t>(q);
+    store_quant(q_out, lane, q);
     if (lane == 0) *d_out = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
 }
 
@@ -89,8 +104,8 @@ __device__ __forceinline__ void q8_0_block_warp(float v, int lane, int8_t *q_out
 // so a Q8_0 block belongs to 32 / EPL neighbouring lanes (residual_rmsnorm_kernel, src/warodecode.cu:1408). The sum of
 // squares is the binary tree in double of the MoE stack's RMSNorm. `token` (optional): the step starts here, and
 // hidden is first filled with the token's embedding row (embedding_q4_kernel).
-template <int EPL>
-__device__ __forceinline__ void dense_norm_quant_body(float *hidden, const float *proj, const float *w, int n, float eps, int8_t *xq,
+template <int EPL, class Quant>
+__device__ __forceinline__ void dense_norm_quant_body(float *hidden, const float *proj, const float *w, int n, float eps, Quant *xq,
                                                       float *xd, const uint8_t *embd_row, bool embd_q8 = false) {
     __shared__ double red[kDecThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -155,7 +170,7 @@ __device__ __forceinline__ void dense_norm_quant_body(float *hidden, const float
     for (int i = 0; i < EPL; ++i) {
         int q = amax != 0.0f ? __float2int_rn(__fmul_rn(v[i], inv)) : 0;
         q = max(-128, min(127, q));
-        xq[tid * EPL + i] = static_cast<int8_t>(q);
+        store_quant(xq, tid * EPL + i, q);
     }
     if ((tid * EPL & 31) == 0) xd[(tid * EPL) >> 5] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
 }
@@ -194,7 +209,8 @@ __global__ void __launch_bounds__(kDecThreads, 4) dense_gemv_q4_0_kernel(const u
     float *sd = reinterpret_cast<float *>(dsm + static_cast<size_t>(nb) * 32);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const uint4 *q_all = reinterpret_cast<const uint4 *>(wp);
-    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * nb * 16);
+    const int stride = dense_row_stride(nb);
+    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * stride * 16);
     uint4 w[R][U];
     uint16_t dw[R][U];
     auto load = [&](int row0, int b0) {
@@ -204,8 +220,8 @@ __global__ void __launch_bounds__(kDecThreads, 4) dense_gemv_q4_0_kernel(const u
             for (int u = 0; u < U; ++u) {
                 const int b = b0 + 32 * u;
                 if (b < nb && row0 + r < rows) {
-                    w[r][u] = __ldg(q_all + static_cast<size_t>(row0 + r) * nb + b);
-                    dw[r][u] = __ldg(d_all + static_cast<size_t>(row0 + r) * nb + b);
+                    w[r][u] = __ldg(q_all + static_cast<size_t>(row0 + r) * stride + b);
+                    dw[r][u] = __ldg(d_all + static_cast<size_t>(row0 + r) * stride + b);
                 }
             }
     };
@@ -275,14 +291,15 @@ __global__ void __launch_bounds__(kDecThreads, 4) dense_gemv_q4_0_kernel(const u
     }
 }
 
-// ggml Q8_0 [rows][nb] blocks of 34 bytes -> the row layout of dense_gemv_q8_0_kernel: [rows][nb][32 B] quants, then
-// [rows][nb] f16 scales. One thread per block.
-__global__ void repack_q8_0_dense_kernel(const uint8_t *src, uint8_t *dst, long long nblocks) {
+// ggml Q8_0 [rows][nb] blocks of 34 bytes -> the row layout of dense_gemv_q8_0_kernel: [rows][stride][32 B] quants, then
+// [rows][stride] f16 scales. One thread per block.
+__global__ void repack_q8_0_dense_kernel(const uint8_t *src, uint8_t *dst, long long nblocks, int nb) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (i >= nblocks) return;
+    const long long row = i / nb, stride = dense_row_stride(nb), o = row * stride + (i - row * nb);
     const uint8_t *s = src + i * 34;
-    uint8_t *q = dst + i * 32;
-    uint16_t *d = reinterpret_cast<uint16_t *>(dst + nblocks * 32) + i;
+    uint8_t *q = dst + o * 32;
+    uint16_t *d = reinterpret_cast<uint16_t *>(dst + nblocks / nb * stride * 32) + o;
     *d = static_cast<uint16_t>(s[0] | (s[1] << 8));
     for (int j = 0; j < 32; ++j) q[j] = s[2 + j];
 }
@@ -300,7 +317,8 @@ __global__ void __launch_bounds__(kDecThreads, 4) dense_gemv_q8_0_kernel(const u
     float *sd = reinterpret_cast<float *>(dsm + static_cast<size_t>(nb) * 32);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const uint4 *q_all = reinterpret_cast<const uint4 *>(wp);
-    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * nb * 32);
+    const int stride = dense_row_stride(nb);
+    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * stride * 32);
     uint4 wl[R][U], wh[R][U];
     uint16_t dw[R][U];
     auto load = [&](int row0, int b0) {
@@ -310,7 +328,7 @@ __global__ void __launch_bounds__(kDecThreads, 4) dense_gemv_q8_0_kernel(const u
             for (int u = 0; u < U; ++u) {
                 const int b = b0 + 32 * u;
                 if (b < nb && row0 + r < rows) {
-                    const size_t blk = static_cast<size_t>(row0 + r) * nb + b;
+                    const size_t blk = static_cast<size_t>(row0 + r) * stride + b;
                     wl[r][u] = __ldg(q_all + 2 * blk);
                     wh[r][u] = __ldg(q_all + 2 * blk + 1);
                     dw[r][u] = __ldg(d_all + blk);

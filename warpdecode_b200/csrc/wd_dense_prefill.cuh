@@ -14,7 +14,7 @@ constexpr int kPrefillChunk = 512;      // tokens per pass at most (workspace: a
 
 // RMSNorm + Q8_0 of every token of the chunk, one CTA per token; the body is the one-token kernel's.
 __global__ void __launch_bounds__(kDecThreads) prefill_norm_quant_kernel(float *hidden, const float *proj, const float *w, int n, float eps,
-                                                                       int8_t *xq, float *xd, const uint8_t *embd, const int *tokens,
+                                                                       PairedQuant *xq, float *xd, const uint8_t *embd, const int *tokens,
                                                                        int vocab, int embd_q8) {
     grid_dep_launch();
     grid_dep_wait();
@@ -38,43 +38,76 @@ __global__ void __launch_bounds__(kDecThreads) prefill_norm_quant_kernel(float *
 // ---- Y[m][row] = W[row] . X[m] for the tokens of a chunk ---------------------------------------------------------------
 // The one-token order is: lane l of 32 runs one fmaf(d_w * d_x, (float)int_dot, acc) per block b = l, l + 32, ... ascending,
 // then the butterfly ^16 ^8 ^4 ^2 ^1. The integer dot of one block is a contraction of depth 32, i.e. exactly one
-// mma.m16n8k32 (s8) for 16 rows x 8 tokens; its result cannot be accumulated over blocks, because every block is scaled
-// by its own d_w * d_x in float. That float side (convert, scale, fmaf: 12 instructions per lane and MMA) is what bounds
-// the kernel, so the fragments are taken from mma.sync, whose result is already in registers; tcgen05 would add a TMEM
-// read-back per block to the same float work.
+// mma.m16n8k32 (s8) for 16 rows x 8 tokens; it cannot be accumulated over blocks, because every block is scaled by its own
+// d_w * d_x in float. That float side (packed subtract, multiply and fmaf, two of each per lane and tile), the expansion
+// of the nibbles and the staging are what the kernel issues. The form on halves (two m16n8k16 per block, the sums exact as
+// well, no conversion afterwards) measured 10 % slower: its operands take twice the shared memory and more instructions.
 //
 // A warp owns 16 rows, 8 * NT tokens and one residue c = l mod 4 of the lanes: ^16, ^8 and ^4 pair lanes of one residue,
 // so it walks the lanes l = 4 x + c with x in bit-reversed order and folds the finished lane sums with a three-deep stack;
 // the four residues meet in shared memory at the end ((c0 + c2) + (c1 + c3)). A stage of the copy pipeline holds, for
 // every row and token, the four neighbouring blocks 32 t + 4 x + {0..3} of two values of t.
+__device__ __forceinline__ void cp_async8(void *dst, const void *src, int bytes) {     // the rest of the eight bytes is zeroed
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp_async4(void *dst, const void *src, bool live) {
     const int bytes = live ? 4 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+// Two floats per instruction (each half rounded like the scalar operation).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
-// Shared-memory plan of one stage (TC = 2 values of t, four blocks each). The 16-byte pads put the eight rows (or tokens)
-// of a fragment into different banks.
+// The integer accumulator starts at the bit pattern of 12582912.0f = 1.5 * 2^23: for |sum| < 2^22 the result read as a float
+// is 12582912 + sum, and one exact subtraction gives (float)sum. Sums here stay below 2^20.
+constexpr int kMagicBits = 0x4b400000;
+constexpr float kMagic = 12582912.0f;
+__device__ __forceinline__ void mma_s8(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    int i[4];
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=r"(i[0]), "=r"(i[1]), "=r"(i[2]), "=r"(i[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(kMagicBits));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) d[k] = __int_as_float(i[k]);
+}
+
+// Shared-memory plan of one stage (TC = 2 values of t, four blocks each). The pads put the rows (or tokens) of a
+// fragment into different banks.
 template <bool Q8, int RG, int NT>
 struct PrefillGemm {
     static constexpr int kTc = 2, kRows = 16 * RG, kTok = 8 * NT, kThreads = 128 * RG;
     static constexpr int kBlk = Q8 ? 32 : 16;
-    static constexpr int kWStride = kTc * 4 * kBlk + 16, kXStride = kTc * 4 * 32 + 16;
-    static constexpr int kDwStride = kTc * 4 * 2 + 8, kDxStride = kTc * 4 * 4 + 16;
+    static constexpr int kWStride = kTc * 4 * kBlk + 16, kXStride = kTc * 4 * 32 + 32;
+    static constexpr int kDwStride = kTc * 4 * 2 + 8, kDxStride = kTok * 4;     // d_x: [block][token]
     static constexpr int kOffX = kRows * kWStride, kOffDw = kOffX + kTok * kXStride, kOffDx = kOffDw + kRows * kDwStride;
-    static constexpr int kStage = (kOffDx + kTok * kDxStride + 127) / 128 * 128;
+    static constexpr int kStage = (kOffDx + kTc * 4 * kDxStride + 127) / 128 * 128;
     static constexpr int kRed = 4 * kTok * (kRows + 4) * 4;              // the residues' sums, after the last stage
     static constexpr int kStages = NT == 4 ? 4 : 6;
     static constexpr int kSmem = kStages * kStage > kRed ? kStages * kStage : kRed;
-    static constexpr int kDwPer = kRows * kTc * 4 / kThreads;            // scales one thread moves per stage
 };
 
 template <bool Q8, int RG, int NT>
-__global__ void __launch_bounds__(128 * RG) prefill_gemm_kernel(const uint8_t *wp, int rows, int nb, const int8_t *xq, const float *xd, int m_tokens,
+__global__ void __launch_bounds__(128 * RG) prefill_gemm_kernel(const uint8_t *wp, int rows, int nb, const PairedQuant *xq, const float *xd, int m_tokens,
                                                                float *y) {
     using G = PrefillGemm<Q8, RG, NT>;
     extern __shared__ __align__(128) uint8_t gsm[];
@@ -83,148 +116,147 @@ __global__ void __launch_bounds__(128 * RG) prefill_gemm_kernel(const uint8_t *w
     const int res = warp & 3, rg = warp >> 2, g = lane >> 2, q = lane & 3;
     const int row0 = blockIdx.x * G::kRows, tok0 = blockIdx.y * G::kTok;
     const uint8_t *q_all = wp;
-    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * nb * G::kBlk);
+    const int nbp = dense_row_stride(nb);
+    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * nbp * G::kBlk);
     const int n_t = (nb + 31) >> 5, n_tc = (n_t + G::kTc - 1) / G::kTc, n_stage = 8 * n_tc;
     auto bitrev3 = [](int j) { return ((j & 1) << 2) | (j & 2) | ((j >> 2) & 1); };
-
-    uint16_t dw_next[G::kDwPer];
-    auto load_dw = [&](int s) {
-        const int x4 = 4 * bitrev3(s / n_tc), t0 = (s % n_tc) * G::kTc;
-#pragma unroll
-        for (int i = 0; i < G::kDwPer; ++i) {
-            const int e = tid + i * G::kThreads, r = e / (G::kTc * 4), k = e % (G::kTc * 4);
-            const int b = 32 * (t0 + (k >> 2)) + x4 + (k & 3);
-            dw_next[i] = (row0 + r < rows && b < nb) ? __ldg(d_all + static_cast<size_t>(row0 + r) * nb + b) : static_cast<uint16_t>(0);
+    // position of a producer in the sequence of stages: slot in the ring, first block of the stage
+    struct Cursor {
+        int slot = 0, j = 0, tc = 0;
+    };
+    auto base_of = [&](const Cursor &c) { return 32 * G::kTc * c.tc + 4 * bitrev3(c.j); };
+    auto advance = [&](Cursor &c) {
+        if (++c.slot == G::kStages) c.slot = 0;
+        if (++c.tc == n_tc) {
+            c.tc = 0;
+            ++c.j;
         }
     };
-    auto store_dw = [&](int s) {
-        uint8_t *st = gsm + (s % G::kStages) * G::kStage + G::kOffDw;
-#pragma unroll
-        for (int i = 0; i < G::kDwPer; ++i) {
-            const int e = tid + i * G::kThreads, r = e / (G::kTc * 4), k = e % (G::kTc * 4);
-            *reinterpret_cast<uint16_t *>(st + r * G::kDwStride + k * 2) = dw_next[i];
-        }
-    };
-    auto issue_w = [&](int s) {
-        uint8_t *st = gsm + (s % G::kStages) * G::kStage;
-        const int x4 = 4 * bitrev3(s / n_tc), t0 = (s % n_tc) * G::kTc;
+    auto issue_w = [&](const Cursor &c) {
+        uint8_t *st = gsm + c.slot * G::kStage;
+        const int b0 = base_of(c);
         constexpr int kPer = G::kTc * 4 * (G::kBlk / 16);       // 16-byte pieces of a row
 #pragma unroll
-        for (int e = tid; e < G::kRows * kPer; e += G::kThreads) {
-            const int r = e / kPer, p = e % kPer, k = p / (G::kBlk / 16), h = p % (G::kBlk / 16);
-            const int b = 32 * (t0 + (k >> 2)) + x4 + (k & 3);
+        for (int i = 0; i < G::kRows * kPer / G::kThreads; ++i) {
+            const int e = tid + i * G::kThreads, r = e / kPer, p = e % kPer, k = p / (G::kBlk / 16), h = p % (G::kBlk / 16);
+            const int b = b0 + 32 * (k >> 2) + (k & 3);
             const bool live = row0 + r < rows && b < nb;
-            cp_async16(st + r * G::kWStride + p * 16, live ? q_all + (static_cast<size_t>(row0 + r) * nb + b) * G::kBlk + h * 16 : q_all, live);
+            cp_async16(st + r * G::kWStride + p * 16, live ? q_all + static_cast<size_t>((row0 + r) * nbp + b) * G::kBlk + h * 16 : q_all, live);
+        }
+        if (tid < G::kRows * G::kTc) {      // four scales of a row (zero past its end, so a missing block adds nothing)
+            const int r = tid / G::kTc, k = tid % G::kTc, b = b0 + 32 * k;
+            const bool live = row0 + r < rows && b < nb;
+            cp_async8(st + G::kOffDw + r * G::kDwStride + k * 8, live ? d_all + static_cast<size_t>(row0 + r) * nbp + b : d_all,
+                      live ? 2 * min(4, nb - b) : 0);
         }
     };
-    auto issue_x = [&](int s) {
-        uint8_t *st = gsm + (s % G::kStages) * G::kStage;
-        const int x4 = 4 * bitrev3(s / n_tc), t0 = (s % n_tc) * G::kTc;
+    auto issue_x = [&](const Cursor &c) {
+        uint8_t *st = gsm + c.slot * G::kStage;
+        const int b0 = base_of(c);
         constexpr int kPer = G::kTc * 4 * 2;
 #pragma unroll
-        for (int e = tid; e < G::kTok * kPer; e += G::kThreads) {
-            const int r = e / kPer, p = e % kPer, b = 32 * (t0 + (p >> 3)) + x4 + ((p >> 1) & 3);
+        for (int i = 0; i < (G::kTok * kPer + G::kThreads - 1) / G::kThreads; ++i) {
+            const int e = tid + i * G::kThreads, r = e / kPer, p = e % kPer, b = b0 + 32 * (p >> 3) + ((p >> 1) & 3);
             const bool live = tok0 + r < m_tokens && b < nb;
-            cp_async16(st + G::kOffX + r * G::kXStride + p * 16,
-                       live ? xq + (static_cast<size_t>(tok0 + r) * nb + b) * 32 + (p & 1) * 16 : xq, live);
+            if (G::kTok * kPer >= G::kThreads || e < G::kTok * kPer)
+                cp_async16(st + G::kOffX + r * G::kXStride + p * 16,
+                           live ? xq + static_cast<size_t>((tok0 + r) * nb + b) * 32 + (p & 1) * 16 : xq, live);
         }
-        for (int e = tid; e < G::kTok * G::kTc * 4; e += G::kThreads) {
-            const int r = e / (G::kTc * 4), k = e % (G::kTc * 4), b = 32 * (t0 + (k >> 2)) + x4 + (k & 3);
+        if (tid < G::kTok * G::kTc * 4) {
+            const int r = tid / (G::kTc * 4), k = tid % (G::kTc * 4), b = b0 + 32 * (k >> 2) + (k & 3);
             const bool live = tok0 + r < m_tokens && b < nb;
-            cp_async4(st + G::kOffDx + r * G::kDxStride + k * 4, live ? xd + static_cast<size_t>(tok0 + r) * nb + b : xd, live);
+            cp_async4(st + G::kOffDx + k * G::kDxStride + r * 4, live ? xd + static_cast<size_t>(tok0 + r) * nb + b : xd, live);
         }
     };
+    static_assert(G::kRows * G::kTc <= G::kThreads && G::kTok * G::kTc * 4 <= G::kThreads, "one piece of the scales per thread and stage");
 
     // the weights do not depend on the kernel before this one: the first stages' rows leave before the wait for it
+    Cursor cw, cx;
     for (int s = 0; s < G::kStages - 1; ++s)
         if (s < n_stage) {
-            issue_w(s);
-            load_dw(s);
-            store_dw(s);
+            issue_w(cw);
+            advance(cw);
         }
     grid_dep_wait();
     for (int s = 0; s < G::kStages - 1; ++s) {
-        if (s < n_stage) issue_x(s);
+        if (s < n_stage) {
+            issue_x(cx);
+            advance(cx);
+        }
         cp_async_commit();
     }
-    float acc[NT][4], s0[NT][4], s1[NT][4], s2[NT][4];
+    f32x2 acc[NT][2], s0[NT][2], s1[NT][2], s2[NT][2];      // (token 2 q, token 2 q + 1) of row g, then of row g + 8
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[n][i] = s0[n][i] = s1[n][i] = s2[n][i] = 0.0f;
-    int j = 0, tc = 0;
+        for (int i = 0; i < 2; ++i) acc[n][i] = s0[n][i] = s1[n][i] = s2[n][i] = 0ull;
+    const f32x2 unmagic = pack2(-kMagic, -kMagic);
+    int slot = 0, left = n_stage - (G::kStages - 1);        // stages still to be requested
+    const uint8_t *wbase = gsm + (rg * 16 + g) * G::kWStride, *xbase = gsm + G::kOffX + g * G::kXStride + q * 8;
+    const uint8_t *dwbase = gsm + G::kOffDw + (rg * 16 + g) * G::kDwStride, *dxbase = gsm + G::kOffDx + 8 * q;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
 #pragma unroll 1
-    for (int s = 0; s < n_stage; ++s) {
+        for (int tc = 0; tc < n_tc; ++tc) {
         cp_async_wait<G::kStages - 2>();
-        __syncthreads();            // stage s has landed for everyone; the slot of stage s - 1 is free
-        const int nx = s + G::kStages - 1;
-        if (nx < n_stage) {
-            issue_w(nx);
-            issue_x(nx);
-            load_dw(nx);
+        __syncthreads();            // this stage has landed for everyone; the slot of the one before is free
+        if (left > 0) {
+            --left;
+            issue_w(cw);
+            issue_x(cw);
+            advance(cw);
         }
         cp_async_commit();
-        const uint8_t *st = gsm + (s % G::kStages) * G::kStage;
-        const uint8_t *wrow = st + (rg * 16 + g) * G::kWStride, *xrow = st + G::kOffX + g * G::kXStride;
-        const uint8_t *dwr = st + G::kOffDw + (rg * 16 + g) * G::kDwStride, *dxr = st + G::kOffDx + 2 * q * G::kDxStride;
+        const int so = slot * G::kStage;
+        if (++slot == G::kStages) slot = 0;
+        const uint8_t *wrow = wbase + so, *xrow = xbase + so, *dwr = dwbase + so, *dxr = dxbase + so;
 #pragma unroll
         for (int t = 0; t < G::kTc; ++t) {
             const int k = t * 4 + res;
-            uint32_t a0, a1, a2, a3;
+            uint32_t a[4];
             if constexpr (Q8) {
-                a0 = *reinterpret_cast<const uint32_t *>(wrow + k * 32 + q * 4);
-                a1 = *reinterpret_cast<const uint32_t *>(wrow + 8 * G::kWStride + k * 32 + q * 4);
-                a2 = *reinterpret_cast<const uint32_t *>(wrow + k * 32 + 16 + q * 4);
-                a3 = *reinterpret_cast<const uint32_t *>(wrow + 8 * G::kWStride + k * 32 + 16 + q * 4);
+                a[0] = *reinterpret_cast<const uint32_t *>(wrow + k * 32 + q * 4);
+                a[1] = *reinterpret_cast<const uint32_t *>(wrow + 8 * G::kWStride + k * 32 + q * 4);
+                a[2] = *reinterpret_cast<const uint32_t *>(wrow + k * 32 + 16 + q * 4);
+                a[3] = *reinterpret_cast<const uint32_t *>(wrow + 8 * G::kWStride + k * 32 + 16 + q * 4);
             } else {        // a nibble at the top of its byte with the top bit flipped is 16 * (q - 8)
                 const uint32_t w0 = *reinterpret_cast<const uint32_t *>(wrow + k * 16 + q * 4);
                 const uint32_t w1 = *reinterpret_cast<const uint32_t *>(wrow + 8 * G::kWStride + k * 16 + q * 4);
-                a0 = ((w0 << 4) & 0xf0f0f0f0u) ^ 0x80808080u;
-                a1 = ((w1 << 4) & 0xf0f0f0f0u) ^ 0x80808080u;
-                a2 = (w0 & 0xf0f0f0f0u) ^ 0x80808080u;
-                a3 = (w1 & 0xf0f0f0f0u) ^ 0x80808080u;
+                a[0] = ((w0 << 4) & 0xf0f0f0f0u) ^ 0x80808080u;
+                a[1] = ((w1 << 4) & 0xf0f0f0f0u) ^ 0x80808080u;
+                a[2] = (w0 & 0xf0f0f0f0u) ^ 0x80808080u;
+                a[3] = (w1 & 0xf0f0f0f0u) ^ 0x80808080u;
             }
             // d_w carries the 1/16 of a Q4_0 sum (a power of two: exact)
             const float f = Q8 ? 1.0f : 0.0625f;
             const float dw0 = half_bits_to_float(*reinterpret_cast<const uint16_t *>(dwr + k * 2)) * f;
             const float dw1 = half_bits_to_float(*reinterpret_cast<const uint16_t *>(dwr + 8 * G::kDwStride + k * 2)) * f;
+            const f32x2 dwp0 = pack2(dw0, dw0), dwp1 = pack2(dw1, dw1);
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                const uint8_t *xb = xrow + n * 8 * G::kXStride + k * 32 + q * 4;
-                int d[4];
-                mma_s8(d, a0, a1, a2, a3, *reinterpret_cast<const uint32_t *>(xb), *reinterpret_cast<const uint32_t *>(xb + 16));
-                const float dx0 = *reinterpret_cast<const float *>(dxr + n * 8 * G::kDxStride + k * 4);
-                const float dx1 = *reinterpret_cast<const float *>(dxr + (n * 8 + 1) * G::kDxStride + k * 4);
-                acc[n][0] = __fmaf_rn(__fmul_rn(dw0, dx0), static_cast<float>(d[0]), acc[n][0]);
-                acc[n][1] = __fmaf_rn(__fmul_rn(dw0, dx1), static_cast<float>(d[1]), acc[n][1]);
-                acc[n][2] = __fmaf_rn(__fmul_rn(dw1, dx0), static_cast<float>(d[2]), acc[n][2]);
-                acc[n][3] = __fmaf_rn(__fmul_rn(dw1, dx1), static_cast<float>(d[3]), acc[n][3]);
+                const uint2 x = *reinterpret_cast<const uint2 *>(xrow + n * 8 * G::kXStride + k * 32);
+                float d[4];
+                mma_s8(d, a, x.x, x.y);
+                const f32x2 dx = *reinterpret_cast<const f32x2 *>(dxr + k * G::kDxStride + n * 32);
+                acc[n][0] = fma2(mul2(dwp0, dx), add2(pack2(d[0], d[1]), unmagic), acc[n][0]);
+                acc[n][1] = fma2(mul2(dwp1, dx), add2(pack2(d[2], d[3]), unmagic), acc[n][1]);
             }
         }
-        if (nx < n_stage) store_dw(nx);
-        if (++tc == n_tc) {         // lane 4 x + c is complete: fold it into the tree
-            tc = 0;
-#pragma unroll
-            for (int n = 0; n < NT; ++n)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    float v = acc[n][i];
-                    if (j & 1) {
-                        v = __fadd_rn(s0[n][i], v);
-                        if (j & 2) {
-                            v = __fadd_rn(s1[n][i], v);
-                            if (j & 4) acc[n][i] = __fadd_rn(s2[n][i], v);
-                            else s2[n][i] = v;
-                        } else {
-                            s1[n][i] = v;
-                        }
-                    } else {
-                        s0[n][i] = v;
-                    }
-                    if (j != 7) acc[n][i] = 0.0f;
-                }
-            ++j;
         }
+        // lane 4 x + c is complete: fold it into the tree
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                f32x2 v = acc[n][i];
+                if (j & 1) v = add2(s0[n][i], v);
+                else s0[n][i] = v;
+                if ((j & 3) == 3) v = add2(s1[n][i], v);
+                else if (j & 1) s1[n][i] = v;
+                if (j == 7) v = add2(s2[n][i], v);
+                else if (j == 3) s2[n][i] = v;
+                acc[n][i] = j == 7 ? v : 0ull;
+            }
     }
     cp_async_wait<0>();
     __syncthreads();
@@ -234,8 +266,13 @@ __global__ void __launch_bounds__(128 * RG) prefill_gemm_kernel(const uint8_t *w
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            red[(res * G::kTok + n * 8 + 2 * q + (i & 1)) * kRs + rg * 16 + g + (i >> 1) * 8] = acc[n][i];
+        for (int i = 0; i < 2; ++i) {
+            float lo, hi;
+            unpack2(acc[n][i], lo, hi);
+            float *dst = red + (res * G::kTok + n * 8 + 2 * q) * kRs + rg * 16 + g + i * 8;
+            dst[0] = lo;
+            dst[kRs] = hi;
+        }
     __syncthreads();
     for (int e = tid; e < G::kTok * G::kRows; e += G::kThreads) {
         const int t = e / G::kRows, r = e % G::kRows;
@@ -248,56 +285,98 @@ __global__ void __launch_bounds__(128 * RG) prefill_gemm_kernel(const uint8_t *w
 }
 
 // ---- rotary embedding and cache store of the chunk ----------------------------------------------------------------------
-// One CTA of 128 threads per (token, head): the q heads go to `qrot` [token][heads * head_dim], the k heads (with their v
-// head) into the caches. Biases, head norms and the rotation are the one-token kernel's, in the same order.
-__global__ void __launch_bounds__(128) prefill_rope_kernel(const float *qkv, const float *table, float *kcache, float *vcache, int pos0,
-                                                           int heads, int kv_heads, int head_dim, float *qrot, const float *bqkv,
-                                                           const float *q_norm, const float *k_norm, float eps) {
-    __shared__ float row[128];
-    __shared__ double red[4];
+// One CTA of eight warps per token, one warp per head: the q heads go to `qrot` [token][heads * head_dim], the k heads (with
+// their v head) into the caches. Biases, head norms and the rotation are the one-token kernel's, in the same order: the sum
+// of squares is the binary tree in double over the head's elements, zero-padded to 128 leaves (lane l holds leaves l + 32 i).
+constexpr int kRopeWarps = 8;
+__global__ void __launch_bounds__(32 * kRopeWarps) prefill_rope_kernel(const float *qkv, const float *table, float *kcache, float *vcache,
+                                                                     int pos0, int heads, int kv_heads, int head_dim, float *qrot,
+                                                                     const float *bqkv, const float *q_norm, const float *k_norm, float eps) {
+    __shared__ float rows[kRopeWarps][128];
     grid_dep_launch();
     grid_dep_wait();
-    const int m = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = head_dim / 2;
+    const int m = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = head_dim / 2, nd = head_dim / 32;
     const int kv_dim = kv_heads * head_dim, pos = pos0 + m;
     const float *src = qkv + static_cast<size_t>(m) * (heads + 2 * kv_heads) * head_dim;
-    const bool is_q = h < heads;
-    const float *norm = is_q ? q_norm : k_norm;
-    float x = 0.0f;
-    if (tid < head_dim) {
-        const size_t e = static_cast<size_t>(h) * head_dim + tid;       // q heads, then k heads
-        x = src[e];
-        if (bqkv != nullptr) x = __fadd_rn(x, bqkv[e]);
-    }
-    if (norm != nullptr) {      // the binary tree in double over the head's elements, zero-padded to 128 leaves
-        double s2 = __dmul_rn(static_cast<double>(x), static_cast<double>(x));
+    float *row = rows[warp];
+    for (int h = warp; h < heads + kv_heads; h += kRopeWarps) {
+        const bool is_q = h < heads;
+        const float *norm = is_q ? q_norm : k_norm;
+        float x[4];
 #pragma unroll
-        for (int s = 1; s < 32; s <<= 1) s2 = __dadd_rn(s2, __shfl_xor_sync(0xffffffffu, s2, s));
-        if (lane == 0) red[warp] = s2;
-        __syncthreads();
-        const double t = __dadd_rn(__dadd_rn(red[0], red[1]), __dadd_rn(red[2], red[3]));
-        const float sc = __double2float_rn(
-            __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__ddiv_rn(t, static_cast<double>(head_dim)), static_cast<double>(eps)))));
-        if (tid < head_dim) x = __fmul_rn(__fmul_rn(x, sc), norm[tid]);
-    }
-    row[tid] = x;
-    __syncthreads();
-    float *dst = is_q ? qrot + (static_cast<size_t>(m) * heads + h) * head_dim
-                      : kcache + static_cast<size_t>(pos) * kv_dim + static_cast<size_t>(h - heads) * head_dim;
-    if (tid < half) {
-        const float cs = table[(static_cast<size_t>(pos) * half + tid) * 2], sn = table[(static_cast<size_t>(pos) * half + tid) * 2 + 1];
-        const float a = row[tid], b = row[tid + half];
-        dst[tid] = __fadd_rn(__fmul_rn(a, cs), -__fmul_rn(b, sn));
-        dst[tid + half] = __fadd_rn(__fmul_rn(a, sn), __fmul_rn(b, cs));
-    }
-    if (!is_q && tid < head_dim) {
-        const size_t e = static_cast<size_t>(h + kv_heads) * head_dim + tid;
-        float v = src[e];
-        if (bqkv != nullptr) v = __fadd_rn(v, bqkv[e]);
-        vcache[static_cast<size_t>(pos) * kv_dim + static_cast<size_t>(h - heads) * head_dim + tid] = v;
+        for (int i = 0; i < 4; ++i) {
+            const int e = h * head_dim + i * 32 + lane;         // q heads, then k heads
+            x[i] = i < nd ? src[e] : 0.0f;
+            if (i < nd && bqkv != nullptr) x[i] = __fadd_rn(x[i], bqkv[e]);
+        }
+        if (norm != nullptr) {
+            double s2[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                s2[i] = __dmul_rn(static_cast<double>(x[i]), static_cast<double>(x[i]));
+#pragma unroll
+                for (int s = 1; s < 32; s <<= 1) s2[i] = __dadd_rn(s2[i], __shfl_xor_sync(0xffffffffu, s2[i], s));
+            }
+            const double t = __dadd_rn(__dadd_rn(s2[0], s2[1]), __dadd_rn(s2[2], s2[3]));
+            const float sc = __double2float_rn(
+                __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__ddiv_rn(t, static_cast<double>(head_dim)), static_cast<double>(eps)))));
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < nd) x[i] = __fmul_rn(__fmul_rn(x[i], sc), norm[i * 32 + lane]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < nd) row[i * 32 + lane] = x[i];
+        __syncwarp();
+        float *dst = is_q ? qrot + (static_cast<size_t>(m) * heads + h) * head_dim
+                          : kcache + static_cast<size_t>(pos) * kv_dim + static_cast<size_t>(h - heads) * head_dim;
+        for (int p = lane; p < half; p += 32) {
+            const float2 c = reinterpret_cast<const float2 *>(table)[static_cast<size_t>(pos) * half + p];
+            const float a = row[p], b = row[p + half];
+            dst[p] = __fadd_rn(__fmul_rn(a, c.x), -__fmul_rn(b, c.y));
+            dst[p + half] = __fadd_rn(__fmul_rn(a, c.y), __fmul_rn(b, c.x));
+        }
+        if (!is_q) {
+            for (int i = lane; i < head_dim; i += 32) {
+                const int e = (h + kv_heads) * head_dim + i;
+                float v = src[e];
+                if (bqkv != nullptr) v = __fadd_rn(v, bqkv[e]);
+                vcache[static_cast<size_t>(pos) * kv_dim + static_cast<size_t>(h - heads) * head_dim + i] = v;
+            }
+        }
     }
 }
 
 // ---- attention of the chunk ----------------------------------------------------------------------------------------------
+// lane_order_dot with two lanes per instruction
+template <int HD>
+__device__ __forceinline__ float lane_order_dot2(const float *q, const ulonglong2 (&k)[HD / 4]) {
+    auto quad = [&](int b, f32x2 (&a)[2]) {         // lanes 4 b .. 4 b + 3
+        a[0] = a[1] = 0ull;
+#pragma unroll
+        for (int r = 0; r < HD / 32; ++r) {
+            const ulonglong2 qv = *reinterpret_cast<const ulonglong2 *>(q + r * 32 + b * 4);
+            a[0] = fma2(qv.x, k[r * 8 + b].x, a[0]);
+            a[1] = fma2(qv.y, k[r * 8 + b].y, a[1]);
+        }
+    };
+    f32x2 s8[2][2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        f32x2 a[2], b[2], c[2], d[2];
+        quad(p, a);
+        quad(p + 4, b);
+        quad(p + 2, c);
+        quad(p + 6, d);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) s8[p][i] = add2(add2(a[i], b[i]), add2(c[i], d[i]));
+    }
+    float e0, e1;
+    unpack2(add2(add2(s8[0][0], s8[1][0]), add2(s8[0][1], s8[1][1])), e0, e1);      // lanes (0, 1) + (2, 3)
+    return __fadd_rn(e0, e1);
+}
+
 constexpr int kPrefillAttnThreads = 288;    // eight warps on scores and values, one on the sums of the weights
 
 // One CTA per (head, QT consecutive tokens). Scores, weights and the sums over positions keep the one-token order: maximum,
@@ -305,9 +384,9 @@ constexpr int kPrefillAttnThreads = 288;    // eight warps on scores and values,
 // element) runs side by side for QT tokens; a thread holds one element of several tokens, so a value is loaded once for
 // all of them. Shared memory: [positions][QT] scores, then the QT query heads.
 template <int HD, int QT>
-__global__ void __launch_bounds__(kPrefillAttnThreads) prefill_attention_kernel(const float *qrot, const float *kcache, const float *vcache,
+__global__ void __launch_bounds__(kPrefillAttnThreads, HD <= 64 ? 2 : 1) prefill_attention_kernel(const float *qrot, const float *kcache, const float *vcache,
                                                                               int pos0, int m_tokens, int heads, int kv_heads,
-                                                                              float inv_sqrt, int8_t *oq, float *od) {
+                                                                              float inv_sqrt, PairedQuant *oq, float *od) {
     extern __shared__ __align__(16) float asm_[];
     __shared__ float mx[QT], lsum[QT], part[QT * 16];
     grid_dep_launch();
@@ -323,13 +402,13 @@ __global__ void __launch_bounds__(kPrefillAttnThreads) prefill_attention_kernel(
     }
     __syncthreads();
     for (int t = tid; t <= last; t += kPrefillAttnThreads) {
-        float4 k[HD / 4];
+        ulonglong2 k[HD / 4];
 #pragma unroll
-        for (int i = 0; i < HD / 4; ++i) k[i] = *reinterpret_cast<const float4 *>(kc + static_cast<size_t>(t) * kv_dim + i * 4);
+        for (int i = 0; i < HD / 4; ++i) k[i] = *reinterpret_cast<const ulonglong2 *>(kc + static_cast<size_t>(t) * kv_dim + i * 4);
 #pragma unroll 1
         for (int r = 0; r < QT; r += 2) {
-            const float a = __fmul_rn(lane_order_dot<HD>(qs + r * HD, k), inv_sqrt);
-            const float b = __fmul_rn(lane_order_dot<HD>(qs + (r + 1) * HD, k), inv_sqrt);
+            const float a = __fmul_rn(lane_order_dot2<HD>(qs + r * HD, k), inv_sqrt);
+            const float b = __fmul_rn(lane_order_dot2<HD>(qs + (r + 1) * HD, k), inv_sqrt);
             *reinterpret_cast<float2 *>(sc + static_cast<size_t>(t) * QT + r) = make_float2(a, b);
         }
     }
@@ -355,10 +434,11 @@ __global__ void __launch_bounds__(kPrefillAttnThreads) prefill_attention_kernel(
     for (int i = tid; i < (last + 1) * QT; i += kPrefillAttnThreads) sc[i] = exp_ggml(__fadd_rn(sc[i], -mx[i % QT]));
     __syncthreads();
     constexpr int kGroups = 256 / HD < QT ? 256 / HD : QT, kPer = QT / kGroups;   // tokens of one thread
-    float acc[kPer];
+    constexpr int kPairs = (kPer + 1) / 2;
+    f32x2 acc[kPairs];
     const int grp = tid / HD, d = tid - grp * HD;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) acc[i] = 0.0f;
+    for (int i = 0; i < kPairs; ++i) acc[i] = 0ull;
     if (warp == 8) {
         if (lane < QT) {
             float l = 0.0f;
@@ -368,23 +448,53 @@ __global__ void __launch_bounds__(kPrefillAttnThreads) prefill_attention_kernel(
         }
     } else if (grp < kGroups) {
         const float *pr = sc + grp * kPer, *v = vc + d;
+        auto weights = [&](int t, f32x2 (&p)[kPairs]) {
+            const float *s = pr + static_cast<size_t>(t) * QT;
+            if constexpr (kPer >= 4) {
+#pragma unroll
+                for (int i = 0; i < kPer / 4; ++i) {
+                    const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(s + 4 * i);
+                    p[2 * i] = w.x;
+                    p[2 * i + 1] = w.y;
+                }
+            } else if constexpr (kPer == 2) {
+                p[0] = *reinterpret_cast<const f32x2 *>(s);
+            } else {
+                p[0] = pack2(s[0], 0.0f);
+            }
+        };
 #pragma unroll 8
         for (int t = 0; t <= first; ++t) {          // positions every token of the CTA attends to
             const float x = v[static_cast<size_t>(t) * kv_dim];
+            const f32x2 xx = pack2(x, x);
+            f32x2 p[kPairs];
+            weights(t, p);
 #pragma unroll
-            for (int i = 0; i < kPer; ++i) acc[i] = __fmaf_rn(pr[static_cast<size_t>(t) * QT + i], x, acc[i]);
+            for (int i = 0; i < kPairs; ++i) acc[i] = fma2(p[i], xx, acc[i]);
         }
-        for (int t = first + 1; t <= last; ++t) {
+        for (int t = first + 1; t <= last; ++t) {   // the causal edge: token i stops at position first + i
             const float x = v[static_cast<size_t>(t) * kv_dim];
 #pragma unroll
-            for (int i = 0; i < kPer; ++i)
-                if (t <= first + grp * kPer + i) acc[i] = __fmaf_rn(pr[static_cast<size_t>(t) * QT + i], x, acc[i]);
+            for (int i = 0; i < kPairs; ++i) {
+                float lo, hi;
+                unpack2(acc[i], lo, hi);
+                const int r = grp * kPer + 2 * i;
+                if (t <= first + r) lo = __fmaf_rn(sc[static_cast<size_t>(t) * QT + r], x, lo);
+                if (2 * i + 1 < kPer && t <= first + r + 1) hi = __fmaf_rn(sc[static_cast<size_t>(t) * QT + r + 1], x, hi);
+                acc[i] = pack2(lo, hi);
+            }
         }
     }
     __syncthreads();
     if (warp < 8 && grp < kGroups) {
 #pragma unroll
-        for (int i = 0; i < kPer; ++i) qs[(grp * kPer + i) * HD + d] = __fdiv_rn(acc[i], lsum[grp * kPer + i]);
+        for (int i = 0; i < kPairs; ++i) {
+            const int r = grp * kPer + 2 * i;
+            float lo, hi;
+            unpack2(acc[i], lo, hi);
+            qs[r * HD + d] = __fdiv_rn(lo, lsum[r]);
+            if (2 * i + 1 < kPer) qs[(r + 1) * HD + d] = __fdiv_rn(hi, lsum[r + 1]);
+        }
     }
     __syncthreads();
     for (int b = warp; b < n_tok * (HD / 32); b += kPrefillAttnThreads / 32) {
@@ -394,16 +504,36 @@ __global__ void __launch_bounds__(kPrefillAttnThreads) prefill_attention_kernel(
     }
 }
 
-// act = SiLU(g) * u of every token, -> Q8_0; one warp per block of 32.
-__global__ void prefill_swiglu_quant_kernel(const float *gate_up, int n, int8_t *xq, float *xd) {
+// act = SiLU(g) * u of every token, -> Q8_0; a thread takes four values, eight neighbouring lanes a block of 32.
+__global__ void __launch_bounds__(256) prefill_swiglu_quant_kernel(const float *gate_up, int n, PairedQuant *xq, float *xd) {
     grid_dep_launch();
     grid_dep_wait();
     const size_t m = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const int ch = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = 4 * ch < n;       // n is a multiple of 32: the lanes of a block leave together
     gate_up += m * 2 * n;
-    const float v = __fmul_rn(silu_ggml(gate_up[i]), gate_up[n + i]);
-    q8_0_block_warp(v, threadIdx.x & 31, xq + m * n + (i & ~31), xd + m * (n >> 5) + (i >> 5));
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (live) {
+        const float4 g = reinterpret_cast<const float4 *>(gate_up)[ch], u = reinterpret_cast<const float4 *>(gate_up + n)[ch];
+        v[0] = __fmul_rn(silu_ggml(g.x), u.x);
+        v[1] = __fmul_rn(silu_ggml(g.y), u.y);
+        v[2] = __fmul_rn(silu_ggml(g.z), u.z);
+        v[3] = __fmul_rn(silu_ggml(g.w), u.w);
+    }
+    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    if (!live) return;
+    int q[4] = {0, 0, 0, 0};
+    if (amax != 0.0f) {
+        const float inv = __fdiv_rn(127.0f, amax);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) q[j] = max(-128, min(127, __float2int_rn(__fmul_rn(v[j], inv))));
+    }
+    const uint32_t packed = (q[0] & 0xff) | ((q[1] & 0xff) << 8) | ((q[2] & 0xff) << 16) | (static_cast<uint32_t>(q[3]) << 24);
+    *reinterpret_cast<uint32_t *>(xq + m * n + (4 * ch & ~31) + paired_place(4 * ch & 31)) = packed;
+    if ((ch & 7) == 0) xd[m * (n >> 5) + (ch >> 3)] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
 }
 
 }  // namespace wd
