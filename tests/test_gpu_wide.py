@@ -1,0 +1,50 @@
+"""Wide tiles (one 4-bit code per weight) against the CPU oracle and against the compact tiles, at every number of
+superblocks per row, for both codebooks and their mixture, in one-token and batch calls and in a stack step."""
+import numpy as np
+import pytest
+
+import oracle_lib as ol
+from warpdecode_b200 import synth
+
+pytestmark = pytest.mark.gpu
+bits = ol.fbits
+
+
+@pytest.mark.parametrize("H,F,gate,down", [(256, 256, 21, 21), (512, 512, 22, 22), (1024, 256, 22, 21), (2048, 512, 21, 21),
+                                           (4096, 1024, 21, 21), (1024, 2048, 21, 21), (2048, 512, 22, 22)])
+def test_wide_tiles_give_the_oracle_bits(oracle, monkeypatch, H, F, gate, down):
+    import warpdecode_b200 as wd
+    E, K, SF = 8, 2, 128
+    m = synth.make_moe_block(H + F, H, F, E, K, SF, gate, down)
+    rng = np.random.Generator(np.random.PCG64(H))
+    for k in ("gate", "up"):
+        m[k] = synth.random_blocks(rng, gate, E * F * H // 256)         # every code and scale, not only what the encoder picks
+    m["down"] = synth.random_blocks(rng, down, E * H * F // 256)
+    x = rng.standard_normal((3, H)).astype(np.float32)
+    want = [oracle.moe_block(m, v) for v in x]
+    size, res = {}, {}
+    for wide in ("1", "0"):
+        monkeypatch.setenv("WD_WIDE_TILES", wide)
+        eng = wd.Engine(H, F, E, K, SF, 1, expert_type=gate, down_type=down, max_tokens=3)
+        eng.load_block(0, m)
+        size[wide] = eng.slot_bytes()
+        out = eng.forward_host(0, x)
+        one = eng.forward_host(0, x[0])
+        for name in ("act", "expert_out"):
+            assert np.array_equal(bits(eng.tap(name)), bits(want[0][name])), (wide, name)
+        assert np.array_equal(bits(one), bits(want[0]["out"]))
+        for t in range(3):
+            assert np.array_equal(bits(out[t]), bits(want[t]["out"])), (wide, t)
+        res[wide] = eng.stack_step_host(x[1])
+        assert eng.device_status() == 0
+        eng.close()
+    assert size["1"] > size["0"] and np.array_equal(bits(res["1"]), bits(res["0"]))
+
+
+def test_a_pool_that_only_fits_compact_keeps_compact_tiles():
+    import warpdecode_b200 as wd
+    H, F, E, L = 512, 256, 64, 4                        # compact: 168,960 bytes per expert, 41.3 MiB in all
+    open_, tight = wd.Engine(H, F, E, 4, 128, L), wd.Engine(H, F, E, 4, 128, L, cache_mib=42)
+    assert tight.slot_count() == open_.slot_count() == E * L
+    assert tight.slot_bytes() == 168960 < open_.slot_bytes()
+    open_.close(), tight.close()

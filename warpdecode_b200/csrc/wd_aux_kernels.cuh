@@ -64,6 +64,57 @@ __global__ void repack_iq2s_kernel(const uint8_t *__restrict__ src, uint8_t *__r
     }
 }
 
+// The same two into wide tiles (wd_formats.cuh): `grid` is the packed codebook of the type.
+__global__ void repack_iq3s_wide_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, long long nblocks, long long src_stride,
+                                        long long dst_stride, const uint16_t *__restrict__ grid) {
+    const long long b = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (b >= nblocks) return;
+    const uint8_t *s = src + blockIdx.y * src_stride + b * 110;
+    uint8_t *tile = dst + blockIdx.y * dst_stride + (b >> 5) * kWide3TileBytes;
+    const int lane = static_cast<int>(b & 31);
+    *reinterpret_cast<uint16_t *>(tile + kWide3OffD + lane * 2) = static_cast<uint16_t>(s[0] | (s[1] << 8));
+    const uint8_t *qs = s + 2, *qh = s + 66, *sg = s + 74;
+    auto nibbles = [&](int i, int c) {          // four 4-bit codes, one per byte
+        const uint32_t m = grid[qs[i * 8 + c] | (((qh[i] >> c) & 1) << 8)], sign = sg[i * 4 + (c >> 1)] >> (4 * (c & 1));
+        uint32_t w = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w |= (((m >> (3 * j)) & 7u) ^ (((sign >> j) & 1u) ? 15u : 0u)) << (8 * j);
+        return w;
+    };
+    for (int i = 0; i < 8; ++i) {
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[k] = nibbles(i, k) | (nibbles(i, k + 4) << 4);
+        *reinterpret_cast<uint4 *>(tile + i * 512 + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    for (int k = 0; k < 4; ++k) tile[kWideOffSC + lane * 4 + k] = s[106 + k];
+}
+__global__ void repack_iq2s_wide_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, long long nblocks, long long src_stride,
+                                        long long dst_stride, const uint16_t *__restrict__ grid) {
+    const long long b = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (b >= nblocks) return;
+    const uint8_t *s = src + blockIdx.y * src_stride + b * 82;
+    uint8_t *tile = dst + blockIdx.y * dst_stride + (b >> 5) * kWide2TileBytes;
+    const int lane = static_cast<int>(b & 31);
+    *reinterpret_cast<uint16_t *>(tile + kWide2OffD + lane * 2) = static_cast<uint16_t>(s[0] | (s[1] << 8));
+    const uint8_t *qs = s + 2, *sg = s + 34, *qh = s + 66, *sc = s + 74;
+    auto codes = [&](int i, int c) {            // four 4-bit codes (magnitude, sign) in 16 bits; chunk c is half c & 1 of its index
+        const uint32_t m = grid[qs[i * 4 + (c >> 1)] | (((qh[i] >> (2 * (c >> 1))) & 3) << 8)] >> (8 * (c & 1));
+        const uint32_t sign = sg[i * 4 + (c >> 1)] >> (4 * (c & 1));
+        uint32_t w = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w |= (((m >> (2 * j)) & 3u) | (((sign >> j) & 1u) << 2)) << (4 * j);
+        return w;
+    };
+    for (int i = 0; i < 8; ++i) {
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[k] = codes(i, k) | (codes(i, k + 4) << 16);
+        *reinterpret_cast<uint4 *>(tile + i * 512 + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+        tile[kWideOffSC + lane * 8 + i] = sc[i];
+    }
+}
+
 // repack: ggml Q8_0 [rows][nb] blocks (34 B) -> 4-row tasks
 __global__ void repack_q8_0_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, int rows, int nb) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;

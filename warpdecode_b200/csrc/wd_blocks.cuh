@@ -192,6 +192,38 @@ __device__ __forceinline__ void iq_tile_rows(const int partial[8], float scale, 
     __syncwarp();
 }
 
+// The same for the two row lengths of the 48-layer model (eight superblocks: gate/up rows, two: down rows), without loops:
+// every value and scale of a chain is requested before the first step. Used by the wide decoders, whose integer side is
+// short enough for the dependent loads of the general form to show.
+template <int NSB>
+__device__ __forceinline__ void iq_tile_rows_fixed(const int partial[8], float scale, int lane, float *scr, float *rows_out, float post) {
+    constexpr int R = 32 / NSB, kStripe = NSB * 8 + 8;
+    float *dst = scr + (lane / NSB) * kStripe + (lane % NSB) * 8;
+    *reinterpret_cast<float4 *>(dst) = make_float4(static_cast<float>(partial[0]), static_cast<float>(partial[1]),
+                                                   static_cast<float>(partial[2]), static_cast<float>(partial[3]));
+    *reinterpret_cast<float4 *>(dst + 4) = make_float4(static_cast<float>(partial[4]), static_cast<float>(partial[5]),
+                                                       static_cast<float>(partial[6]), static_cast<float>(partial[7]));
+    float *sc = scr + R * kStripe;
+    sc[lane] = scale;
+    __syncwarp();
+#pragma unroll
+    for (int it = 0; it < R / 4; ++it) {
+        const int rr = it * 4 + (lane >> 3), c = lane & 7;
+        float v[NSB], d[NSB];
+#pragma unroll
+        for (int s = 0; s < NSB; ++s) {
+            v[s] = scr[rr * kStripe + s * 8 + c];
+            d[s] = sc[rr * NSB + s];
+        }
+        float acc = 0.0f;
+#pragma unroll
+        for (int s = 0; s < NSB; ++s) acc = __fmaf_rn(d[s], v[s], acc);
+        acc = hsum8_lanes(acc);
+        if (c == 0) rows_out[rr] = __fmul_rn(post, acc);
+    }
+    __syncwarp();
+}
+
 // One IQ3_S tile (32 blocks, lane = block) against Q8_K activations: integer partials, then the row
 // sums into rows_out. `a` / `dx` are this lane's superblock of activations and its scale. The single
 // shared copy of the decoder: gate tiles, up tiles and down tiles all come through here.
@@ -230,6 +262,53 @@ __device__ __forceinline__ void iq_tile_to_rows_any(int type, const uint8_t *til
                                                     float *scr, float *rows_out, int *partial_dump) {
     if (type == kTypeIq2s) iq2_tile_to_rows(tile, a, dx, nsb, lane, tab2, scr, rows_out, partial_dump);
     else iq3_tile_to_rows<UNROLL>(tile, a, dx, nsb, lane, lane4x2, tab3, scr, rows_out, partial_dump);
+}
+
+// ---- wide tiles (kinds kWide + type) -------------------------------------------------------------------------
+template <int UNROLL>
+__device__ __forceinline__ void wide_partials(int kind, const uint8_t *tile, int lane, const uint8_t *a, int p[8], int i0, int i1) {
+    if (kind == kWide + kTypeIq2s) wide2_partials<UNROLL>(tile, lane, a, p, i0, i1);
+    else wide3_partials<UNROLL>(tile, lane, a, p, i0, i1);
+}
+// float side of a wide tile whose integer sums are known
+__device__ __forceinline__ void wide_rows(int kind, const uint8_t *tile, const int p[8], float dx, int nsb, int lane, float *scr, float *rows_out) {
+    const float dw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(tile + wide_tile_off_d(kind - kWide) + lane * 2));
+    const float scale = __fmul_rn(dw, dx), post = iq_row_post(kind - kWide);
+    if (nsb == 8) iq_tile_rows_fixed<8>(p, scale, lane, scr, rows_out, post);
+    else if (nsb == 2) iq_tile_rows_fixed<2>(p, scale, lane, scr, rows_out, post);
+    else iq_tile_rows(p, scale, nsb, lane, scr, rows_out, post);
+}
+template <int UNROLL>
+__device__ __noinline__ void wide_tile_to_rows(int kind, const uint8_t *tile, const uint8_t *a, float dx, int nsb, int lane, float *scr,
+                                               float *rows_out) {
+    int p[8];
+    wide_partials<UNROLL>(kind, tile, lane, a, p, 0, 8);
+    wide_rows(kind, tile, p, dx, nsb, lane, scr, rows_out);
+}
+
+// What a layer kernel calls: the decoder of its pool's form. UNROLL: sub-blocks per loop iteration of the compact decoder.
+template <bool WIDE, int UNROLL>
+__device__ __forceinline__ void tile_to_rows(int kind, const uint8_t *tile, const uint8_t *a, float dx, int nsb, int lane, uint32_t lane4x2,
+                                             const uint8_t *tab3, const uint8_t *tab2, float *scr, float *rows_out) {
+    if constexpr (WIDE) wide_tile_to_rows<8>(kind, tile, a, dx, nsb, lane, scr, rows_out);
+    else iq_tile_to_rows_any<UNROLL>(kind, tile, a, dx, nsb, lane, lane4x2, tab3, tab2, scr, rows_out, nullptr);
+}
+// integer sums of sub-blocks [i0, i1)
+template <bool WIDE>
+__device__ __forceinline__ void tile_partials(int kind, const uint8_t *tile, const uint8_t *a, int lane, uint32_t lane4x2, const uint8_t *tab3,
+                                              const uint8_t *tab2, int p[8], int i0, int i1) {
+    if constexpr (WIDE) wide_partials<1>(kind, tile, lane, a, p, i0, i1);
+    else if (kind == kTypeIq2s) iq2_block_partials_range(tile, lane, a, tab2, p, i0, i1);
+    else iq3_block_partials_range(tile, lane, a, lane4x2, tab3, p, i0, i1);
+}
+template <bool WIDE>
+__device__ __forceinline__ void tile_rows(int kind, const uint8_t *tile, const int p[8], float dx, int nsb, int lane, float *scr, float *rows_out) {
+    if constexpr (WIDE) {
+        wide_rows(kind, tile, p, dx, nsb, lane, scr, rows_out);
+    } else {
+        const float dw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(tile + iq_tile_off_d(kind) + lane * 2));
+        iq_tile_rows(p, __fmul_rn(dw, dx), nsb, lane, scr, rows_out, iq_row_post(kind));
+    }
 }
 
 }  // namespace wd

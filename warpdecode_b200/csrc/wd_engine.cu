@@ -174,7 +174,9 @@ struct wd_engine {
     int n_sm = 0;
     cudaStream_t stream = nullptr;
     int nsb_h = 0, nsb_f = 0, e_first = 0, e_count = 0;
-    size_t gate_bytes = 0, down_bytes = 0, slot_bytes = 0;
+    size_t gate_bytes = 0, down_bytes = 0;      // one expert's gate (or up) and down tensor in ggml layout
+    bool wide = false;                          // the pool holds wide tiles (wd_formats.cuh)
+    size_t gate_slot = 0, down_slot = 0, slot_bytes = 0;    // the same tensors as tiles, and a slot of all three
     int64_t n_slots = 0;
     bool resident = false;
     uint8_t *pool = nullptr;
@@ -326,6 +328,26 @@ int plan_fast(wd_engine *e) {
     return WD_OK;
 }
 
+// Tile form of the pool's slots: sizes of a slot, and kind and size of a tile for the kernels.
+void set_slot_form(wd_engine *e, bool wide) {
+    const wd_config &c = e->cfg;
+    e->wide = wide;
+    const auto tensor = [&](int type, size_t blocks) {
+        return wide ? (blocks + 31) / 32 * wd::wide_tile_bytes(type) : blocks * wd::iq_block_bytes(type);
+    };
+    e->gate_slot = tensor(c.gate_type, static_cast<size_t>(c.expert_ffn) * e->nsb_h);
+    e->down_slot = tensor(c.down_type, static_cast<size_t>(c.hidden) * e->nsb_f);
+    e->slot_bytes = align_up(2 * e->gate_slot + e->down_slot, 256);
+}
+void set_tile_form(wd_engine *e) {
+    wd::MoeParams &p = e->base;
+    const wd_config &c = e->cfg;
+    p.gu_type = c.gate_type + (e->wide ? wd::kWide : 0);
+    p.d_type = c.down_type + (e->wide ? wd::kWide : 0);
+    p.gu_tile = e->wide ? wd::wide_tile_bytes(c.gate_type) : wd::iq_tile_bytes(c.gate_type);
+    p.d_tile = e->wide ? wd::wide_tile_bytes(c.down_type) : wd::iq_tile_bytes(c.down_type);
+}
+
 int plan_shared_memory(wd_engine *e) {
     wd::MoeParams &p = e->base;
     const wd_config &c = e->cfg;
@@ -337,8 +359,8 @@ int plan_shared_memory(wd_engine *e) {
         off = align_up(off + bytes, 128);
         return static_cast<unsigned>(o);
     };
-    const bool any3 = c.gate_type == WD_TYPE_IQ3_S || c.down_type == WD_TYPE_IQ3_S;
-    const bool any2 = c.gate_type == WD_TYPE_IQ2_S || c.down_type == WD_TYPE_IQ2_S;
+    const bool any3 = !e->wide && (c.gate_type == WD_TYPE_IQ3_S || c.down_type == WD_TYPE_IQ3_S);
+    const bool any2 = !e->wide && (c.gate_type == WD_TYPE_IQ2_S || c.down_type == WD_TYPE_IQ2_S);
     p.off_tab = take(any3 ? wd::kGridTableBytes : 128);
     p.off_tab2 = take(any2 ? wd::kIq2TableBytes : 128);
     p.off_xq0 = take(c.hidden);
@@ -385,6 +407,23 @@ int plan_shared_memory(wd_engine *e) {
     return WD_OK;
 }
 
+// Wide tiles (wd_formats.cuh) are the faster form wherever they can be kept: every owned expert resident, the larger pool
+// within the caller's cache_mib or (when that is open) within the free memory less 4 GiB for everything else of the
+// program, the tiles of a CTA's share within shared memory, and the generic kernels running. Otherwise compact tiles.
+void choose_slot_form(wd_engine *e) {
+    const wd_config &c = e->cfg;
+    if (!e->resident || (c.shared_ffn > 0 && find_fast_kernel(c))) return;
+    if (const char *v = std::getenv("WD_WIDE_TILES"))
+        if (v[0] == '0') return;
+    set_slot_form(e, true);
+    const size_t pool = static_cast<size_t>(e->n_slots) * e->slot_bytes;
+    size_t room = 0, total = 0;
+    if (c.cache_mib > 0) room = static_cast<size_t>(c.cache_mib) << 20;
+    else if (cudaMemGetInfo(&room, &total) == cudaSuccess) room -= std::min<size_t>(room, 4ull << 30);
+    set_tile_form(e);
+    if (pool > room || plan_shared_memory(e) != WD_OK) set_slot_form(e, false);
+}
+
 // Shared-memory plan of the batch kernel for up to cfg.max_tokens tokens. Leaves e->batch_ok false (and the batch on
 // the single-token kernel's token loop) when the geometry does not fit.
 void plan_batch(wd_engine *e) {
@@ -413,8 +452,8 @@ void plan_batch(wd_engine *e) {
         off = align_up(off + bytes, 128);
         return static_cast<unsigned>(o);
     };
-    const bool any3 = c.gate_type == WD_TYPE_IQ3_S || c.down_type == WD_TYPE_IQ3_S;
-    const bool any2 = c.gate_type == WD_TYPE_IQ2_S || c.down_type == WD_TYPE_IQ2_S;
+    const bool any3 = !e->wide && (c.gate_type == WD_TYPE_IQ3_S || c.down_type == WD_TYPE_IQ3_S);
+    const bool any2 = !e->wide && (c.gate_type == WD_TYPE_IQ2_S || c.down_type == WD_TYPE_IQ2_S);
     p.off_tab = take(any3 ? wd::kGridTableBytes : 128);
     p.off_tab2 = take(any2 ? wd::kIq2TableBytes : 128);
     {   // one token's region
@@ -504,10 +543,14 @@ int upload_f32(wd_engine *e, const float *host, size_t n, float **dev_out) {
 }
 
 // ggml blocks -> tiles for either expert format (grid.y batches of `src_stride` / `dst_stride` bytes)
-static void launch_repack_iq(int type, const uint8_t *src, uint8_t *dst, long long nblocks, long long src_stride,
+static void launch_repack_iq(const wd_engine *e, int type, const uint8_t *src, uint8_t *dst, long long nblocks, long long src_stride,
                              long long dst_stride, unsigned batches, cudaStream_t s) {
     const dim3 grid(static_cast<unsigned>((nblocks + 127) / 128), batches);
-    if (type == WD_TYPE_IQ2_S) wd::repack_iq2s_kernel<<<grid, 128, 0, s>>>(src, dst, nblocks, src_stride, dst_stride);
+    if (e->wide && type == WD_TYPE_IQ2_S)
+        wd::repack_iq2s_wide_kernel<<<grid, 128, 0, s>>>(src, dst, nblocks, src_stride, dst_stride, e->grid2_packed);
+    else if (e->wide)
+        wd::repack_iq3s_wide_kernel<<<grid, 128, 0, s>>>(src, dst, nblocks, src_stride, dst_stride, e->grid_packed);
+    else if (type == WD_TYPE_IQ2_S) wd::repack_iq2s_kernel<<<grid, 128, 0, s>>>(src, dst, nblocks, src_stride, dst_stride);
     else wd::repack_iq3s_kernel<<<grid, 128, 0, s>>>(src, dst, nblocks, src_stride, dst_stride);
 }
 
@@ -517,9 +560,9 @@ int repack_expert_into_slot(wd_engine *e, const uint8_t *g, const uint8_t *u, co
     uint8_t *dst = e->pool + static_cast<size_t>(slot) * e->slot_bytes;
     const long long nb_gu = static_cast<long long>(e->cfg.expert_ffn) * e->nsb_h;
     const long long nb_d = static_cast<long long>(e->cfg.hidden) * e->nsb_f;
-    launch_repack_iq(e->cfg.gate_type, g, dst, nb_gu, 0, 0, 1, s);
-    launch_repack_iq(e->cfg.gate_type, u, dst + e->gate_bytes, nb_gu, 0, 0, 1, s);
-    launch_repack_iq(e->cfg.down_type, d, dst + 2 * e->gate_bytes, nb_d, 0, 0, 1, s);
+    launch_repack_iq(e, e->cfg.gate_type, g, dst, nb_gu, 0, 0, 1, s);
+    launch_repack_iq(e, e->cfg.gate_type, u, dst + e->gate_slot, nb_gu, 0, 0, 1, s);
+    launch_repack_iq(e, e->cfg.down_type, d, dst + 2 * e->gate_slot, nb_d, 0, 0, 1, s);
     WD_CUDA(cudaGetLastError());
     return WD_OK;
 }
@@ -548,6 +591,13 @@ int sync_layer_table(wd_engine *e, cudaStream_t s) {
     WD_CUDA(cudaStreamSynchronize(s));      // `host` goes out of scope
     e->layer_table_dirty = false;
     return WD_OK;
+}
+
+const void *layer_kernel(const wd_engine *e) {
+    return e->wide ? reinterpret_cast<const void *>(wd::moe_layer_kernel<true>) : reinterpret_cast<const void *>(wd::moe_layer_kernel<false>);
+}
+const void *batch_kernel(const wd_engine *e) {
+    return e->wide ? reinterpret_cast<const void *>(wd::moe_batch_kernel<true>) : reinterpret_cast<const void *>(wd::moe_batch_kernel<false>);
 }
 
 // Layers [begin, end) in one cooperative launch.
@@ -594,8 +644,7 @@ int launch_layers(wd_engine *e, int begin, int end, const float *x, float *resid
         p.stamps = e->profiling ? e->stamps : nullptr;
         p.select_only = select_only ? 1 : 0;
         void *args[] = {&p};
-        WD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(wd::moe_layer_kernel), dim3(e->n_sm),
-                                            dim3(wd::kThreads), args, e->smem_bytes, s));
+        WD_CUDA(cudaLaunchCooperativeKernel(layer_kernel(e), dim3(e->n_sm), dim3(wd::kThreads), args, e->smem_bytes, s));
     }
     // the kernel advances the device's epoch by the length of its sequence (layers, or the tokens of a batch)
     e->epoch += static_cast<uint32_t>(n_tokens > 1 && !e->fast_fn ? n_tokens : end - begin);
@@ -631,8 +680,7 @@ int launch_batch(wd_engine *e, int layer, const float *x, float *out, int n_toke
     p.routed = e->routed;
     p.stamps = e->profiling ? e->stamps : nullptr;
     void *args[] = {&p};
-    WD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(wd::moe_batch_kernel), dim3(e->n_sm), dim3(wd::kThreads), args,
-                                        e->batch_smem, s));
+    WD_CUDA(cudaLaunchCooperativeKernel(batch_kernel(e), dim3(e->n_sm), dim3(wd::kThreads), args, e->batch_smem, s));
     e->epoch += 1u;         // the whole batch carries one tag
     e->last_parity = static_cast<int>(e->epoch & 1u);
     e->last_tokens = n_tokens;
@@ -929,7 +977,7 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
     e->e_first = c.ep_rank * e->e_count;
     e->gate_bytes = static_cast<size_t>(c.expert_ffn) * e->nsb_h * wd::iq_block_bytes(c.gate_type);
     e->down_bytes = static_cast<size_t>(c.hidden) * e->nsb_f * wd::iq_block_bytes(c.down_type);
-    e->slot_bytes = align_up(2 * e->gate_bytes + e->down_bytes, 256);
+    set_slot_form(e, false);
     const int64_t owned = static_cast<int64_t>(e->e_count) * c.n_layers;
     if (c.cache_mib <= 0) {
         e->n_slots = owned;
@@ -941,6 +989,7 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
         }
     }
     e->resident = e->n_slots == owned;
+    choose_slot_form(e);
     if (const char *v = std::getenv("WD_THRESHOLD_SELECT")) e->threshold_select = v[0] != '0';
     int rc = WD_OK;
     auto bail = [&](int code) {
@@ -1026,11 +1075,10 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
     p.w_scale = c.w_scale; p.eps = c.rms_eps > 0 ? c.rms_eps : 1e-6f;
     p.inv_h = (H & (H - 1)) == 0 ? 1.0 / static_cast<double>(H) : 0.0;
     p.pool = e->pool; p.slot_bytes = e->slot_bytes;
-    p.gate_off = 0; p.up_off = static_cast<unsigned>(e->gate_bytes); p.down_off = static_cast<unsigned>(2 * e->gate_bytes);
+    p.gate_off = 0; p.up_off = static_cast<unsigned>(e->gate_slot); p.down_off = static_cast<unsigned>(2 * e->gate_slot);
     p.grid_packed = e->grid_packed;
     p.grid2_packed = e->grid2_packed;
-    p.gu_type = c.gate_type; p.d_type = c.down_type;
-    p.gu_tile = wd::iq_tile_bytes(c.gate_type); p.d_tile = wd::iq_tile_bytes(c.down_type);
+    set_tile_form(e);
     p.ids = e->ids; p.weights = e->weights; p.routed = e->routed;
     p.t_logits = e->tagged + tw_logits; p.t_shared_act = e->tagged + tw_shact; p.t_shared_gate = e->tagged + tw_shgate;
     p.t_act = e->tagged + tw_act; p.t_expert_out = e->tagged + tw_eo; p.t_shared_down = e->tagged + tw_shdown;
@@ -1043,14 +1091,14 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
     p.host_status = e->host_status;
     { int t2 = F * e->nsb_h / 32, t3 = H * e->nsb_f / 32; p.t2_log2 = 0; while ((1 << p.t2_log2) < t2) ++p.t2_log2; p.t3_log2 = 0; while ((1 << p.t3_log2) < t3) ++p.t3_log2; }
     if ((rc = plan_shared_memory(e)) != WD_OK) return bail(rc);
-    cudaError_t ae = cudaFuncSetAttribute(wd::moe_layer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(e->smem_bytes));
+    // all of an SM, whatever this engine needs: the attribute belongs to the function, and engines of several sizes live side by side
+    cudaError_t ae = cudaFuncSetAttribute(layer_kernel(e), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (ae != cudaSuccess) {
         fail(WD_E_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ae));
         return bail(WD_E_CUDA);
     }
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wd::moe_layer_kernel, wd::kThreads, e->smem_bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, layer_kernel(e), wd::kThreads, e->smem_bytes);
     if (occ < 1) {
         fail(WD_E_INVALID, "the layer kernel does not fit one CTA per SM with this geometry");
         return bail(WD_E_INVALID);
@@ -1099,9 +1147,9 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
         cudaError_t be = cudaMalloc(&e->btagged, w_end * sizeof(wd::tagged_t));
         if (be == cudaSuccess) be = cudaMemset(e->btagged, 0, w_end * sizeof(wd::tagged_t));
         if (be == cudaSuccess)
-            be = cudaFuncSetAttribute(wd::moe_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(e->batch_smem));
+            be = cudaFuncSetAttribute(batch_kernel(e), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         int bocc = 0;
-        if (be == cudaSuccess) be = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bocc, wd::moe_batch_kernel, wd::kThreads, e->batch_smem);
+        if (be == cudaSuccess) be = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bocc, batch_kernel(e), wd::kThreads, e->batch_smem);
         if (be != cudaSuccess) {
             fail(WD_E_CUDA, std::string("setting up the batch kernel: ") + cudaGetErrorString(be));
             return bail(WD_E_CUDA);
@@ -1290,9 +1338,9 @@ static int load_layer_resident(wd_engine *e, int layer) {
         WD_CUDA(cudaMemcpyAsync(st, pin, static_cast<size_t>(n) * one, cudaMemcpyHostToDevice, s));
         uint8_t *dst = e->pool + static_cast<size_t>(layer * e->e_count + x0) * e->slot_bytes;
         const long long so = static_cast<long long>(one), sb = static_cast<long long>(e->slot_bytes);
-        launch_repack_iq(e->cfg.gate_type, st, dst, nb_gu, so, sb, n, s);
-        launch_repack_iq(e->cfg.gate_type, st + gb, dst + gb, nb_gu, so, sb, n, s);
-        launch_repack_iq(e->cfg.down_type, st + 2 * gb, dst + 2 * gb, nb_d, so, sb, n, s);
+        launch_repack_iq(e, e->cfg.gate_type, st, dst, nb_gu, so, sb, n, s);
+        launch_repack_iq(e, e->cfg.gate_type, st + gb, dst + e->gate_slot, nb_gu, so, sb, n, s);
+        launch_repack_iq(e, e->cfg.down_type, st + 2 * gb, dst + 2 * e->gate_slot, nb_d, so, sb, n, s);
         WD_CUDA(cudaGetLastError());
         WD_CUDA(cudaEventRecord(e->load_done[half], s));
         used[half] = true;
@@ -1386,9 +1434,9 @@ int wd_set_experts_device(wd_engine *e, int layer, const void *gate, const void 
         const long long nb_d = static_cast<long long>(e->cfg.hidden) * e->nsb_f;
         const long long gb = static_cast<long long>(e->gate_bytes), db = static_cast<long long>(e->down_bytes);
         const long long sb = static_cast<long long>(e->slot_bytes);
-        launch_repack_iq(e->cfg.gate_type, g + e->e_first * gb, dst, nb_gu, gb, sb, e->e_count, e->stream);
-        launch_repack_iq(e->cfg.gate_type, u + e->e_first * gb, dst + gb, nb_gu, gb, sb, e->e_count, e->stream);
-        launch_repack_iq(e->cfg.down_type, d + e->e_first * db, dst + 2 * gb, nb_d, db, sb, e->e_count, e->stream);
+        launch_repack_iq(e, e->cfg.gate_type, g + e->e_first * gb, dst, nb_gu, gb, sb, e->e_count, e->stream);
+        launch_repack_iq(e, e->cfg.gate_type, u + e->e_first * gb, dst + e->gate_slot, nb_gu, gb, sb, e->e_count, e->stream);
+        launch_repack_iq(e, e->cfg.down_type, d + e->e_first * db, dst + 2 * e->gate_slot, nb_d, db, sb, e->e_count, e->stream);
         WD_CUDA(cudaGetLastError());
     }
     for (int x = 0; x < e->e_count; ++x) {

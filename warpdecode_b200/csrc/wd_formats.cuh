@@ -25,6 +25,19 @@
 //   D   off 2560: [lane][2 B]               f16 block scale
 // Its codebook (1024 entries of eight magnitudes) is a plain 8 KB shared-memory table.
 //
+// WIDE tiles: what a pool that holds every expert keeps instead, when it fits. The compact forms above spend 16 instructions
+// on four weights (index bits, codebook lookup, sign mask, negate, select, dp4a, scale); with one 4-bit code per weight the
+// codebooks are gone and four weights take 3.5. An IQ3_S weight is +-(2 m + 1), m = 0..7: with n = m or -m - 1 it is
+// 2 n + 1, so the nibble n at the top of its byte with 8 below it IS 8 * weight as an int8. An IQ2_S weight is one of
+// six values, which one prmt selects for four nibbles at once. Measured (one SM, tiles in shared memory): see
+// wide_tile_to_rows. The price is HBM bytes: 134 instead of 110 per 256 weights (IQ3_S), 138 instead of 82 (IQ2_S); the
+// expert products of a token are bound by instruction issue, not by these bytes. A capped cache keeps the compact tiles
+// (a slot then holds the most experts per byte, and a miss costs a repack of the bytes it streams).
+//   Q   off    0: [sub-block i=0..7][lane][16 B] word k (0..3) holds chunks k and k + 4: IQ3_S in the low and the high nibbles
+//                                                of its bytes, IQ2_S in its low and its high 16 bits (nibble j = value j)
+//   SC  off 4096: [lane][4 B or 8 B]             scale nibbles as in the compact tile
+//   D   off 4224 (IQ3_S) / 4352 (IQ2_S): [lane][2 B] f16 block scale
+//
 // Q8_0 "task" = 4 consecutive rows of nb = cols / 32 blocks (nb a multiple of 4):
 //   QS  [group g = b/4][row r][chunk-lane l][16 B], word i = values 4l..4l+3 of block 4g+i
 //   D   off nb*128: [row r][nb] f16
@@ -46,6 +59,11 @@ constexpr int kTypeIq3s = 21, kTypeIq2s = 22; // ggml type ids (src/gguf.hpp:26-
 __host__ __device__ constexpr int iq_tile_bytes(int type) { return type == kTypeIq2s ? kIq2TileBytes : kIq3TileBytes; }
 __host__ __device__ constexpr int iq_block_bytes(int type) { return type == kTypeIq2s ? 82 : 110; }
 __host__ __device__ constexpr int iq_tile_off_d(int type) { return type == kTypeIq2s ? kIq2OffD : kIq3OffD; }
+// tile kinds of the wide form: the ggml type + kWide
+constexpr int kWide = 100;
+constexpr int kWideOffSC = 4096, kWide3OffD = 4224, kWide3TileBytes = 4288, kWide2OffD = 4352, kWide2TileBytes = 4416;
+__host__ __device__ constexpr int wide_tile_bytes(int type) { return type == kTypeIq2s ? kWide2TileBytes : kWide3TileBytes; }
+__host__ __device__ constexpr int wide_tile_off_d(int type) { return type == kTypeIq2s ? kWide2OffD : kWide3OffD; }
 // factor applied to a finished row sum (ggml's IQ2_S row dot ends with * 0.125, src/qwen38_cpu_moe.cuh:298-335)
 __host__ __device__ constexpr float iq_row_post(int type) { return type == kTypeIq2s ? 0.125f : 1.0f; }
 constexpr int kActSbStride = 272;             // 256 int8 + 16 pad: the 8 superblocks of a row hit 8 bank groups
@@ -183,6 +201,53 @@ __device__ __forceinline__ void iq2_block_partials_range(const uint8_t *tile, in
     const uint4 *av = reinterpret_cast<const uint4 *>(a);
 #pragma unroll 1
     for (int i = i0; i < i1; ++i) iq2_subblock(tile, h, i, lane, av[2 * i], av[2 * i + 1], tab2, partial);
+}
+
+// ---- wide tiles ----------------------------------------------------------------------------------------
+// partial[c] of sub-blocks [i0, i1) of this lane's block, exactly the integers of the compact decoders.
+template <int UNROLL>
+__device__ __forceinline__ void wide3_partials(const uint8_t *tile, int lane, const uint8_t *a, int partial[8], int i0, int i1) {
+    const uint32_t sc = *reinterpret_cast<const uint32_t *>(tile + kWideOffSC + lane * 4);
+    const uint4 *av = reinterpret_cast<const uint4 *>(a);
+    const uint4 *qv = reinterpret_cast<const uint4 *>(tile) + lane;
+    int p8[8];              // eight times the sums
+#pragma unroll
+    for (int c = 0; c < 8; ++c) p8[c] = 0;
+#pragma unroll(UNROLL)
+    for (int i = i0; i < i1; ++i) {
+        const uint4 q = qv[i * 32], lo = av[2 * i], hi = av[2 * i + 1];
+        const int ls = 1 + 2 * static_cast<int>((sc >> (4 * i)) & 15u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t w = word_of(q, k);
+            p8[k] += dp4a_s8(static_cast<int>(((w << 4) & 0xf0f0f0f0u) | 0x08080808u), static_cast<int>(word_of(lo, k)), 0) * ls;
+            p8[k + 4] += dp4a_s8(static_cast<int>((w & 0xf0f0f0f0u) | 0x08080808u), static_cast<int>(word_of(hi, k)), 0) * ls;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) partial[c] = p8[c] >> 3;
+}
+
+template <int UNROLL>
+__device__ __forceinline__ void wide2_partials(const uint8_t *tile, int lane, const uint8_t *a, int partial[8], int i0, int i1) {
+    const uint2 sc = *reinterpret_cast<const uint2 *>(tile + kWideOffSC + lane * 8);
+    const uint4 *av = reinterpret_cast<const uint4 *>(a);
+    const uint4 *qv = reinterpret_cast<const uint4 *>(tile) + lane;
+    const uint32_t pos = 0x3b2b1908u, neg = 0xc5d5e7f8u;       // 8, 25, 43 (59) and their negatives: the value of a 3-bit code
+#pragma unroll
+    for (int c = 0; c < 8; ++c) partial[c] = 0;
+#pragma unroll(UNROLL)
+    for (int i = i0; i < i1; ++i) {
+        const uint4 q = qv[i * 32], lo = av[2 * i], hi = av[2 * i + 1];
+        const uint32_t scb = ((i & 4) ? sc.y : sc.x) >> (8 * (i & 3));
+        const int ls_lo = 1 + 2 * static_cast<int>(scb & 15u), ls_hi = 1 + 2 * static_cast<int>((scb >> 4) & 15u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t w = word_of(q, k);
+            partial[k] += dp4a_s8(static_cast<int>(prmt(pos, neg, w)), static_cast<int>(word_of(lo, k)), 0) * ls_lo;
+            partial[k + 4] += dp4a_s8(static_cast<int>(prmt(pos, neg, w >> 16)), static_cast<int>(word_of(hi, k)), 0) * ls_hi;
+        }
+    }
 }
 
 // Full block.

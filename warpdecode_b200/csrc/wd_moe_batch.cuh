@@ -88,6 +88,7 @@ __device__ __forceinline__ float pick4(const float (&a)[kMaxTokens], int t) {
     return t == 0 ? a[0] : t == 1 ? a[1] : t == 2 ? a[2] : a[3];
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_constant__ BatchParams P) {
     uint8_t *sm = wd_smem;
     uint8_t *tab = sm + P.off_tab, *tab2 = sm + P.off_tab2;
@@ -224,8 +225,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
             bulk_load(gate_vec_stage, L.sh_gate_vec, static_cast<unsigned>(P.H) * 4u, &bars[bar_gv]);
         }
     }
-    if (P.gu_type == kTypeIq3s || P.d_type == kTypeIq3s) build_grid_table(tab, P.grid_packed);      // first needed by the tiles
-    if (P.gu_type == kTypeIq2s || P.d_type == kTypeIq2s) build_iq2_table(tab2, P.grid2_packed);
+    if constexpr (!WIDE) {
+        if (P.gu_type == kTypeIq3s || P.d_type == kTypeIq3s) build_grid_table(tab, P.grid_packed);      // first needed by the tiles
+        if (P.gu_type == kTypeIq2s || P.d_type == kTypeIq2s) build_iq2_table(tab2, P.grid2_packed);
+    }
 
     WD_BSTAMP(1);
     // ---- the T activations: Q8_0 (router, shared expert) and Q8_K (routed experts) ----------------------------
@@ -517,8 +520,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
                 const int up = (d >> 21) & 1;
                 float *buf = pairbuf + aux * 2 * R2;
                 wait_slot();
-                iq_tile_to_rows_any<8>(P.gu_type, tile_mem, xk_of(t) + sb2 * kActSbStride, xdk_of(t)[sb2], P.nsb_h, lane, lane4x2, tab,
-                                    tab2, scr, buf + up * R2, nullptr);
+                tile_to_rows<WIDE, 8>(P.gu_type, tile_mem, xk_of(t) + sb2 * kActSbStride, xdk_of(t)[sb2], P.nsb_h, lane, lane4x2, tab,
+                                      tab2, scr, buf + up * R2);
                 reissue();
                 int second = 0;
                 if (lane == 0) {
@@ -540,8 +543,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
                 }
                 const int ab = aux + sb3;
                 wait_slot();
-                iq_tile_to_rows_any<8>(P.d_type, tile_mem, actk + ab * kActSbStride, actd[ab], P.nsb_f, lane, lane4x2, tab, tab2, scr,
-                                    rows_a, nullptr);
+                tile_to_rows<WIDE, 8>(P.d_type, tile_mem, actk + ab * kActSbStride, actd[ab], P.nsb_f, lane, lane4x2, tab, tab2, scr,
+                                      rows_a);
                 reissue();
 #pragma unroll 1
                 for (int rr = lane; rr < R3; rr += 32)

@@ -71,7 +71,7 @@ struct MoeParams {
     unsigned gate_off, up_off, down_off;        // offsets of the three matrices inside a slot
     const uint16_t *grid_packed; // packed IQ3_S codebook in global memory
     const uint16_t *grid2_packed;// packed IQ2_S codebook
-    int gu_type, d_type;         // ggml type of the gate/up tensors and of the down tensor (IQ3_S or IQ2_S)
+    int gu_type, d_type;         // tile kind of the gate/up tensors and of the down tensor: ggml type (IQ3_S or IQ2_S), + kWide
     unsigned gu_tile, d_tile;    // bytes of one tile of 32 blocks of each
     // activations
     const float *x;              // [H] (used when residual == nullptr)
@@ -220,6 +220,8 @@ __device__ __forceinline__ void issue_phase1_copies(const MoeParams &P, const La
 
 extern __shared__ __align__(128) uint8_t wd_smem[];
 
+// WIDE: the pool holds wide tiles (wd_formats.cuh), gu_type / d_type are their kinds and no codebook is needed.
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads, 1) moe_layer_kernel(const __grid_constant__ MoeParams P) {
     uint8_t *sm = wd_smem;
     uint8_t *tab = sm + P.off_tab;                                   // IQ3_S codebook, lane-private copies
@@ -270,8 +272,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_layer_kernel(const __grid_con
         mbar_fence_init();
     }
     if (cta == 0 && tid == 0) P.sync[5] = smem_u32(bars);      // so that a copy timeout can be reported by barrier index
-    if (P.gu_type == kTypeIq3s || P.d_type == kTypeIq3s) build_grid_table(tab, P.grid_packed);   // first needed in phase 2
-    if (P.gu_type == kTypeIq2s || P.d_type == kTypeIq2s) build_iq2_table(tab2, P.grid2_packed);
+    if constexpr (!WIDE) {
+        if (P.gu_type == kTypeIq3s || P.d_type == kTypeIq3s) build_grid_table(tab, P.grid_packed);   // first needed in phase 2
+        if (P.gu_type == kTypeIq2s || P.d_type == kTypeIq2s) build_iq2_table(tab2, P.grid2_packed);
+    }
     __syncthreads();
 
     const int seq_end = P.n_tokens > 1 ? P.layer_begin + P.n_tokens : P.layer_end;   // end of the launch's sequence
