@@ -381,10 +381,11 @@ int plan_shared_memory(wd_engine *e) {
     const int t2 = c.expert_ffn / r_h, t3 = c.hidden / r_f;
     p.n1r = (n_rt + ncta - 1) / ncta;
     p.n1s = (n_st + ncta - 1) / ncta;
-    p.n2 = (c.top_k * t2 + ncta - 1) / ncta;
+    const int tcta = e->wide ? ncta - 1 : ncta;     // with wide tiles the last CTA proves the selection instead of taking tiles
+    p.n2 = (c.top_k * t2 + tcta - 1) / tcta;
     const int n_sd = c.shared_ffn > 0 ? c.hidden / 4 : 0;
     // a CTA takes every ncta-th entry of [tiles | shared-down tasks]: at most ceil(len / ncta) of each part
-    p.n3 = (c.top_k * t3 + ncta - 1) / ncta;
+    p.n3 = (c.top_k * t3 + tcta - 1) / tcta;
     p.nsd = (n_sd + ncta - 1) / ncta;
     if (p.n1r + p.n1s + p.n2 + p.n3 + p.nsd > wd::kMaxBars - 2)
         return fail(WD_E_INVALID, "geometry needs more staging slots per CTA than the kernel supports");
@@ -397,9 +398,10 @@ int plan_shared_memory(wd_engine *e) {
                                              static_cast<size_t>(p.n2) * 2 * p.gu_tile),
                                     static_cast<size_t>(c.top_k) * c.expert_ffn * 4);
     p.off_stage_a = take(stage_a);
-    // stage B also holds the F32 shared gate vector during phase 1
-    p.off_stage_b = take(std::max(static_cast<size_t>(p.n3) * p.d_tile + static_cast<size_t>(p.nsd) * nbs * 136,
-                                  static_cast<size_t>(c.hidden) * 4));
+    // stage B also holds the F32 shared gate vector during phase 1; with wide tiles the shared-down tasks travel beside it
+    const size_t tiles_b = static_cast<size_t>(p.n3) * p.d_tile, gate_vec = static_cast<size_t>(c.hidden) * 4;
+    p.sd_off = static_cast<unsigned>(e->wide ? align_up(std::max(tiles_b, gate_vec), 128) : tiles_b);
+    p.off_stage_b = take(std::max(p.sd_off + static_cast<size_t>(p.nsd) * nbs * 136, gate_vec));
     e->smem_bytes = off;
     if (e->smem_bytes > 227 * 1024)
         return fail(WD_E_INVALID, "geometry needs " + std::to_string(e->smem_bytes) +
@@ -1041,10 +1043,10 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
     auto up16 = [](size_t w) { return (w + 15) / 16 * 16; };
     const size_t tw_logits = 0, tw_shact = up16(tw_logits + 2 * static_cast<size_t>(E)),
                  tw_shgate = up16(tw_shact + 2 * static_cast<size_t>(SF)), tw_act = tw_shgate + 32,
-                 tw_eo = up16(tw_act + 2 * static_cast<size_t>(K) * F),
+                 tw_eo = up16(tw_act + 4 * static_cast<size_t>(K) * F),
                  tw_shdown = up16(tw_eo + 2 * static_cast<size_t>(K) * H), tw_res = up16(tw_shdown + 2 * static_cast<size_t>(H)),
                  tw_prog = up16(tw_res + 2 * static_cast<size_t>(H)), tw_left = up16(tw_prog + static_cast<size_t>(e->n_sm)),
-                 tw_end = tw_left + 16;
+                 tw_sel = tw_left + 16, tw_end = tw_sel + 128;
     e->tagged_words = tw_end;
     WD_TRY(cudaMalloc(&e->tagged, e->tagged_words * sizeof(wd::tagged_t)));
     WD_TRY(cudaMemset(e->tagged, 0, e->tagged_words * sizeof(wd::tagged_t)));
@@ -1086,6 +1088,7 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
     e->tagged_eo_offset = tw_eo;
     e->tagged_left_offset = tw_left;
     p.t_peer_left = e->tagged + tw_left;
+    p.t_sel = e->tagged + tw_sel;
     p.n_peers = 0;
     p.sync = e->sync;
     p.host_status = e->host_status;

@@ -83,7 +83,8 @@ struct MoeParams {
     tagged_t *t_logits;          // [2][E]
     tagged_t *t_shared_act;      // [2][SF]
     tagged_t *t_shared_gate;     // [2][1]
-    tagged_t *t_act;             // [2][K][F]
+    tagged_t *t_act;             // [2][K][F], then [2][K][F] for a layer whose picked ids were replaced (WIDE)
+    tagged_t *t_sel;             // [2][64] the selection as the proof CTA publishes it (WIDE)
     tagged_t *t_expert_out;      // [2][K][H]
     tagged_t *t_shared_down;     // [2][H]
     tagged_t *t_residual;        // [2][H]   updated residual = next layer's input
@@ -107,6 +108,7 @@ struct MoeParams {
     // shared memory plan (byte offsets from the dynamic shared base; all 128-byte aligned)
     unsigned off_tab, off_tab2, off_xq0, off_xd0, off_xk, off_xdk, off_actk, off_actd, off_shq, off_shd,
         off_misc, off_scr, off_bar, off_slots, off_rowbuf, off_stage_a, off_stage_b;
+    unsigned sd_off;             // the shared-down tasks inside stage B
     unsigned scr_bytes;          // per-warp transposition scratch
     unsigned scr_rows;           // float offset of the two 32-float row buffers inside it
     unsigned n1r, n1s, n2, n3, nsd;   // staging slots per CTA: router tasks, shared g/u tasks, phase-2 units,
@@ -317,6 +319,21 @@ __global__ void __launch_bounds__(kThreads, 1) moe_layer_kernel(const __grid_con
     if (warp == 0) {
         fence_proxy_async();        // the staging buffers were last read by ordinary loads (previous layer)
         issue_phase1_copies(P, L, lane, cta, ncta, rt_bytes, stage_a, stage_b, slot_tab, bars, layer == P.layer_begin, true);
+    }
+    // WIDE: the shared expert's down rows do not depend on the picked experts: they travel now, not with the tiles
+    if (WIDE && warp == 1) {
+        const unsigned sd_bytes = static_cast<unsigned>(nbs) * 136u;
+        const int n_sd = P.SF > 0 ? (P.H >> 2) : 0, bar_sd = P.n1r + P.n1s + P.n2 + P.n3;
+        uint8_t *stage_sd = stage_b + P.sd_off;
+        for (int s = lane; s < static_cast<int>(P.nsd); s += 32) {
+            const int t = cta + s * ncta;
+            if (t < n_sd) {
+                mbar_expect_tx(&bars[bar_sd + s], sd_bytes);
+                bulk_load(stage_sd + s * sd_bytes, L.sh_down + static_cast<size_t>(t) * sd_bytes, sd_bytes, &bars[bar_sd + s]);
+            } else {
+                mbar_arrive(&bars[bar_sd + s]);
+            }
+        }
     }
     WD_STAMP(1);
 
