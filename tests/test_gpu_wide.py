@@ -48,3 +48,29 @@ def test_a_pool_that_only_fits_compact_keeps_compact_tiles():
     assert tight.slot_count() == open_.slot_count() == E * L
     assert tight.slot_bytes() == 168960 < open_.slot_bytes()
     open_.close(), tight.close()
+
+
+@pytest.mark.parametrize("H,F,gate,up,down,f32", [(256 * 3, 64, 21, 21, 20, False), (2560, 640, 22, 22, 20, True), (1280, 192, 21, 22, 20, True),
+                                                  (768, 768, 22, 22, 21, True), (4096, 256, 21, 21, 22, True), (1792, 512, 22, 21, 22, False)])
+def test_wide_rows_of_the_plain_layout_path(oracle, monkeypatch, H, F, gate, up, down, f32):
+    import warpdecode_b200 as wd
+    E, K, SF = 8, 3, 128
+    m = synth.make_moe_block(H + F, H, F, E, K, SF, gate, down, router_f32=f32)
+    m["up_type"] = up
+    rng = np.random.Generator(np.random.PCG64(F))
+    m["gate"], m["up"] = (synth.random_blocks(rng, t, E * F * H // 256) for t in (gate, up))
+    m["down"] = synth.random_blocks(rng, down, E * H * F // (32 if down == 20 else 256))
+    x = rng.standard_normal((2, H)).astype(np.float32)
+    want = [oracle.moe_block(m, v) for v in x]
+    for wide in ("1", "0"):
+        monkeypatch.setenv("WD_WIDE_TILES", wide)
+        eng = wd.Engine(H, F, E, K, SF, 1, expert_type=gate, down_type=down, max_tokens=2, router_f32=f32)
+        eng.load_block(0, m)
+        assert eng.kernel_name() == "plain_gate_up_kernel"
+        out = eng.forward_host(0, x)
+        for t in range(2):
+            for name in ("act", "expert_out"):
+                assert np.array_equal(bits(eng.tap(name, t)), bits(want[t][name])), (wide, t, name)
+            assert np.array_equal(bits(out[t]), bits(want[t]["out"])), (wide, t)
+        assert eng.device_status() == 0
+        eng.close()

@@ -26,6 +26,7 @@
 #include "wd_dense_token.cuh"
 #include "wd_dense_prefill.cuh"
 #include "wd_plain_moe.cuh"
+#include "wd_plain_wide.cuh"
 #include "wd_grids.h"
 
 namespace {
@@ -911,6 +912,7 @@ int check_device_status(wd_engine *e) {
         if (e->xbuf) cudaMemset(e->xbuf, 0, e->xbuf_words * sizeof(wd::tagged_t));
         cudaDeviceSynchronize();                // the next launch runs on a stream that is not ordered behind these
         e->epoch = 0;
+        if (e->host_status) *e->host_status = 0u;
         return fail(WD_E_DEVICE, "kernel raised status " + std::to_string(st) +
                                      " (1 wait timeout, 2 copy timeout, 4 expert without slot, 8 geometry, "
                                      "16 exchange word overwritten before it was read)" + bar);
@@ -1579,7 +1581,7 @@ int wd_stack_step_host(wd_engine *e, const float *in_host, float *out_host) {
     WD_CUDA(cudaMemcpyAsync(pin + e->cfg.hidden, e->residual_buf, bytes, cudaMemcpyDeviceToHost, e->stream));
     WD_CUDA(cudaStreamSynchronize(e->stream));
     memcpy(out_host, pin + e->cfg.hidden, bytes);
-    // the last CTA of every launch leaves the status word in pinned host memory: no copy to read it.
+    // the last CTA of a launch that raised a status leaves it in pinned host memory: no copy to read it.
     // (Letting the kernel read and write the residual in pinned memory directly was measured slower: every CTA
     // fetches the whole vector over PCIe.)
     if (!e->plain && *e->host_status == 0u) return WD_OK;
@@ -1862,6 +1864,7 @@ int wd_reset_exchange(wd_engine *e) {
     if (e->xbuf) WD_CUDA(cudaMemset(e->xbuf, 0, e->xbuf_words * sizeof(wd::tagged_t)));
     WD_CUDA(cudaDeviceSynchronize());           // the next launch runs on a stream that is not ordered behind these
     e->epoch = 0;
+    if (e->host_status) *e->host_status = 0u;
     return WD_OK;
 }
 
@@ -1878,6 +1881,7 @@ int wd_device_status(wd_engine *e, int *status) {
         if (e->xbuf) WD_CUDA(cudaMemset(e->xbuf, 0, e->xbuf_words * sizeof(wd::tagged_t)));
         WD_CUDA(cudaDeviceSynchronize());       // the next launch runs on a stream that is not ordered behind these
         e->epoch = 0;
+        if (e->host_status) *e->host_status = 0u;
     }
     return WD_OK;
 }

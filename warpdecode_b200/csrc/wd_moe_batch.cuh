@@ -614,7 +614,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
             P.sync[9] = 0u;
             P.sync[8] = epoch + 1u;
             __threadfence();
-            if (P.host_status) *P.host_status = *reinterpret_cast<volatile unsigned *>(err);
+            const unsigned st = *reinterpret_cast<volatile unsigned *>(err);
+            if (P.host_status && st) *P.host_status = st;      // a write over PCIe that the launch would wait for: only when there is news
         }
     }
 }

@@ -419,7 +419,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_layer_kernel(const __grid_con
             __threadfence();
             for (int p = 0; p < P.n_peers; ++p)
                 st_tagged_sys_release(P.peer_left_out[p], 0.0f, epoch + static_cast<uint32_t>(seq_done));
-            if (P.host_status) *P.host_status = *reinterpret_cast<volatile unsigned *>(err);
+            const unsigned st = *reinterpret_cast<volatile unsigned *>(err);
+            if (P.host_status && st) *P.host_status = st;      // a write over PCIe that the launch would wait for: only when there is news
         }
     }
 }
