@@ -220,6 +220,44 @@ __device__ __forceinline__ float plain_rows4_iq4nl_wide(const uint8_t *rows, siz
     return __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 1));
 }
 
+// plain_quantize_q8_0_cta with four groups of a thread in flight: its chain of shuffles and divisions is 0.6 us, and the
+// activations of ten slots (6400 values) take three rounds of it.
+__device__ __forceinline__ void plain_quantize_q8_0_cta4(const float *xf, int n, int8_t *q_out, float *d_out) {
+    const int nchunks = n >> 2;         // a multiple of eight: the lanes of a block are live together
+    for (int base = threadIdx.x; base < ((nchunks + 31) & ~31); base += 4 * blockDim.x) {
+        float4 v[4];
+        float amax[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int ch = base + k * blockDim.x;
+            v[k] = ch < nchunks ? *reinterpret_cast<const float4 *>(xf + 4 * ch) : make_float4(0, 0, 0, 0);
+            amax[k] = fmaxf(fmaxf(fabsf(v[k].x), fabsf(v[k].y)), fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
+        }
+#pragma unroll
+        for (int s = 1; s < 8; s <<= 1)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) amax[k] = fmaxf(amax[k], __shfl_xor_sync(0xffffffffu, amax[k], s));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int ch = base + k * blockDim.x;
+            if (ch >= nchunks) continue;
+            uint32_t packed = 0;
+            if (amax[k] != 0.0f) {
+                const float inv = __fdiv_rn(127.0f, amax[k]);
+                const float f[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    int q = __float2int_rn(__fmul_rn(f[j], inv));
+                    q = max(-128, min(127, q));
+                    packed |= static_cast<uint32_t>(q & 0xff) << (8 * j);
+                }
+            }
+            *reinterpret_cast<uint32_t *>(q_out + 4 * ch) = packed;
+            if ((ch & 7) == 0) d_out[ch >> 3] = __half2float(__float2half_rn(__fdiv_rn(amax[k], 127.0f)));
+        }
+    }
+}
+
 // Q8_K superblocks of the activations of an IQ down tensor sit kPlainActStride apart; IQ4_NL's Q8_0 quants are plain.
 __host__ __device__ inline size_t plain_down_wide_act_bytes(int F, int K, bool nl) {
     return nl ? static_cast<size_t>(K) * F : static_cast<size_t>(K) * (F / 256) * kPlainActStride;
@@ -270,7 +308,10 @@ __global__ void __launch_bounds__(kThreads) plain_down_wide_kernel(const PlainPa
         if (lane < K) bulk_load(chunks + static_cast<size_t>(lane) * 16 * drb, P.down + (e * P.H + h0) * drb, static_cast<uint32_t>(16 * drb), bar);
         if (lane == K && shb) bulk_load(shs, P.sh_down + static_cast<size_t>(h0 / 4) * nbs * 136, shb, bar);
     }
-    // the shared expert's activation is older than the kernel before this one
+    // the shared expert's activation, its gate and the weights are older than the kernel before this one
+    float *w_s = reinterpret_cast<float *>(psm + 64), *gate_s = reinterpret_cast<float *>(psm + 16);
+    if (warp == kWarps - 1 && lane < K) w_s[lane] = P.weights[t * K + lane];
+    if (warp == kWarps - 2 && lane == 0 && SF > 0) *gate_s = P.sgate[t];
     for (int i = threadIdx.x; i < SF / 4; i += kThreads)
         reinterpret_cast<float4 *>(actf)[i] = reinterpret_cast<const float4 *>(P.shact + static_cast<size_t>(t) * SF)[i];
     __syncthreads();
@@ -287,7 +328,7 @@ __global__ void __launch_bounds__(kThreads) plain_down_wide_kernel(const PlainPa
     __syncthreads();
     WD_PSTAMP(1, 3)
     if (nl) {
-        plain_quantize_q8_0_cta(actf, K * F, actq, actd);
+        plain_quantize_q8_0_cta4(actf, K * F, actq, actd);
     } else {
         for (int s = warp; s < K * nsb; s += kWarps)
             quantize_q8_K_warp(actf + s * 256, lane, reinterpret_cast<uint8_t *>(actq) + s * kPlainActStride, actd + s);
@@ -327,20 +368,16 @@ __global__ void __launch_bounds__(kThreads) plain_down_wide_kernel(const PlainPa
     }
     __syncthreads();
     WD_PSTAMP(1, 6)
-    for (int i = threadIdx.x; i < K * 16; i += kThreads)
-        P.eo[(static_cast<size_t>(t) * K + (i >> 4)) * P.H + h0 + (i & 15)] = eo_s[i];
     if (threadIdx.x < 16) {
         const size_t o = static_cast<size_t>(t) * P.H + h0 + threadIdx.x;
         float r = 0.0f;
-        for (int j = 0; j < K; ++j) r = __fadd_rn(r, __fmul_rn(eo_s[j * 16 + threadIdx.x], P.weights[t * K + j]));
+        for (int j = 0; j < K; ++j) r = __fadd_rn(r, __fmul_rn(eo_s[j * 16 + threadIdx.x], w_s[j]));
+        P.out[o] = SF > 0 ? __fadd_rn(r, __fmul_rn(shd_s[threadIdx.x], *gate_s)) : r;
         P.routed[o] = r;
-        if (SF > 0) {
-            P.shdown[o] = shd_s[threadIdx.x];
-            P.out[o] = __fadd_rn(r, __fmul_rn(shd_s[threadIdx.x], P.sgate[t]));
-        } else {
-            P.out[o] = r;
-        }
+        if (SF > 0) P.shdown[o] = shd_s[threadIdx.x];
     }
+    for (int i = threadIdx.x; i < K * 16; i += kThreads)
+        P.eo[(static_cast<size_t>(t) * K + (i >> 4)) * P.H + h0 + (i & 15)] = eo_s[i];
     WD_PSTAMP(1, 7)
 }
 
