@@ -99,97 +99,90 @@ __device__ __forceinline__ void q8_0_block_warp(float v, int lane, Quant *q_out,
     if (lane == 0) *d_out = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
 }
 
-// hidden += proj (when given); y = RMSNorm(hidden) * w -> Q8_0 (plain layout: int8 [n], float scale per block).
-// One CTA of 256 threads, thread t owns the EPL = n / 256 consecutive elements from t * EPL (EPL in {1, 2, 4, 8, 16}),
-// so a Q8_0 block belongs to 32 / EPL neighbouring lanes (residual_rmsnorm_kernel, src/warodecode.cu:1408). The sum of
-// squares is the binary tree in double of the MoE stack's RMSNorm. `token` (optional): the step starts here, and
-// hidden is first filled with the token's embedding row (embedding_q4_kernel).
-template <int EPL, class Quant>
+// Four quants of one thread (values e .. e + 3, e a multiple of four) with one store.
+__device__ __forceinline__ void store_quant4(int8_t *out, int e, uint32_t packed) { *reinterpret_cast<uint32_t *>(out + e) = packed; }
+__device__ __forceinline__ void store_quant4(PairedQuant *out, int e, uint32_t packed) {
+    *reinterpret_cast<uint32_t *>(out + (e & ~31) + paired_place(e & 31)) = packed;
+}
+
+// hidden += proj (when given); y = RMSNorm(hidden) * w -> Q8_0 (plain layout: int8 [n], float scale per block), by one CTA of
+// n / 4 threads, n = 256 * 2^k up to 4096: thread t owns elements 4 t .. 4 t + 3, a Q8_0 block eight neighbouring lanes
+// (residual_rmsnorm_kernel, src/warodecode.cu:1408). The sum of squares is the binary tree in double of the MoE stack's
+// RMSNorm. `embd_row` (optional): the step starts here, and hidden is first filled with the token's embedding row
+// (embedding_q4_kernel). `wait`: what the norm weights, which no kernel writes, are fetched in front of.
+// Bound: latency (a chain of one load, two reductions and two divisions, run once); 256 threads with eight elements each and
+// scalar loads took 3.2 us per call inside the step.
+template <class Quant, class Wait>
 __device__ __forceinline__ void dense_norm_quant_body(float *hidden, const float *proj, const float *w, int n, float eps, Quant *xq,
-                                                      float *xd, const uint8_t *embd_row, bool embd_q8 = false) {
-    __shared__ double red[kDecThreads / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float v[EPL];
-    if (embd_row != nullptr) {
+                                                      float *xd, const uint8_t *embd, const int *token, int vocab, bool embd_q8, Wait wait) {
+    __shared__ double red[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5, e0 = tid * 4;
+    const float4 nw = w != nullptr ? *reinterpret_cast<const float4 *>(w + e0) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    wait();
+    float v[4];
+    if (embd != nullptr) {
+        const int bytes = embd_q8 ? 34 : 18, j = e0 & 31;
+        const uint8_t *wb = embd + (static_cast<size_t>(max(0, min(vocab - 1, *token))) * (n >> 5) + (e0 >> 5)) * bytes;
+        const float d = half_bits_to_float(static_cast<uint16_t>(wb[0] | (wb[1] << 8)));
 #pragma unroll
-        for (int i = 0; i < EPL; ++i) {
-            const int e = tid * EPL + i, b = e >> 5, j = e & 31;
-            const uint8_t *wb = embd_row + b * (embd_q8 ? 34 : 18);
-            const float d = half_bits_to_float(static_cast<uint16_t>(wb[0] | (wb[1] << 8)));
-            const int q = embd_q8 ? static_cast<int>(static_cast<int8_t>(wb[2 + j]))
-                                  : (j < 16 ? (wb[2 + j] & 0x0f) : (wb[2 + j - 16] >> 4)) - 8;
+        for (int i = 0; i < 4; ++i) {
+            const int q = embd_q8 ? static_cast<int>(static_cast<int8_t>(wb[2 + j + i]))
+                                  : (j < 16 ? (wb[2 + j + i] & 0x0f) : (wb[2 + j + i - 16] >> 4)) - 8;
             v[i] = __fmul_rn(d, static_cast<float>(q));
-            hidden[e] = v[i];
         }
     } else {
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) v[i] = hidden[tid * EPL + i];
+        const float4 h = *reinterpret_cast<const float4 *>(hidden + e0);
+        v[0] = h.x; v[1] = h.y; v[2] = h.z; v[3] = h.w;
         if (proj != nullptr) {
-#pragma unroll
-            for (int i = 0; i < EPL; ++i) {
-                v[i] = __fadd_rn(v[i], proj[tid * EPL + i]);
-                hidden[tid * EPL + i] = v[i];
-            }
+            const float4 p = *reinterpret_cast<const float4 *>(proj + e0);
+            v[0] = __fadd_rn(v[0], p.x);
+            v[1] = __fadd_rn(v[1], p.y);
+            v[2] = __fadd_rn(v[2], p.z);
+            v[3] = __fadd_rn(v[3], p.w);
         }
     }
-    float nw[EPL];
+    if (embd != nullptr || proj != nullptr) *reinterpret_cast<float4 *>(hidden + e0) = make_float4(v[0], v[1], v[2], v[3]);
+    double sq[4];
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) nw[i] = w != nullptr ? w[tid * EPL + i] : 1.0f;
-    double loc[EPL];
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) loc[i] = __dmul_rn(static_cast<double>(v[i]), static_cast<double>(v[i]));
-#pragma unroll
-    for (int s = 1; s < EPL; s <<= 1)
-#pragma unroll
-        for (int i = 0; i + s < EPL; i += 2 * s) loc[i] = __dadd_rn(loc[i], loc[i + s]);
-    double ss = loc[0];
+    for (int i = 0; i < 4; ++i) sq[i] = __dmul_rn(static_cast<double>(v[i]), static_cast<double>(v[i]));
+    double ss = __dadd_rn(__dadd_rn(sq[0], sq[1]), __dadd_rn(sq[2], sq[3]));
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, s));
     if (lane == 0) red[warp] = ss;
     __syncthreads();
-    double tot[kDecThreads / 32];
+    ss = lane < nwarps ? red[lane] : 0.0;           // a power of two of warps; adding +0.0 beyond them changes nothing
 #pragma unroll
-    for (int i = 0; i < kDecThreads / 32; ++i) tot[i] = red[i];
-#pragma unroll
-    for (int s = 1; s < kDecThreads / 32; s <<= 1)
-#pragma unroll
-        for (int i = 0; i + s < kDecThreads / 32; i += 2 * s) tot[i] = __dadd_rn(tot[i], tot[i + s]);
-    const float scale = __double2float_rn(
-        __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__ddiv_rn(tot[0], static_cast<double>(n)), static_cast<double>(eps)))));
+    for (int s = 1; s < 32; s <<= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, s));
+    // n is a power of two: the division by it is an exact multiplication
+    const double inv_n = __longlong_as_double(static_cast<long long>(1023 - (31 - __clz(n))) << 52);
+    const float scale = __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dmul_rn(ss, inv_n), static_cast<double>(eps)))));
+    const float g[4] = {nw.x, nw.y, nw.z, nw.w};
     float amax = 0.0f;
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) {
+    for (int i = 0; i < 4; ++i) {
         v[i] = __fmul_rn(v[i], scale);
-        if (w != nullptr) v[i] = __fmul_rn(v[i], nw[i]);
+        if (w != nullptr) v[i] = __fmul_rn(v[i], g[i]);
         amax = fmaxf(amax, fabsf(v[i]));
     }
 #pragma unroll
-    for (int s = 1; s < 32 / EPL; s <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
+    for (int s = 1; s < 8; s <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
     const float inv = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+    uint32_t packed = 0;
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) {
+    for (int i = 0; i < 4; ++i) {
         int q = amax != 0.0f ? __float2int_rn(__fmul_rn(v[i], inv)) : 0;
         q = max(-128, min(127, q));
-        store_quant(xq, tid * EPL + i, q);
+        packed |= static_cast<uint32_t>(q & 0xff) << (8 * i);
     }
-    if ((tid * EPL & 31) == 0) xd[(tid * EPL) >> 5] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
+    store_quant4(xq, e0, packed);
+    if ((lane & 7) == 0) xd[e0 >> 5] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
 }
 
-__global__ void __launch_bounds__(kDecThreads) dense_norm_quant_kernel(float *hidden, const float *proj, const float *w, int n,
-                                                                     float eps, int8_t *xq, float *xd, const uint8_t *embd,
-                                                                     const int *token, int vocab, int embd_q8) {
+__global__ void __launch_bounds__(1024) dense_norm_quant_kernel(float *hidden, const float *proj, const float *w, int n, float eps, int8_t *xq,
+                                                               float *xd, const uint8_t *embd, const int *token, int vocab, int embd_q8) {
     grid_dep_launch();
-    grid_dep_wait();
-    const uint8_t *row = nullptr;     // the embedding table in ggml layout: Q4_0 blocks of 18 bytes, or Q8_0 blocks of 34
-    if (embd != nullptr) row = embd + static_cast<size_t>(max(0, min(vocab - 1, *token))) * (n >> 5) * (embd_q8 ? 34 : 18);
-    const bool q8 = embd_q8 != 0;
-    switch (n / kDecThreads) {
-        case 1: dense_norm_quant_body<1>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-        case 2: dense_norm_quant_body<2>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-        case 4: dense_norm_quant_body<4>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-        case 8: dense_norm_quant_body<8>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-        default: dense_norm_quant_body<16>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-    }
+    // the embedding table in ggml layout: Q4_0 blocks of 18 bytes, or Q8_0 blocks of 34
+    dense_norm_quant_body(hidden, proj, w, n, eps, xq, xd, embd, token, vocab, embd_q8 != 0, [] { grid_dep_wait(); });
 }
 
 // y = W x: W Q4_0 in the row layout, x already Q8_0 (plain layout, copied into shared memory once per CTA).
@@ -475,14 +468,14 @@ __device__ __forceinline__ float dense_attention_core(const float *qs, const flo
 // The dot q . k of the one-token order - lane l runs fmaf over d = l, l + 32, ..., then the butterfly - by ONE thread, four
 // lanes at a time: quads of lanes meet in the butterfly's own pairs (16 apart, 8 apart, 4, 2, 1), so nothing is shuffled.
 template <int HD>
-__device__ __forceinline__ float lane_order_dot(const float *q, const float4 (&k)[HD / 4]) {
+__device__ __forceinline__ float lane_order_dot(const float *q, const float *k) {
     auto quad = [&](int b, float (&a)[4]) {         // lanes 4 b .. 4 b + 3
 #pragma unroll
         for (int i = 0; i < 4; ++i) a[i] = 0.0f;
 #pragma unroll
         for (int r = 0; r < HD / 32; ++r) {
             const float4 qv = *reinterpret_cast<const float4 *>(q + r * 32 + b * 4);
-            const float4 kv = k[r * 8 + b];
+            const float4 kv = *reinterpret_cast<const float4 *>(k + r * 32 + b * 4);
             a[0] = __fmaf_rn(qv.x, kv.x, a[0]);
             a[1] = __fmaf_rn(qv.y, kv.y, a[1]);
             a[2] = __fmaf_rn(qv.z, kv.z, a[2]);
@@ -495,12 +488,10 @@ __device__ __forceinline__ float lane_order_dot(const float *q, const float4 (&k
         float a[4], b[4], c[4], d[4];
         quad(p, a);
         quad(p + 4, b);
-        asm volatile("" ::: "memory");              // the loads of q stay behind this point: registers belong to the key
         quad(p + 2, c);
         quad(p + 6, d);
 #pragma unroll
         for (int i = 0; i < 4; ++i) s8[p][i] = __fadd_rn(__fadd_rn(a[i], b[i]), __fadd_rn(c[i], d[i]));
-        asm volatile("" ::: "memory");
     }
     float s4[4];
 #pragma unroll
@@ -517,11 +508,18 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Geometry of the decode attention for a head dimension: threads, and the ring of value chunks (64 positions each).
+// Geometry of the decode attention for a head dimension: chunks of 64 cache rows (keys or values) in padded rows, so that
+// neighbouring positions start in different banks.
 template <int HD>
 struct DecodeAttn {
-    static constexpr int kThreads = HD <= 64 ? 512 : 256;       // a thread keeps a whole key in registers
-    static constexpr int kChunk = 64, kRing = HD <= 64 ? 8 : 4; // values in flight: 128 KB at most
+    static constexpr int kThreads = 512, kChunk = 64, kRow = HD + 4;
+    static constexpr int kSlotBytes = kChunk * kRow * 4;
+    static constexpr int kRoom = 190 * 1024;                    // slots and scores together; the rest of an SM is for the product before it
+    // slots of the ring: both caches of the longest context, or what fits beside its scores
+    static int slots(int max_ctx) {
+        const int want = 2 * ((max_ctx + kChunk - 1) / kChunk), fit = (kRoom - max_ctx * 4) / kSlotBytes;
+        return want < fit ? want : fit;
+    }
 };
 
 // Rotary embedding + cache store + decode attention + Q8_0 of the head's output, one CTA per query head (rope_store_kernel
@@ -532,47 +530,48 @@ struct DecodeAttn {
 // copy, so no CTA waits for another's store.
 //
 // Bound: latency. The sums over positions run ascending (one fmaf per position and element, four cycles each), so the
-// keys and values must be there when they are needed: the cache below pos was written by earlier graph launches, and
-// its first 256 or 512 keys (one per thread, in registers) and the first chunks of the values (shared memory) are
+// keys and values must be there when they are needed: the cache below pos was written by earlier tokens, and the first
+// chunks of it (all of it up to 320 positions of 64) are copied to shared memory in a ring, keys before values,
 // requested BEFORE the wait for the QKV product; a score is one thread's work, without shuffles.
-// Measured on the 16-layer model (32 heads of 64): 512 positions 1.8 ms -> see the design table, 72 positions likewise.
+// Measured per layer inside the step of the 16-layer model (32 heads of 64), start -> now: 2.1 us at 72 positions (6.6 us
+// before), and at 512 positions 74 us before.
 //
 // EXTRAS: the layer has q/k/v biases (Qwen2-style files: added to the QKV product's rows) and / or RMSNorm weights for
 // the q and k heads (Qwen3-style: qk_norm_kernel, src/warodecode.cu:1836), applied in that order before the rotary
 // embedding (emit_step :2069-2075). Layers without them run the instantiation that has none of that code.
-// Dynamic shared memory: `ring` value chunks, then max_ctx scores.
+// Dynamic shared memory: `slots` chunks, then max_ctx scores.
 template <int HD, bool EXTRAS>
 __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kernel(const float *qkv, const float *table, float *kcache,
                                                                                  float *vcache, const int *pos_ptr, int heads,
-                                                                                 int kv_heads, int ring, float inv_sqrt, int8_t *oq,
+                                                                                 int kv_heads, int slots, float inv_sqrt, int8_t *oq,
                                                                                  float *od, const float *bqkv, const float *q_norm,
                                                                                  const float *k_norm, float eps) {
     using A = DecodeAttn<HD>;
-    constexpr int kNt = A::kThreads, kChunk = A::kChunk, kHalf = HD / 2, kRow16 = HD / 4;
+    constexpr int kNt = A::kThreads, kChunk = A::kChunk, kRow = A::kRow, kHalf = HD / 2, kRow16 = HD / 4;
     extern __shared__ __align__(16) float vring[];
     __shared__ __align__(16) float qs[HD], kn[HD];
     __shared__ float vn[HD], outv[HD], wmax[kNt / 32];
-    float *sc = vring + static_cast<size_t>(ring) * kChunk * HD;
+    float *sc = vring + static_cast<size_t>(slots) * kChunk * kRow;
     grid_dep_launch();
     const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int pos = *pos_ptr, kv_dim = kv_heads * HD, kvh = (h * kv_heads) / heads;
     float *kc = kcache + static_cast<size_t>(kvh) * HD, *vc = vcache + static_cast<size_t>(kvh) * HD;
-    const int n_chunks = (pos + kChunk - 1) / kChunk;           // positions 0 .. pos - 1
-    auto request = [&](int c) {
-        float *dst = vring + static_cast<size_t>(c % ring) * kChunk * HD;
+    const int n_chunks = (pos + kChunk - 1) / kChunk, n_items = 2 * n_chunks;      // positions 0 .. pos - 1: key chunks, then value chunks
+    auto slot_of = [&](int item) { return vring + static_cast<size_t>(item % slots) * kChunk * kRow; };
+    auto request = [&](int item) {
+        if (item >= n_items) return;
+        const int c = item < n_chunks ? item : item - n_chunks;
+        const float *src = item < n_chunks ? kc : vc;
+        float *dst = slot_of(item);
         for (int i = tid; i < kChunk * kRow16; i += kNt) {
             const int r = i / kRow16, e = i - r * kRow16, t = c * kChunk + r;
-            if (t < pos) cp_async16(dst + r * HD + e * 4, vc + static_cast<size_t>(t) * kv_dim + e * 4, true);
+            if (t < pos) cp_async16(dst + r * kRow + e * 4, src + static_cast<size_t>(t) * kv_dim + e * 4, true);
         }
     };
-    for (int c = 0; c < min(ring, n_chunks); ++c) request(c);
+    for (int i = 0; i < min(slots, n_chunks); ++i) request(i);
     cp_async_commit();
-    float4 k[HD / 4];
-    auto load_key = [&](int t) {
-#pragma unroll
-        for (int i = 0; i < HD / 4; ++i) k[i] = *reinterpret_cast<const float4 *>(kc + static_cast<size_t>(t) * kv_dim + i * 4);
-    };
-    if (tid < pos) load_key(tid);
+    for (int i = n_chunks; i < min(slots, n_items); ++i) request(i);
+    cp_async_commit();
     float cs = 0.0f, sn = 0.0f;
     if (tid < kHalf) {
         cs = table[(static_cast<size_t>(pos) * kHalf + tid) * 2];
@@ -652,16 +651,32 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
     }
     __syncthreads();
     float m = -INFINITY;
-    for (int t = tid; t <= pos; t += kNt) {
-        if (t == pos) {
-#pragma unroll
-            for (int i = 0; i < HD / 4; ++i) k[i] = *reinterpret_cast<const float4 *>(kn + i * 4);
-        } else if (t != tid) {
-            load_key(t);
+    const int batch = min(kNt / kChunk, slots);         // key chunks scored side by side, one position per thread
+#pragma unroll 1
+    for (int c0 = 0; c0 < max(n_chunks, 1); c0 += batch) {
+        if (c0 == 0) cp_async_wait<1>();
+        else cp_async_wait<0>();
+        __syncthreads();
+        const int c = c0 + tid / kChunk, t = c * kChunk + (tid & (kChunk - 1));
+        const bool newest = c0 == 0 && tid == kNt - 1;
+        if ((tid < batch * kChunk && c < n_chunks && t < pos) || newest) {
+            // the last thread scores the new position, and an old one too when it has one
+            if (!newest || (tid < batch * kChunk && t < pos)) {
+                const float v = __fmul_rn(lane_order_dot<HD>(qs, slot_of(c) + (tid & (kChunk - 1)) * kRow), inv_sqrt);
+                sc[t] = v;
+                m = v > m ? v : m;          // a NaN score never becomes the maximum
+            }
+            if (newest) {
+                const float v = __fmul_rn(lane_order_dot<HD>(qs, kn), inv_sqrt);
+                sc[pos] = v;
+                m = v > m ? v : m;
+            }
         }
-        const float v = __fmul_rn(lane_order_dot<HD>(qs, k), inv_sqrt);
-        sc[t] = v;
-        m = v > m ? v : m;          // a NaN score never becomes the maximum
+        if (n_items > slots) {
+            __syncthreads();
+            for (int k = c0; k < min(c0 + batch, n_chunks); ++k) request(k + slots);
+            cp_async_commit();
+        }
     }
 #pragma unroll
     for (int s = 16; s >= 1; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
@@ -677,22 +692,37 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
 #pragma unroll 1
     for (int c = 0; c < n_chunks; ++c) {
         if (tid < HD) {
-            const float *v = vring + static_cast<size_t>(c % ring) * kChunk * HD + tid, *p = sc + c * kChunk;
+            const float *v = slot_of(n_chunks + c) + tid, *p = sc + c * kChunk;
             const int n = min(kChunk, pos - c * kChunk);
-#pragma unroll 8
-            for (int r = 0; r < n; ++r) {
+            // the two chains advance four cycles a step; a whole chunk's weights and values are requested well ahead of them
+            int r = 0;
+            for (; r + 32 <= n; r += 32) {
+                float4 p4[8];
+                float x[32];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) p4[i] = *reinterpret_cast<const float4 *>(p + r + 4 * i);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) x[i] = v[(r + i) * kRow];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    l = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(l, p4[i].x), p4[i].y), p4[i].z), p4[i].w);
+                    acc = __fmaf_rn(p4[i].x, x[4 * i], acc);
+                    acc = __fmaf_rn(p4[i].y, x[4 * i + 1], acc);
+                    acc = __fmaf_rn(p4[i].z, x[4 * i + 2], acc);
+                    acc = __fmaf_rn(p4[i].w, x[4 * i + 3], acc);
+                }
+            }
+            for (; r < n; ++r) {
                 l = __fadd_rn(l, p[r]);
-                acc = __fmaf_rn(p[r], v[r * HD], acc);
+                acc = __fmaf_rn(p[r], v[r * kRow], acc);
             }
         }
-        if (n_chunks > ring) {      // longer than the ring: refill the slot, and wait when the next one was refilled too
+        if (n_chunks > slots) {     // longer than the ring: refill the slot; when a refilled chunk is read, more than three requests are younger
             __syncthreads();
-            if (c + ring < n_chunks) request(c + ring);
+            request(n_chunks + c + slots);
             cp_async_commit();
-            if (c + 1 >= ring) {
-                cp_async_wait<A::kRing - 1>();
-                __syncthreads();
-            }
+            cp_async_wait<3>();
+            __syncthreads();
         }
     }
     if (tid < HD) {

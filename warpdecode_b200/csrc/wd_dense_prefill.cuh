@@ -13,26 +13,13 @@ namespace wd {
 constexpr int kPrefillChunk = 512;      // tokens per pass at most (workspace: about 100 KB per token at ffn 8192)
 
 // RMSNorm + Q8_0 of every token of the chunk, one CTA per token; the body is the one-token kernel's.
-__global__ void __launch_bounds__(kDecThreads) prefill_norm_quant_kernel(float *hidden, const float *proj, const float *w, int n, float eps,
-                                                                       PairedQuant *xq, float *xd, const uint8_t *embd, const int *tokens,
-                                                                       int vocab, int embd_q8) {
+__global__ void __launch_bounds__(1024) prefill_norm_quant_kernel(float *hidden, const float *proj, const float *w, int n, float eps,
+                                                                 PairedQuant *xq, float *xd, const uint8_t *embd, const int *tokens, int vocab,
+                                                                 int embd_q8) {
     grid_dep_launch();
-    grid_dep_wait();
     const size_t m = blockIdx.x;
-    hidden += m * n;
-    if (proj != nullptr) proj += m * n;
-    xq += m * n;
-    xd += m * (n >> 5);
-    const uint8_t *row = nullptr;
-    if (embd != nullptr) row = embd + static_cast<size_t>(max(0, min(vocab - 1, tokens[m]))) * (n >> 5) * (embd_q8 ? 34 : 18);
-    const bool q8 = embd_q8 != 0;
-    switch (n / kDecThreads) {
-        case 1: dense_norm_quant_body<1>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-        case 2: dense_norm_quant_body<2>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-        case 4: dense_norm_quant_body<4>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-        case 8: dense_norm_quant_body<8>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-        default: dense_norm_quant_body<16>(hidden, proj, w, n, eps, xq, xd, row, q8); break;
-    }
+    dense_norm_quant_body(hidden + m * n, proj != nullptr ? proj + m * n : nullptr, w, n, eps, xq + m * n, xd + m * (n >> 5), embd,
+                          tokens + m, vocab, embd_q8 != 0, [] { grid_dep_wait(); });
 }
 
 // ---- Y[m][row] = W[row] . X[m] for the tokens of a chunk ---------------------------------------------------------------
