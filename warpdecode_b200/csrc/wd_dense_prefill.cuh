@@ -89,7 +89,9 @@ struct PrefillGemm {
     static constexpr int kOffX = kRows * kWStride, kOffDw = kOffX + kTok * kXStride, kOffDx = kOffDw + kRows * kDwStride;
     static constexpr int kStage = (kOffDx + kTc * 4 * kDxStride + 127) / 128 * 128;
     static constexpr int kRed = 4 * kTok * (kRows + 4) * 4;              // the residues' sums, after the last stage
-    static constexpr int kStages = NT == 4 ? 4 : 6;
+    // few tokens: the weights are all there is to stream, so more of them travel
+    static constexpr int kDeep = NT == 4 ? 4 : NT == 2 ? 8 : 12, kFit = 200 * 1024 / kStage;
+    static constexpr int kStages = kDeep < kFit ? kDeep : kFit;
     static constexpr int kSmem = kStages * kStage > kRed ? kStages * kStage : kRed;
 };
 
@@ -149,13 +151,14 @@ __global__ void __launch_bounds__(128 * RG) prefill_gemm_kernel(const uint8_t *w
                 cp_async16(st + G::kOffX + r * G::kXStride + p * 16,
                            live ? xq + static_cast<size_t>((tok0 + r) * nb + b) * 32 + (p & 1) * 16 : xq, live);
         }
-        if (tid < G::kTok * G::kTc * 4) {
-            const int r = tid / (G::kTc * 4), k = tid % (G::kTc * 4), b = b0 + 32 * (k >> 2) + (k & 3);
+#pragma unroll
+        for (int e = tid; e < G::kTok * G::kTc * 4; e += G::kThreads) {
+            const int r = e / (G::kTc * 4), k = e % (G::kTc * 4), b = b0 + 32 * (k >> 2) + (k & 3);
             const bool live = tok0 + r < m_tokens && b < nb;
             cp_async4(st + G::kOffDx + k * G::kDxStride + r * 4, live ? xd + static_cast<size_t>(tok0 + r) * nb + b : xd, live);
         }
     };
-    static_assert(G::kRows * G::kTc <= G::kThreads && G::kTok * G::kTc * 4 <= G::kThreads, "one piece of the scales per thread and stage");
+    static_assert(G::kRows * G::kTc <= G::kThreads, "one piece of the scales per thread and stage");
 
     // the weights do not depend on the kernel before this one: the first stages' rows leave before the wait for it
     Cursor cw, cx;
@@ -283,10 +286,11 @@ __global__ void __launch_bounds__(32 * kRopeWarps) prefill_rope_kernel(const flo
     grid_dep_launch();
     grid_dep_wait();
     const int m = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = head_dim / 2, nd = head_dim / 32;
+    const int step = kRopeWarps * gridDim.y;            // short prompts: several CTAs share a token's heads
     const int kv_dim = kv_heads * head_dim, pos = pos0 + m;
     const float *src = qkv + static_cast<size_t>(m) * (heads + 2 * kv_heads) * head_dim;
     float *row = rows[warp];
-    for (int h = warp; h < heads + kv_heads; h += kRopeWarps) {
+    for (int h = blockIdx.y * kRopeWarps + warp; h < heads + kv_heads; h += step) {
         const bool is_q = h < heads;
         const float *norm = is_q ? q_norm : k_norm;
         float x[4];
@@ -388,12 +392,17 @@ __global__ void __launch_bounds__(kPrefillAttnThreads, HD <= 64 ? 2 : 1) prefill
         qs[i] = r < n_tok ? qrot[(static_cast<size_t>(tok0 + r) * heads + h) * HD + d] : 0.0f;
     }
     __syncthreads();
-    for (int t = tid; t <= last; t += kPrefillAttnThreads) {
+    // scores: a thread takes one position and, while there are fewer positions than threads, a share of the tokens
+    int groups = 1;
+    while (groups < QT / 2 && 2 * groups * (last + 1) <= 256) groups *= 2;
+    const int rows = QT / groups;
+    for (int i = tid; i < (last + 1) * groups; i += kPrefillAttnThreads) {
+        const int gidx = i / (last + 1), t = i - gidx * (last + 1);
         ulonglong2 k[HD / 4];
 #pragma unroll
-        for (int i = 0; i < HD / 4; ++i) k[i] = *reinterpret_cast<const ulonglong2 *>(kc + static_cast<size_t>(t) * kv_dim + i * 4);
+        for (int e = 0; e < HD / 4; ++e) k[e] = *reinterpret_cast<const ulonglong2 *>(kc + static_cast<size_t>(t) * kv_dim + e * 4);
 #pragma unroll 1
-        for (int r = 0; r < QT; r += 2) {
+        for (int r = gidx * rows; r < (gidx + 1) * rows; r += 2) {
             const float a = __fmul_rn(lane_order_dot2<HD>(qs + r * HD, k), inv_sqrt);
             const float b = __fmul_rn(lane_order_dot2<HD>(qs + (r + 1) * HD, k), inv_sqrt);
             *reinterpret_cast<float2 *>(sc + static_cast<size_t>(t) * QT + r) = make_float2(a, b);
