@@ -74,3 +74,26 @@ def test_wide_rows_of_the_plain_layout_path(oracle, monkeypatch, H, F, gate, up,
             assert np.array_equal(bits(out[t]), bits(want[t]["out"])), (wide, t)
         assert eng.device_status() == 0
         eng.close()
+
+
+@pytest.mark.parametrize("bad", [(1,), (0, 3), (0, 1, 2, 3)])
+def test_a_batch_whose_early_picks_do_not_stand_is_decoded_again(oracle, bad):
+    """Huge activations push most probabilities to zero: the k largest logits are then not the k rungs, and the tiles asked
+    for before the proof belong to the wrong experts. One such token makes the whole batch decode again."""
+    import warpdecode_b200 as wd
+    H, F, E, K, SF = 512, 256, 64, 6, 128
+    m = synth.make_moe_block(77, H, F, E, K, SF, 21, 22)
+    x = np.random.Generator(np.random.PCG64(5)).standard_normal((4, H)).astype(np.float32)
+    x[list(bad)] *= np.float32(1000.0)
+    want = [oracle.moe_block(m, v) for v in x]
+    eng = wd.Engine(H, F, E, K, SF, 1, expert_type=21, down_type=22, max_tokens=4)
+    eng.load_block(0, m)
+    for _ in range(3):
+        out = eng.forward_host(0, x)
+        for t in range(4):
+            assert np.array_equal(eng.tap("ids", t), want[t]["ids"])
+            for name in ("weights", "act", "expert_out"):
+                assert np.array_equal(bits(eng.tap(name, t)), bits(want[t][name])), (t, name)
+            assert np.array_equal(bits(out[t]), bits(want[t]["out"])), t
+    assert eng.fallbacks() == 3 * len(bad) and eng.device_status() == 0
+    eng.close()

@@ -442,6 +442,8 @@ void plan_batch(wd_engine *e) {
     e->batch_single = true;
     if (const char *v = std::getenv("WD_BATCH_SINGLE")) e->batch_single = std::atoi(v) != 0;
     const int nbh = H / 32, nbs = SF / 32;
+    const int wcta = e->wide ? ncta - Tm : ncta;     // with wide tiles one CTA per token proves the selection instead of taking tiles
+    if (wcta < 1) return;
     p.H = H; p.F = F; p.SF = SF; p.E = E; p.K = K; p.T = Tm;
     p.nsb_h = m.nsb_h; p.nsb_f = m.nsb_f; p.t2_log2 = m.t2_log2; p.t3_log2 = m.t3_log2;
     p.w_scale = m.w_scale;
@@ -478,19 +480,19 @@ void plan_batch(wd_engine *e) {
     p.scr_rows = static_cast<unsigned>(scr_floats);
     p.scr_bytes = static_cast<unsigned>(align_up((scr_floats + 64) * 4, 128));
     p.off_scr = take(static_cast<size_t>(p.scr_bytes) * wd::kWarps);
-    p.off_bar = take(wd::kBatchMaxBars * 8);
+    p.off_bar = take(wd::kBatchMaxBars * 8 * (e->wide ? 2 : 1));
     p.off_slots = take(static_cast<size_t>(E) * 4);
     p.off_seq = take(wd::kBatchMaxRing * 4);
     p.off_seg = take(96 * 4 + static_cast<size_t>(wd::kMaxTokens) * K * m.nsb_f * 4);     // segments, pair counters, activation states
     {
         const int t2 = F / r_h, t3d = H / r_f;
         if (t2 > 4096 || t3d > 4096) return;
-        p.max_tasks = static_cast<unsigned>(Tm * (2 * ((K * t2 + ncta - 1) / ncta) + (K * t3d + ncta - 1) / ncta + 1));
+        p.max_tasks = static_cast<unsigned>(Tm * (2 * ((K * t2 + wcta - 1) / wcta) + (K * t3d + wcta - 1) / wcta + 1));
         p.off_tasks = take(static_cast<size_t>(p.max_tasks) * 16);
     }
     p.off_pairbuf = take(static_cast<size_t>(32) * 2 * r_h * 4);
     const int t3 = H / r_f;                                  // down tiles per pair
-    const int max3 = (K * t3 + ncta - 1) / ncta;             // longest run of one token's down tiles in one CTA
+    const int max3 = (K * t3 + wcta - 1) / wcta;             // longest run of one token's down tiles in one CTA
     const int n_exp_tok = std::min(K, (max3 - 1) / t3 + 2);  // pairs such a run can touch
     p.n_act = static_cast<unsigned>(wd::kMaxTokens * n_exp_tok * m.nsb_f);
     if (p.n_act > 62) return;
@@ -1148,7 +1150,8 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
         auto up16 = [](size_t w) { return (w + 15) / 16 * 16; };
         const size_t w_logits = 0, w_shact = up16(w_logits + Tm * E), w_shgate = up16(w_shact + Tm * std::max(c.shared_ffn, 1)),
                      w_act = w_shgate + 16, w_eo = up16(w_act + Tm * K * F), w_shdown = up16(w_eo + Tm * K * H),
-                     w_sel = up16(w_shdown + Tm * H), w_end = up16(w_sel + Tm * 2 * wd::kMaxK);
+                     w_sel = up16(w_shdown + Tm * H), w_act2 = up16(w_sel + Tm * wd::kBatchSelStride), w_eo2 = up16(w_act2 + Tm * K * F),
+                     w_end = up16(w_eo2 + Tm * K * H);
         cudaError_t be = cudaMalloc(&e->btagged, w_end * sizeof(wd::tagged_t));
         if (be == cudaSuccess) be = cudaMemset(e->btagged, 0, w_end * sizeof(wd::tagged_t));
         if (be == cudaSuccess)
@@ -1163,6 +1166,7 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
         b.t_logits = e->btagged + w_logits; b.t_shact = e->btagged + w_shact; b.t_shgate = e->btagged + w_shgate;
         b.t_act = e->btagged + w_act; b.t_eo = e->btagged + w_eo; b.t_shdown = e->btagged + w_shdown;
         b.t_sel = e->btagged + w_sel;
+        b.alt_act = static_cast<unsigned>(w_act2 - w_act); b.alt_eo = static_cast<unsigned>(w_eo2 - w_eo);
     }
     *out = e;
     return WD_OK;

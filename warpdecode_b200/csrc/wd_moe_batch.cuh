@@ -27,6 +27,8 @@ namespace wd {
 constexpr int kMaxTokens = 4;
 constexpr int kBatchMaxBars = 128;
 constexpr int kBatchMaxRing = 48;
+// words of a token's selection: [0, K) picked ids, [kMaxK, kMaxK + K) weights, then whether the ids stand, then the final ids
+constexpr int kBatchSelStride = 64, kBatchSelFlag = 2 * kMaxK, kBatchSelFinal = kBatchSelFlag + 1;
 
 struct BatchParams {
     int H, F, SF, E, K, T;
@@ -53,7 +55,8 @@ struct BatchParams {
     tagged_t *t_act;             // [T * K][F]
     tagged_t *t_eo;              // [T * K][H]
     tagged_t *t_shdown;          // [T][H]
-    tagged_t *t_sel;             // [T][2 * kMaxK] picked ids (as bits), then weights
+    tagged_t *t_sel;             // [T][kBatchSelStride] picked ids (as bits), weights; WIDE: the proof's flag and the final ids too
+    unsigned alt_act, alt_eo;    // WIDE: words to the second copy of t_act / t_eo, for a batch whose picked ids were replaced
     unsigned *sync;              // the engine's status / epoch words (see MoeParams::sync)
     unsigned *host_status;
     unsigned *fallbacks;
@@ -111,6 +114,9 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cta = blockIdx.x, ncta = gridDim.x;
     const int T = P.T;
+    // WIDE: the last T CTAs pick the tokens' experts and prove the picks; they take no tiles, because nobody waits for the
+    // proof until the combine (2.5 us that every CTA used to wait for)
+    const int wcta = WIDE ? ncta - T : ncta;
     const int nbh = P.H >> 5, nbs = P.SF >> 5;
     const uint32_t lane4x2 = static_cast<uint32_t>(lane * 4) * 0x0101u;
     float *scr = reinterpret_cast<float *>(sm + P.off_scr + warp * P.scr_bytes);
@@ -140,7 +146,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     // shared-down tasks, the tokens' quantised shared activations, activation superblocks. Every one of them outside the ring completes at most once per launch.
     const int bar_rt = P.ring, bar_st = bar_rt + P.n1r, bar_tab = bar_st + P.n1s, bar_gv = bar_tab + 1, bar_x = bar_gv + 1,
               bar_sd = bar_x + 1, bar_shq = bar_sd + P.nsd, bar_act = bar_shq + kMaxTokens, n_bars = bar_act + P.n_act;
-    if (tid < n_bars) {
+    if (tid < n_bars || (WIDE && tid >= kBatchMaxBars && tid < kBatchMaxBars + n_bars)) {      // WIDE: a second set for a second attempt
         mbar_init(&bars[tid], 1);
         mbar_fence_init();
     }
@@ -162,12 +168,12 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     if (tid == 32) {         // the list does not depend on the picks: laid out while the front's copies travel
         int c2[kMaxTokens], c3[kMaxTokens];
         for (int t = 0; t < T; ++t) {
-            int ct = cta + t * (ncta / kMaxTokens);
-            if (ct >= ncta) ct -= ncta;
+            int ct = cta + t * (wcta / kMaxTokens);
+            if (ct >= wcta) ct -= wcta;
             tok_cta[t] = ct;
-            c2[t] = u_tok > ct ? (u_tok - ct + ncta - 1) / ncta : 0;
-            const int vb = static_cast<int>(static_cast<unsigned>(ct) * static_cast<unsigned>(v_tok) / static_cast<unsigned>(ncta));
-            const int ve = static_cast<int>(static_cast<unsigned>(ct + 1) * static_cast<unsigned>(v_tok) / static_cast<unsigned>(ncta));
+            c2[t] = cta < wcta && u_tok > ct ? (u_tok - ct + wcta - 1) / wcta : 0;
+            const int vb = static_cast<int>(static_cast<unsigned>(ct) * static_cast<unsigned>(v_tok) / static_cast<unsigned>(wcta));
+            const int ve = cta < wcta ? static_cast<int>(static_cast<unsigned>(ct + 1) * static_cast<unsigned>(v_tok) / static_cast<unsigned>(wcta)) : vb;
             tok_vb[t] = vb;
             tok_jl0[t] = vb >> P.t3_log2;
             c3[t] = ve - vb;
@@ -284,10 +290,11 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     // ---- the selections: CTA t picks token t's experts (the whole CTA, as in the single-token kernel) and publishes
     // ids and weights; every CTA then gathers the picks of all tokens ----
     {
-        if (cta < T) {
+        const int sel_tok = WIDE ? ncta - 1 - cta : cta;
+        if (sel_tok < T) {
             const bool h0 = tid < P.E, h1 = tid + kThreads < P.E;
             float lg[2];
-            wait_tagged<2>(P.t_logits + static_cast<size_t>(cta) * P.E + tid, kThreads, (h0 ? 1 : 0) + (h1 ? 1 : 0), tag, lg, err);
+            wait_tagged<2>(P.t_logits + static_cast<size_t>(sel_tok) * P.E + tid, kThreads, (h0 ? 1 : 0) + (h1 ? 1 : 0), tag, lg, err);
             const float l0 = lg[0], l1 = lg[1];
             RouterScratch rs;
             rs.probs = nullptr;
@@ -295,8 +302,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
             rs.red = misc + kMiscRed;
             rs.first = misc + kMiscTop;
             rs.cand = reinterpret_cast<uint32_t *>(misc + kMiscProbs);
-            int *sel_ids = ids_of(cta);
-            float *sel_w = w_of(cta);
+            int *sel_ids = ids_of(sel_tok);
+            float *sel_w = w_of(sel_tok);
+            tagged_t *out_sel = P.t_sel + sel_tok * kBatchSelStride;
+            bool ok = true, early = false;      // early: ids that the proof still has to confirm are published
             if (P.threshold_select) {
                 ThresholdScratch ts;
                 ts.gm = reinterpret_cast<uint32_t *>(misc);
@@ -311,10 +320,14 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
                 __syncthreads();
                 const int nc = *ts.cnt;
                 slow = slow || nc > 32 || nc < P.K;
-                if (!slow && warp == 0) router_threshold_rank_warp(nc, P.K, ts, sel_ids, lane);
+                if (!slow && warp == 0) {
+                    router_threshold_rank_warp(nc, P.K, ts, sel_ids, lane);
+                    if (WIDE && lane < P.K) st_tagged(out_sel + lane, __int_as_float(sel_ids[lane]), tag);
+                }
+                early = WIDE && !slow;
                 __syncthreads();
                 float p0, p1;
-                const bool ok = router_threshold_proof(l0, l1, h0, h1, P.E, P.K, P.w_scale, slow, ts, rs, sel_ids, sel_w, p0, p1);
+                ok = router_threshold_proof(l0, l1, h0, h1, P.E, P.K, P.w_scale, slow, ts, rs, sel_ids, sel_w, p0, p1);
                 if (!ok) {
                     router_rungs_cta(p0, p1, P.E, P.K, P.w_scale, rs, sel_ids, sel_w);
                     if (tid == 0 && P.fallbacks != nullptr) atomicAdd(P.fallbacks, 1u);
@@ -323,8 +336,11 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
                 router_select_cta(l0, l1, P.E, P.K, P.w_scale, rs, sel_ids, sel_w);
             }
             if (tid < P.K) {
-                st_tagged(P.t_sel + cta * 2 * kMaxK + tid, __int_as_float(sel_ids[tid]), tag);
-                st_tagged(P.t_sel + cta * 2 * kMaxK + kMaxK + tid, sel_w[tid], tag);
+                const float id = __int_as_float(sel_ids[tid]);
+                if (!early) st_tagged(out_sel + tid, id, tag);
+                st_tagged(out_sel + kMaxK + tid, sel_w[tid], tag);
+                if (WIDE) st_tagged(out_sel + kBatchSelFinal + tid, id, tag);
+                if (WIDE && tid == 0) st_tagged(out_sel + kBatchSelFlag, early && !ok ? 0.0f : 1.0f, tag);
             }
             __syncthreads();
         }
@@ -342,6 +358,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     //   desc: bit 0 down tile, 1-2 token, 3-8 pair, 9-20 tile inside the pair's matrix, 21 up tile (else gate),
     //         22-27 one more than the activation superblock this task's warp gathers afterwards (0: none)
     //   aux : gate/up tile: entry of the pair buffer; down tile: first activation superblock of its pair
+#pragma unroll 1
+    for (int attempt = 0;; ++attempt) {         // a second time only when a proof replaced picked ids (WIDE)
+    uint64_t *tbars = bars + (attempt ? kBatchMaxBars : 0);       // ring slots and activations
+    tagged_t *t_act = P.t_act + (attempt ? P.alt_act : 0u), *t_eo = P.t_eo + (attempt ? P.alt_eo : 0u);
     unsigned long long *task_src = reinterpret_cast<unsigned long long *>(sm + P.off_tasks);
     uint32_t *task_desc = reinterpret_cast<uint32_t *>(task_src + P.max_tasks);
     int *task_aux = reinterpret_cast<int *>(task_desc + P.max_tasks);
@@ -354,7 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
         unsigned long long src;
         int aux;
         if (!down) {
-            const int u = tok_cta[t] + (li >> 1) * ncta;
+            const int u = tok_cta[t] + (li >> 1) * wcta;
             const int pair = t * P.K + (u >> P.t2_log2), tile = u & ((1 << P.t2_log2) - 1);
             src = ((li & 1) ? P.up_off : P.gate_off) + static_cast<unsigned long long>(tile) * P.gu_tile;
             d = static_cast<uint32_t>(t << 1) | static_cast<uint32_t>(pair << 3) | static_cast<uint32_t>(tile << 9) |
@@ -381,12 +401,42 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
         task_desc[i] = d;
         task_aux[i] = aux;
     }
+    if constexpr (WIDE) {
+        // every thread completes the addresses of its own tasks and asks for the tiles of the first ring round at once; the
+        // ids are polled word by word, without a block-wide gather
+        if (cta == 0 && tid < T * P.K) {
+            const int t = tid / P.K, j = tid - t * P.K;
+            float v[1];
+            wait_tagged<1>(P.t_sel + t * kBatchSelStride + (attempt ? kBatchSelFinal : 0) + j, 1, 1, tag, v, err);
+            P.ids[tid] = __float_as_int(v[0]);
+        }
+        mbar_wait(&bars[bar_tab], 0, err);
+        fence_proxy_async();
+#pragma unroll 1
+        for (int k = tid; k < n_tiles; k += kThreads) {
+            const int pair = static_cast<int>((task_desc[k] >> 3) & 63u), t = static_cast<int>((task_desc[k] >> 1) & 3u);
+            float v[1];
+            wait_tagged<1>(P.t_sel + t * kBatchSelStride + (attempt ? kBatchSelFinal : 0) + (pair - t * P.K), 1, 1, tag, v, err);
+            int slot = slot_tab[__float_as_int(v[0])];
+            if (slot < 0) {
+                atomicOr(err, kErrExpertMiss);
+                slot = 0;
+            }
+            const unsigned long long src = task_src[k] + reinterpret_cast<unsigned long long>(P.pool) + static_cast<unsigned long long>(slot) * P.slot_bytes;
+            task_src[k] = src;
+            if (k < static_cast<int>(P.ring)) {
+                const unsigned bytes = (task_desc[k] & 1u) ? P.d_tile : P.gu_tile;
+                mbar_expect_tx(&tbars[k], bytes);
+                bulk_load(ring + static_cast<size_t>(k) * P.ring_slot, reinterpret_cast<const void *>(src), bytes, &tbars[k]);
+            }
+        }
+    } else
     {
         if (tid < T * 2 * kMaxK) {
             const int t = tid / (2 * kMaxK), j = tid - t * 2 * kMaxK;
             if ((j & (kMaxK - 1)) < P.K) {
                 float v[1];
-                wait_tagged<1>(P.t_sel + tid, 1, 1, tag, v, err);
+                wait_tagged<1>(P.t_sel + t * kBatchSelStride + j, 1, 1, tag, v, err);
                 if (j < kMaxK) {
                     ids_of(t)[j] = __float_as_int(v[0]);
                     if (cta == 0) P.ids[t * P.K + j] = __float_as_int(v[0]);
@@ -435,8 +485,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     // is ahead of that one which phase of the slot's barrier it may wait for.
     auto issue = [&](int i, int slot) {
         const unsigned bytes = (task_desc[i] & 1u) ? P.d_tile : P.gu_tile;
-        mbar_expect_tx(&bars[slot], bytes);
-        bulk_load(ring + static_cast<size_t>(slot) * P.ring_slot, reinterpret_cast<const void *>(task_src[i]), bytes, &bars[slot]);
+        mbar_expect_tx(&tbars[slot], bytes);
+        bulk_load(ring + static_cast<size_t>(slot) * P.ring_slot, reinterpret_cast<const void *>(task_src[i]), bytes, &tbars[slot]);
     };
     int i = warp, slot = warp, round = 0;
     auto reissue = [&]() {
@@ -452,7 +502,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
             for (unsigned it = 0; ld_acquire_shared(&ring_seq[slot]) < round; ++it)
                 if (wait_expired(it, t0, err)) break;
         }
-        mbar_wait(&bars[slot], static_cast<uint32_t>(round & 1), err);
+        mbar_wait(&tbars[slot], static_cast<uint32_t>(round & 1), err);
     };
     // activation superblock g (token g / act_per_tok, then pair of the run, then superblock): whoever asks first polls
     // the published values, quantises them to Q8_K and opens the superblock's barrier
@@ -464,17 +514,17 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
         const int t = g / act_per_tok, r = g - t * act_per_tok;
         const int pl = r / P.nsb_f, sbk = r - pl * P.nsb_f;
         float av[8];
-        wait_tagged<8>(P.t_act + static_cast<size_t>(t * P.K + tok_jl0[t] + pl) * P.F + sbk * 256 + lane, 32, 8, tag, av, err);
+        wait_tagged<8>(t_act + static_cast<size_t>(t * P.K + tok_jl0[t] + pl) * P.F + sbk * 256 + lane, 32, 8, tag, av, err);
 #pragma unroll
         for (int k = 0; k < 8; ++k) scr[lane + 32 * k] = av[k];
         __syncwarp();
         quantize_q8_K_warp(scr, lane, actk + g * kActSbStride, &actd[g]);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[bar_act + g]);
+        if (lane == 0) mbar_arrive(&tbars[bar_act + g]);
     };
-    fence_proxy_async();
+    if constexpr (!WIDE) fence_proxy_async();
     __syncthreads();
-    if (tid < min(ns, n_tiles)) issue(tid, tid);
+    if (!WIDE && tid < min(ns, n_tiles)) issue(tid, tid);
     if (tid >= 64 && tid < 64 + my_sd) {
         const int k = tid - 64;
         mbar_expect_tx(&bars[bar_sd + k], sd_bytes);
@@ -485,7 +535,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     // The shared expert's activation of token t (published by the row tasks long ago) -> Q8_0, by warp 15 - t while the
     // first tiles are on their way; the floats pass through the memory of the token's Q8_0 quants of x, which only
     // the row tasks read. The shared-down tasks at the end of the list wait on the token's barrier.
-    if (P.SF > 0 && warp >= kWarps - T) {
+    if (P.SF > 0 && warp >= kWarps - T && attempt == 0) {
         const int t = kWarps - 1 - warp;
         float *sf = reinterpret_cast<float *>(xq0_of(t));
 #pragma unroll 1
@@ -530,15 +580,19 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
                 }
                 second = __shfl_sync(0xffffffffu, second, 0);
                 __syncwarp();       // orders the other lanes' reads of the buffer after lane 0's acquire
-                if (second && lane < R2)
-                    st_tagged(P.t_act + static_cast<size_t>(pair) * P.F + tile * R2 + lane, __fmul_rn(silu_ggml(buf[lane]), buf[R2 + lane]), tag);
+                if (second && lane < R2) {
+                    const float v = __fmul_rn(silu_ggml(buf[lane]), buf[R2 + lane]);
+                    const size_t at = static_cast<size_t>(pair) * P.F + tile * R2 + lane;
+                    st_tagged(t_act + at, v, tag);
+                    if (WIDE && attempt) st_tagged(P.t_act + at, v, tag);       // for inspection; the first attempt's values are dead
+                }
             } else {
                 // the pair's activations: normally gathered a round ago; else the first warp to need a superblock does it
 #pragma unroll 1
                 for (int sk = 0; sk < P.nsb_f; ++sk) {
-                    if (!mbar_try_wait(&bars[bar_act + aux + sk], 0)) {
+                    if (!mbar_try_wait(&tbars[bar_act + aux + sk], 0)) {
                         gather(aux + sk);
-                        mbar_wait(&bars[bar_act + aux + sk], 0, err);
+                        mbar_wait(&tbars[bar_act + aux + sk], 0, err);
                     }
                 }
                 const int ab = aux + sb3;
@@ -547,8 +601,11 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
                                       rows_a);
                 reissue();
 #pragma unroll 1
-                for (int rr = lane; rr < R3; rr += 32)
-                    st_tagged(P.t_eo + static_cast<size_t>(pair) * P.H + tile * R3 + rr, rows_a[rr], tag);
+                for (int rr = lane; rr < R3; rr += 32) {
+                    const size_t at = static_cast<size_t>(pair) * P.H + tile * R3 + rr;
+                    st_tagged(t_eo + at, rows_a[rr], tag);
+                    if (WIDE && attempt) st_tagged(P.t_eo + at, rows_a[rr], tag);
+                }
                 __syncwarp();
             }
             const int job = static_cast<int>((d >> 22) & 63u);
@@ -569,6 +626,32 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
         }
     }
 
+    if constexpr (WIDE) {
+        // the proofs' flags and the weights (written while the first tiles travelled); all CTAs see the same flags
+        if (tid < T * 32) {
+            const int t = tid >> 5;
+            float v[2];
+            wait_tagged<1>(P.t_sel + t * kBatchSelStride + kMaxK + lane, 1, lane <= kMaxK ? (lane < P.K || lane == kMaxK ? 1 : 0) : 0, tag, v, err);
+            if (lane < P.K) {
+                w_of(t)[lane] = v[0];
+                if (cta == 0) P.weights[t * P.K + lane] = v[0];
+            }
+            if (lane == kMaxK) misc[t] = v[0];
+        }
+        __syncthreads();
+        bool redo = false;
+        for (int t = 0; t < T; ++t) redo = redo || misc[t] == 0.0f;
+        if (redo && attempt == 0) {
+            // every copy of this CTA has landed and been consumed: fresh barriers and counters, then the tiles once more
+            __syncthreads();
+            if (tid < static_cast<int>(P.ring)) ring_seq[tid] = 0;
+            if (tid < 32) unit_cnt[tid] = 0;
+            if (tid < static_cast<int>(P.n_act)) act_state[tid] = 0;
+            my_sd = 0;                      // the shared expert's rows stand
+            __syncthreads();
+            continue;
+        }
+    }
     WD_BSTAMP(10);
     // ---- combine: this CTA's band of output rows, for every token ----------------------------------------------
     {
@@ -578,7 +661,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
         if (t < T && row < P.H && !stopped) {
             const float *sel_w = w_of(t);
             tagged_t w[kMaxK] = {}, wsd = 0, wsg = 0;
-            const tagged_t *src = P.t_eo + static_cast<size_t>(t) * P.K * P.H + row;
+            const tagged_t *src = t_eo + static_cast<size_t>(t) * P.K * P.H + row;
             unsigned long long t0 = 0ull;
             for (unsigned it = 0;; ++it) {
 #pragma unroll
@@ -603,6 +686,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
             if (P.SF > 0) o = __fadd_rn(acc, __fmul_rn(__uint_as_float(static_cast<uint32_t>(wsd)), __uint_as_float(static_cast<uint32_t>(wsg))));
             P.out[static_cast<size_t>(t) * P.H + row] = o;
         }
+    }
+    break;
     }
     WD_BSTAMP(11);
     __syncthreads();
