@@ -146,13 +146,11 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     // shared-down tasks, the tokens' quantised shared activations, activation superblocks. Every one of them outside the ring completes at most once per launch.
     const int bar_rt = P.ring, bar_st = bar_rt + P.n1r, bar_tab = bar_st + P.n1s, bar_gv = bar_tab + 1, bar_x = bar_gv + 1,
               bar_sd = bar_x + 1, bar_shq = bar_sd + P.nsd, bar_act = bar_shq + kMaxTokens, n_bars = bar_act + P.n_act;
-    if (tid < n_bars || (WIDE && tid >= kBatchMaxBars && tid < kBatchMaxBars + n_bars)) {      // WIDE: a second set for a second attempt
-        mbar_init(&bars[tid], 1);
-        mbar_fence_init();
+    if (warp == 1) {
+        for (int b = lane; b < static_cast<int>(P.ring); b += 32) ring_seq[b] = 0;
+        unit_cnt[lane] = 0;
+        for (int b = lane; b < static_cast<int>(P.n_act); b += 32) act_state[b] = 0;
     }
-    if (tid < static_cast<int>(P.ring)) ring_seq[tid] = 0;
-    if (tid < 32) unit_cnt[tid] = 0;
-    if (tid < static_cast<int>(P.n_act)) act_state[tid] = 0;
     if (cta == 0 && tid == 0) P.sync[5] = smem_u32(bars);
     const int u_tok = P.K << P.t2_log2, v_tok = P.K << P.t3_log2;      // gate/up units and down tiles of one token
     const int n_exp_tok = static_cast<int>(P.n_act) / (kMaxTokens * P.nsb_f);     // pairs a run may touch (planned maximum)
@@ -164,8 +162,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     int *seg_begin = reinterpret_cast<int *>(sm + P.off_seg);          // [2T + 1] first task of every segment
     int *seg_info = seg_begin + 9;                                     // [2T] token * 2 + (1: down tiles)
     int *tok_cta = seg_begin + 17, *tok_vb = seg_begin + 21, *tok_jl0 = seg_begin + 25, *tok_ng = seg_begin + 29;
-    __syncthreads();
-    if (tid == 32) {         // the list does not depend on the picks: laid out while the front's copies travel
+    if (tid == 64) {         // the list does not depend on the picks: laid out while the front's copies travel
         int c2[kMaxTokens], c3[kMaxTokens];
         for (int t = 0; t < T; ++t) {
             int ct = cta + t * (wcta / kMaxTokens);
@@ -200,7 +197,14 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     const unsigned rt_bytes = static_cast<unsigned>(nbh) * 136u, a1_slot = 2u * rt_bytes;
     uint8_t *gate_vec_stage = ring + static_cast<size_t>(P.n1r + P.n1s) * a1_slot;
     const float *xs = reinterpret_cast<const float *>(gate_vec_stage + static_cast<size_t>(P.H) * 4);   // [T][H]
-    if (warp == 0) {
+    const int first_st = (wcta - 1 - cta + ncta) % ncta;        // the shared tasks go round from the end; the CTAs that pick come last
+    if (warp == 0) {         // the warp that asks for the front's copies sets their barriers up itself and waits for nobody
+        for (int b = lane; b < n_bars; b += 32) {
+            mbar_init(&bars[b], 1);
+            if (WIDE) mbar_init(&bars[kBatchMaxBars + b], 1);       // a second set for a second attempt
+        }
+        mbar_fence_init();
+        __syncwarp();
         if (lane == 2) {
             const unsigned xb = static_cast<unsigned>(T) * static_cast<unsigned>(P.H) * 4u;
             mbar_expect_tx(&bars[bar_x], xb);
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
             }
         }
         for (int s = lane; s < static_cast<int>(P.n1s); s += 32) {
-            const int t = ncta - 1 - cta + s * ncta;
+            const int t = first_st + s * ncta;
             if (t < n_st) {
                 uint8_t *dst = ring + (P.n1r + s) * a1_slot;
                 mbar_expect_tx(&bars[bar_st + s], 2u * rt_bytes);
@@ -237,22 +241,37 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     }
 
     WD_BSTAMP(1);
-    // ---- the T activations: Q8_0 (router, shared expert) and Q8_K (routed experts) ----------------------------
-    mbar_wait(&bars[bar_x], 0, err);
-    if ((tid >> 7) < T)     // 128 threads per token
-        quantize_q8_0_part(xs + static_cast<size_t>(tid >> 7) * P.H, P.H, xq0_of(tid >> 7), xd0_of(tid >> 7), tid & 127, 128);
-#pragma unroll 1
-    for (int w = warp; w < T * P.nsb_h; w += kWarps) {
-        const int t = w / P.nsb_h, sb = w - t * P.nsb_h;
-        quantize_q8_K_warp(xs + static_cast<size_t>(t) * P.H + sb * 256, lane, xk_of(t) + sb * kActSbStride, &xdk_of(t)[sb]);
+    __syncthreads();        // barriers and counters are set up
+    if (tid == 3 * 32) {
+        // every thread of this CTA has read the epoch; the CTA that comes last knows that of all of them and advances it,
+        // here, where everybody waits for the activations, rather than at the end of the launch (fence and atomic: 2 us)
+        __threadfence();
+        if (atomicAdd(P.sync + 9, 1u) == static_cast<unsigned>(ncta) - 1u) {
+            P.sync[9] = 0u;
+            P.sync[8] = epoch + 1u;
+        }
     }
+    // ---- the T activations: Q8_0 (router, shared expert) and Q8_K (routed experts). With wide tiles the Q8_K form waits
+    // until the row tasks are done: it is first needed by the tiles, and everybody then waits for the picks ----
+    mbar_wait(&bars[bar_x], 0, err);
+    {
+        const int per = T == 1 ? 512 : T == 2 ? 256 : 128, t = tid / per;
+        if (t < T) quantize_q8_0_part(xs + static_cast<size_t>(t) * P.H, P.H, xq0_of(t), xd0_of(t), tid & (per - 1), per);
+    }
+    auto quantise_routed = [&]() {
+#pragma unroll 1
+        for (int w = warp; w < T * P.nsb_h; w += kWarps) {
+            const int t = w / P.nsb_h, sb = w - t * P.nsb_h;
+            quantize_q8_K_warp(xs + static_cast<size_t>(t) * P.H + sb * 256, lane, xk_of(t) + sb * kActSbStride, &xdk_of(t)[sb]);
+        }
+    };
+    if constexpr (!WIDE) quantise_routed();
     __syncthreads();
 
     WD_BSTAMP(2);
     // ---- row tasks: every staged row task meets all T activations, one warp per (task, token) ------------------
     {
         const int my_rt = cta < n_rt ? (n_rt - cta + ncta - 1) / ncta : 0;
-        const int first_st = ncta - 1 - cta;
         const int my_st = first_st < n_st ? (n_st - first_st + ncta - 1) / ncta : 0;
 #pragma unroll 1
         for (int it = warp; it < (my_rt + my_st) * T; it += kWarps) {
@@ -283,6 +302,9 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
         }
     }
 
+    if constexpr (WIDE) {
+        if (cta < wcta) quantise_routed();      // the CTAs that pick have no tiles
+    }
     WD_BSTAMP(3);
     __syncthreads();        // the staged rows are not read any more: their memory becomes the ring
     WD_BSTAMP(4);
@@ -653,6 +675,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
         }
     }
     WD_BSTAMP(10);
+    // the error word as of this warp's last wait but the combine's own; asked for here, looked at when the warp leaves
+    unsigned st = lane == 0 ? *reinterpret_cast<volatile unsigned *>(err) : 0u;
     // ---- combine: this CTA's band of output rows, for every token ----------------------------------------------
     {
         const int rpc = (P.H + ncta - 1) / ncta;
@@ -675,7 +699,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
 #pragma unroll
                 for (int q = 0; q < kMaxK; ++q) bad |= (q < P.K) & tag_behind(w[q], tag);
                 if (!bad) break;
-                if (wait_expired(it, t0, err)) break;
+                if (wait_expired(it, t0, err)) {
+                    st |= kErrBarrierTimeout;
+                    break;
+                }
             }
             float acc = 0.0f;
 #pragma unroll
@@ -687,22 +714,12 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
             P.out[static_cast<size_t>(t) * P.H + row] = o;
         }
     }
+    if (st != 0u && P.host_status != nullptr) *P.host_status = *reinterpret_cast<volatile unsigned *>(err);    // a write over PCIe: only when there is news
     break;
     }
     WD_BSTAMP(11);
-    __syncthreads();
     WD_BSTAMP(12);
 #undef WD_BSTAMP
-    if (tid == 0) {
-        __threadfence();
-        if (atomicAdd(P.sync + 9, 1u) == static_cast<unsigned>(ncta) - 1u) {
-            P.sync[9] = 0u;
-            P.sync[8] = epoch + 1u;
-            __threadfence();
-            const unsigned st = *reinterpret_cast<volatile unsigned *>(err);
-            if (P.host_status && st) *P.host_status = st;      // a write over PCIe that the launch would wait for: only when there is news
-        }
-    }
 }
 
 }  // namespace wd
