@@ -58,3 +58,26 @@ def test_prompt_pass_equals_the_one_token_steps(wd, oracle, H, nh, nkv, hd, F, L
     again, _ = dec.decode(prompt[:max(2, P // 2)], 1)          # a shorter prompt on the used caches and workspace
     assert np.array_equal(again, ref.decode(prompt[:max(2, P // 2)], 1))
     dec.close()
+
+
+@pytest.mark.parametrize("H,hd,F,V,q8", [(4096, 128, 64, 700, False),           # the norm's elements in two passes over the threads
+                                         (4096, 128, 96, 9441, True), (256, 64, 512, 9441, False),       # two head rows per warp, a ragged end
+                                         (512, 64, 320, 20003, False), (512, 64, 320, 20003, True)])     # four rows per warp, a walk over the rows
+def test_norm_and_product_in_one_kernel(wd, oracle, H, hd, F, V, q8):
+    from warpdecode_b200 import synth
+    cfg = dict(hidden=H, n_heads=2, n_kv_heads=1, head_dim=hd, ffn=F, vocab=V, n_layers=2, max_ctx=12, rms_eps=1e-5)
+    dec = wd.DenseDecoder(H, 2, 1, hd, F, V, 2, 12, 1e-5, 500000.0)
+    dec.synth(3, 0.05)
+    rng = np.random.Generator(np.random.PCG64(V))
+    if q8:
+        for l, which in ((0, wd.DT_W_GATE_UP), (1, wd.DT_WQKV), (-1, wd.DT_OUTPUT)):
+            w = (rng.standard_normal(dec.shape(which)) * 0.05).astype(np.float32)
+            dec.set_tensor(l, which, synth.quantize_q8_0(w).reshape(-1), wd.TYPE_Q8_0)
+    prompt = rng.integers(0, V, 3)
+    got, _ = dec.decode(prompt, 6)
+    logits, hidden = dec.read()
+    ref = _oracle_for(wd, oracle, dec, cfg, 500000.0)
+    assert np.array_equal(got, ref.decode(prompt, 6))
+    assert np.array_equal(ol.fbits(logits), ol.fbits(ref.logits))
+    assert np.array_equal(ol.fbits(hidden), ol.fbits(ref.hidden))
+    dec.close()

@@ -105,186 +105,234 @@ __device__ __forceinline__ void store_quant4(PairedQuant *out, int e, uint32_t p
     *reinterpret_cast<uint32_t *>(out + (e & ~31) + paired_place(e & 31)) = packed;
 }
 
-// hidden += proj (when given); y = RMSNorm(hidden) * w -> Q8_0 (plain layout: int8 [n], float scale per block), by one CTA of
-// n / 4 threads, n = 256 * 2^k up to 4096: thread t owns elements 4 t .. 4 t + 3, a Q8_0 block eight neighbouring lanes
-// (residual_rmsnorm_kernel, src/warodecode.cu:1408). The sum of squares is the binary tree in double of the MoE stack's
-// RMSNorm. `embd_row` (optional): the step starts here, and hidden is first filled with the token's embedding row
-// (embedding_q4_kernel). `wait`: what the norm weights, which no kernel writes, are fetched in front of.
-// Bound: latency (a chain of one load, two reductions and two divisions, run once); 256 threads with eight elements each and
-// scalar loads took 3.2 us per call inside the step.
-template <class Quant, class Wait>
-__device__ __forceinline__ void dense_norm_quant_body(float *hidden, const float *proj, const float *w, int n, float eps, Quant *xq,
-                                                      float *xd, const uint8_t *embd, const int *token, int vocab, bool embd_q8, Wait wait) {
+// hidden_out = hidden + proj (proj: when given; hidden_out: when given); y = RMSNorm(that) * w -> Q8_0 (int8 [n], float scale per
+// block), by one CTA, n = 256 * 2^k up to 4096: with blockDim.x threads, thread t owns elements 4 t .. 4 t + 3 (of every
+// 4 * blockDim.x), a Q8_0 block eight neighbouring lanes (residual_rmsnorm_kernel, src/warodecode.cu:1408). The sum of squares
+// is the binary tree in double of the MoE stack's RMSNorm. `embd` (optional): the step starts here, and the token's embedding
+// row takes the place of hidden (embedding_q4_kernel). `wait`: what the norm weights, which no kernel writes, are fetched in
+// front of. PASSES: ceil(n / (4 * blockDim.x)). store(e, packed, d): four quants from element e on, and their block's scale.
+// Bound: latency (a chain of one load, two reductions and two divisions). One warp finishes the sum: done by all 16, the
+// double-precision pipe is busy for longer than the second barrier takes.
+struct NormInput {
+    const float *hidden, *proj, *w;     // proj, w: nullable
+    float *hidden_out;                  // nullable
+    const uint8_t *embd;                // nullable: embedding table in ggml layout, Q4_0 blocks of 18 bytes or Q8_0 blocks of 34
+    const int *token;
+    float eps;
+    int n, vocab, embd_q8;
+};
+template <int PASSES, class Wait, class Store>
+__device__ __forceinline__ void dense_norm_quant_body(const NormInput &in, Wait wait, Store store) {
     __shared__ double red[32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5, e0 = tid * 4;
-    const float4 nw = w != nullptr ? *reinterpret_cast<const float4 *>(w + e0) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    __shared__ float scale_s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = in.n;
+    float v[PASSES][4];
+    float4 nw[PASSES];
+#pragma unroll
+    for (int p = 0; p < PASSES; ++p) {
+        const int e0 = (p * blockDim.x + tid) * 4;
+        nw[p] = in.w != nullptr && e0 < n ? *reinterpret_cast<const float4 *>(in.w + e0) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    }
     wait();
-    float v[4];
-    if (embd != nullptr) {
-        const int bytes = embd_q8 ? 34 : 18, j = e0 & 31;
-        const uint8_t *wb = embd + (static_cast<size_t>(max(0, min(vocab - 1, *token))) * (n >> 5) + (e0 >> 5)) * bytes;
-        const float d = half_bits_to_float(static_cast<uint16_t>(wb[0] | (wb[1] << 8)));
+#pragma unroll
+    for (int p = 0; p < PASSES; ++p) {
+        const int e0 = (p * blockDim.x + tid) * 4;
+        if (e0 >= n) {                      // whole warps: n is a multiple of 256
+            v[p][0] = v[p][1] = v[p][2] = v[p][3] = 0.0f;
+        } else if (in.embd != nullptr) {
+            const int bytes = in.embd_q8 ? 34 : 18, j = e0 & 31;
+            const uint8_t *wb = in.embd + (static_cast<size_t>(max(0, min(in.vocab - 1, *in.token))) * (n >> 5) + (e0 >> 5)) * bytes;
+            const float d = half_bits_to_float(static_cast<uint16_t>(wb[0] | (wb[1] << 8)));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int q = in.embd_q8 ? static_cast<int>(static_cast<int8_t>(wb[2 + j + i]))
+                                         : (j < 16 ? (wb[2 + j + i] & 0x0f) : (wb[2 + j + i - 16] >> 4)) - 8;
+                v[p][i] = __fmul_rn(d, static_cast<float>(q));
+            }
+        } else {
+            const float4 h = *reinterpret_cast<const float4 *>(in.hidden + e0);
+            v[p][0] = h.x; v[p][1] = h.y; v[p][2] = h.z; v[p][3] = h.w;
+            if (in.proj != nullptr) {
+                const float4 q = *reinterpret_cast<const float4 *>(in.proj + e0);
+                v[p][0] = __fadd_rn(v[p][0], q.x);
+                v[p][1] = __fadd_rn(v[p][1], q.y);
+                v[p][2] = __fadd_rn(v[p][2], q.z);
+                v[p][3] = __fadd_rn(v[p][3], q.w);
+            }
+        }
+        if (in.hidden_out != nullptr && e0 < n) *reinterpret_cast<float4 *>(in.hidden_out + e0) = make_float4(v[p][0], v[p][1], v[p][2], v[p][3]);
+        double sq[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sq[i] = __dmul_rn(static_cast<double>(v[p][i]), static_cast<double>(v[p][i]));
+        double ss = __dadd_rn(__dadd_rn(sq[0], sq[1]), __dadd_rn(sq[2], sq[3]));
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, s));
+        if (lane == 0 && e0 < n) red[p * (blockDim.x >> 5) + warp] = ss;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double ss = lane < (n >> 7) ? red[lane] : 0.0;      // a power of two of warps; adding +0.0 beyond them changes nothing
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, s));
+        // n is a power of two: the division by it is an exact multiplication
+        const double inv_n = __longlong_as_double(static_cast<long long>(1023 - (31 - __clz(n))) << 52);
+        if (lane == 0) scale_s = __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dmul_rn(ss, inv_n), static_cast<double>(in.eps)))));
+    }
+    __syncthreads();
+    const float scale = scale_s;
+#pragma unroll
+    for (int p = 0; p < PASSES; ++p) {
+        const int e0 = (p * blockDim.x + tid) * 4;
+        if (e0 >= n) break;
+        const float g[4] = {nw[p].x, nw[p].y, nw[p].z, nw[p].w};
+        float amax = 0.0f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int q = embd_q8 ? static_cast<int>(static_cast<int8_t>(wb[2 + j + i]))
-                                  : (j < 16 ? (wb[2 + j + i] & 0x0f) : (wb[2 + j + i - 16] >> 4)) - 8;
-            v[i] = __fmul_rn(d, static_cast<float>(q));
+            v[p][i] = __fmul_rn(v[p][i], scale);
+            if (in.w != nullptr) v[p][i] = __fmul_rn(v[p][i], g[i]);
+            amax = fmaxf(amax, fabsf(v[p][i]));
         }
-    } else {
-        const float4 h = *reinterpret_cast<const float4 *>(hidden + e0);
-        v[0] = h.x; v[1] = h.y; v[2] = h.z; v[3] = h.w;
-        if (proj != nullptr) {
-            const float4 p = *reinterpret_cast<const float4 *>(proj + e0);
-            v[0] = __fadd_rn(v[0], p.x);
-            v[1] = __fadd_rn(v[1], p.y);
-            v[2] = __fadd_rn(v[2], p.z);
-            v[3] = __fadd_rn(v[3], p.w);
+#pragma unroll
+        for (int s = 1; s < 8; s <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
+        const float inv = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+        uint32_t packed = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            int q = amax != 0.0f ? __float2int_rn(__fmul_rn(v[p][i], inv)) : 0;
+            q = max(-128, min(127, q));
+            packed |= static_cast<uint32_t>(q & 0xff) << (8 * i);
         }
+        store(e0, packed, __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f))));
     }
-    if (embd != nullptr || proj != nullptr) *reinterpret_cast<float4 *>(hidden + e0) = make_float4(v[0], v[1], v[2], v[3]);
-    double sq[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) sq[i] = __dmul_rn(static_cast<double>(v[i]), static_cast<double>(v[i]));
-    double ss = __dadd_rn(__dadd_rn(sq[0], sq[1]), __dadd_rn(sq[2], sq[3]));
-#pragma unroll
-    for (int s = 1; s < 32; s <<= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, s));
-    if (lane == 0) red[warp] = ss;
-    __syncthreads();
-    ss = lane < nwarps ? red[lane] : 0.0;           // a power of two of warps; adding +0.0 beyond them changes nothing
-#pragma unroll
-    for (int s = 1; s < 32; s <<= 1) ss = __dadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, s));
-    // n is a power of two: the division by it is an exact multiplication
-    const double inv_n = __longlong_as_double(static_cast<long long>(1023 - (31 - __clz(n))) << 52);
-    const float scale = __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dmul_rn(ss, inv_n), static_cast<double>(eps)))));
-    const float g[4] = {nw.x, nw.y, nw.z, nw.w};
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        v[i] = __fmul_rn(v[i], scale);
-        if (w != nullptr) v[i] = __fmul_rn(v[i], g[i]);
-        amax = fmaxf(amax, fabsf(v[i]));
-    }
-#pragma unroll
-    for (int s = 1; s < 8; s <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
-    const float inv = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-    uint32_t packed = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int q = amax != 0.0f ? __float2int_rn(__fmul_rn(v[i], inv)) : 0;
-        q = max(-128, min(127, q));
-        packed |= static_cast<uint32_t>(q & 0xff) << (8 * i);
-    }
-    store_quant4(xq, e0, packed);
-    if ((lane & 7) == 0) xd[e0 >> 5] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
 }
 
-__global__ void __launch_bounds__(1024) dense_norm_quant_kernel(float *hidden, const float *proj, const float *w, int n, float eps, int8_t *xq,
-                                                               float *xd, const uint8_t *embd, const int *token, int vocab, int embd_q8) {
-    grid_dep_launch();
-    // the embedding table in ggml layout: Q4_0 blocks of 18 bytes, or Q8_0 blocks of 34
-    dense_norm_quant_body(hidden, proj, w, n, eps, xq, xd, embd, token, vocab, embd_q8 != 0, [] { grid_dep_wait(); });
+__device__ __forceinline__ int dp4a_u8s8(uint32_t a, int b, int c) {
+    int d;
+    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
 }
 
-// y = W x: W Q4_0 in the row layout, x already Q8_0 (plain layout, copied into shared memory once per CTA).
-// One warp per row at a time (grid-stride over the rows); see the header for the order. When `key` is given the
-// kernel also folds the arg-max of the finite results into it (one atomicMax per warp): key = order_key(value) << 32
-// | ~row, so the largest value wins and ties go to the lowest row (dense_argmax_reduce_kernel, :1603-1632).
-// Dynamic shared memory: nb * 32 bytes of quants + nb floats.
-// R rows per warp at once, U blocks per lane and row in flight: R * U 16-byte loads are issued before the first is
-// used. Small matrices take R = 1 and one warp per row, so that every byte of the matrix is requested at once; the
-// output head takes R = 4 and walks its rows grid-stride.
-template <int R, int U>
-__global__ void __launch_bounds__(kDecThreads, 4) dense_gemv_q4_0_kernel(const uint8_t *wp, int rows, int nb, const int8_t *xq,
-                                                                       const float *xd, float *y, unsigned long long *key) {
+// The activation in shared memory as the products read it, nb blocks: their first halves, their second halves (neighbouring
+// lanes read neighbouring 16 bytes), then (scale, -8 * sum) per block.
+struct BlockInput {
+    uint4 *lo, *hi;
+    int2 *x;
+    __device__ __forceinline__ BlockInput(uint8_t *sm, int nb)
+        : lo(reinterpret_cast<uint4 *>(sm)), hi(lo + nb), x(reinterpret_cast<int2 *>(hi + nb)) {}
+    static constexpr int kBlockBytes = 40;
+};
+
+// Weights that a later kernel of the step reads, asked into L2 by one that has its own loads under way: left to themselves they
+// cross DRAM only while the kernel that needs them runs, which is half of the step. Up to two ranges, in pieces of 4 KB, one lane per
+// piece. The qkv product asks for the layer's gate/up matrix, wo for w_down, gate/up for the next layer's qkv and wo.
+struct L2Ahead {
+    const uint8_t *p[2];
+    unsigned bytes[2];          // multiples of 16
+    __device__ __forceinline__ void request() const {
+        constexpr unsigned kPiece = 4096;
+        if ((threadIdx.x & 31) != 0) return;
+        const unsigned warp = threadIdx.x >> 5, first = warp * gridDim.x + blockIdx.x, step = (blockDim.x >> 5) * gridDim.x;
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            for (unsigned i = first; i < (bytes[k] + kPiece - 1) / kPiece; i += step) {
+                const unsigned n = min(kPiece, bytes[k] - i * kPiece);
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p[k] + static_cast<size_t>(i) * kPiece), "r"(n) : "memory");
+            }
+    }
+};
+
+// A block of 32 weights of a packed matrix, and its term of a row's chain: fmaf(d_w * d_x, (float)int_dot, acc).
+template <bool Q8>
+struct RowBlock {
+    uint4 q[Q8 ? 2 : 1];
+    uint16_t d;
+    __device__ __forceinline__ void load(const uint4 *quants, const uint16_t *scales, size_t blk) {
+#pragma unroll
+        for (int i = 0; i < (Q8 ? 2 : 1); ++i) q[i] = __ldg(quants + (Q8 ? 2 : 1) * blk + i);
+        d = __ldg(scales + blk);
+    }
+    // lo, hi: quants 0 .. 15 and 16 .. 31 of the activation's block; x: its scale (as bits) and -8 times the sum of its quants
+    __device__ __forceinline__ float term(const uint4 &lo, const uint4 &hi, const int2 &x, float acc) const {
+        const int al[4] = {static_cast<int>(lo.x), static_cast<int>(lo.y), static_cast<int>(lo.z), static_cast<int>(lo.w)};
+        const int ah[4] = {static_cast<int>(hi.x), static_cast<int>(hi.y), static_cast<int>(hi.z), static_cast<int>(hi.w)};
+        const uint32_t w0[4] = {q[0].x, q[0].y, q[0].z, q[0].w};
+        int s = 0;
+        if constexpr (Q8) {
+            const uint32_t w1[4] = {q[1].x, q[1].y, q[1].z, q[1].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                s = dp4a_s8(static_cast<int>(w0[k]), al[k], s);
+                s = dp4a_s8(static_cast<int>(w1[k]), ah[k], s);
+            }
+        } else {        // sum (q - 8) a = sum q a - 8 sum a, unsigned nibbles; the high ones where they are, worth 16 times as much
+            int s_hi = 0;
+            s = x.y;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                s = dp4a_u8s8(w0[k] & 0x0f0f0f0fu, al[k], s);
+                s_hi = dp4a_u8s8(w0[k] & 0xf0f0f0f0u, ah[k], s_hi);
+            }
+            s += s_hi >> 4;
+        }
+        return __fmaf_rn(__fmul_rn(half_bits_to_float(d), __int_as_float(x.x)), static_cast<float>(s), acc);
+    }
+};
+
+// y = W x: W in the row layout, x already Q8_0 (plain layout, copied into shared memory once per CTA), one warp per row; see
+// the header for the order. A Q8_0 block (what every 2-D tensor of a model file that is not Q4_0 becomes: planarize_q4,
+// src/warodecode.cu:1027-1075) is two 16-byte loads, a Q4_0 block one. Dynamic shared memory: nb * 40
+// bytes. U blocks per lane in flight: with one warp per row every byte of the matrix is requested at once.
+template <bool Q8, int U>
+__global__ void __launch_bounds__(kDecThreads, 4) dense_product_kernel(const uint8_t *wp, int rows, int nb, const int8_t *xq, const float *xd,
+                                                                      float *y, L2Ahead ahead) {
     extern __shared__ __align__(16) uint8_t dsm[];
     grid_dep_launch();
-    uint4 *sq = reinterpret_cast<uint4 *>(dsm);
-    float *sd = reinterpret_cast<float *>(dsm + static_cast<size_t>(nb) * 32);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const BlockInput in(dsm, nb);
+    const int lane = threadIdx.x & 31, row = blockIdx.x * (kDecThreads / 32) + (threadIdx.x >> 5), stride = dense_row_stride(nb);
     const uint4 *q_all = reinterpret_cast<const uint4 *>(wp);
-    const int stride = dense_row_stride(nb);
-    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * stride * 16);
-    uint4 w[R][U];
-    uint16_t dw[R][U];
-    auto load = [&](int row0, int b0) {
+    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * stride * (Q8 ? 32 : 16));
+    RowBlock<Q8> w[U];
+    auto load = [&](int b0) {
 #pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int b = b0 + 32 * u;
-                if (b < nb && row0 + r < rows) {
-                    w[r][u] = __ldg(q_all + static_cast<size_t>(row0 + r) * stride + b);
-                    dw[r][u] = __ldg(d_all + static_cast<size_t>(row0 + r) * stride + b);
-                }
-            }
+        for (int u = 0; u < U; ++u)
+            if (b0 + 32 * u < nb && row < rows) w[u].load(q_all, d_all, static_cast<size_t>(row) * stride + b0 + 32 * u);
     };
     // The weights do not depend on the kernel before this one: the first loads leave before the wait for it, and the
     // activation (its output) is fetched after.
-    const int row_first = (blockIdx.x * nwarps + warp) * R;
-    if (row_first < rows) load(row_first, lane);
+    load(lane);
+    ahead.request();
     grid_dep_wait();
-    for (int i = threadIdx.x; i < nb * 2; i += blockDim.x) sq[i] = reinterpret_cast<const uint4 *>(xq)[i];
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) sd[i] = xd[i];
+#pragma unroll 2
+    for (int i = threadIdx.x; i < ((nb * 2 + 31) & ~31); i += kDecThreads) {        // half a block per thread; whole warps
+        const int b = i >> 1;
+        const uint4 v = b < nb ? reinterpret_cast<const uint4 *>(xq)[i] : make_uint4(0, 0, 0, 0);
+        const float d = b < nb ? xd[b] : 0.0f;
+        int sum = dp4a_s8(static_cast<int>(v.x), 0x01010101, dp4a_s8(static_cast<int>(v.y), 0x01010101, 0));
+        sum = dp4a_s8(static_cast<int>(v.z), 0x01010101, dp4a_s8(static_cast<int>(v.w), 0x01010101, sum));
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        if (b < nb) {
+            ((i & 1) ? in.hi : in.lo)[b] = v;
+            if ((i & 1) == 0) in.x[b] = make_int2(__float_as_int(d), -8 * sum);
+        }
+    }
     __syncthreads();
-    unsigned long long best = 0ull;
-    for (int row0 = row_first; row0 < rows; row0 += gridDim.x * nwarps * R) {
-        float acc[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+    if (row >= rows) return;
+    float acc = 0.0f;
 #pragma unroll 1
-        for (int b0 = lane; b0 < nb; b0 += 32 * U) {
-            if (row0 != row_first || b0 != lane) load(row0, b0);
+    for (int b0 = lane; b0 < nb; b0 += 32 * U) {
+        if (b0 != lane) load(b0);
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int b = b0 + 32 * u;
-                if (b < nb) {
-                    const uint4 lo = sq[2 * b], hi = sq[2 * b + 1];
-                    const uint32_t al[4] = {lo.x, lo.y, lo.z, lo.w}, ah[4] = {hi.x, hi.y, hi.z, hi.w};
-                    const float dx = sd[b];
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        if (row0 + r < rows) {
-                            const uint32_t ww[4] = {w[r][u].x, w[r][u].y, w[r][u].z, w[r][u].w};
-                            int s16 = 0;    // 16 * sum of (q - 8) * a: a nibble at the top of its byte with the top bit flipped
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                s16 = dp4a_s8(static_cast<int>(((ww[k] << 4) & 0xf0f0f0f0u) ^ 0x80808080u), static_cast<int>(al[k]), s16);
-                                s16 = dp4a_s8(static_cast<int>((ww[k] & 0xf0f0f0f0u) ^ 0x80808080u), static_cast<int>(ah[k]), s16);
-                            }
-                            acc[r] = __fmaf_rn(__fmul_rn(half_bits_to_float(dw[r][u]), dx), static_cast<float>(s16 >> 4), acc[r]);
-                        }
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-#pragma unroll
-            for (int s = 16; s >= 1; s >>= 1) acc[r] = __fadd_rn(acc[r], __shfl_xor_sync(0xffffffffu, acc[r], s));
-        }
-        if (lane < R && row0 + lane < rows) {
-            float v = acc[0];
-#pragma unroll
-            for (int r = 1; r < R; ++r) v = lane == r ? acc[r] : v;
-            y[row0 + lane] = v;
-            if (key != nullptr && v == v && fabsf(v) != INFINITY) {
-                const unsigned long long k =
-                    (static_cast<unsigned long long>(order_key(v)) << 32) | (0xffffffffu - static_cast<unsigned>(row0 + lane));
-                best = k > best ? k : best;
-            }
+        for (int u = 0; u < U; ++u) {
+            const int b = b0 + 32 * u;
+            if (b < nb) acc = w[u].term(in.lo[b], in.hi[b], in.x[b], acc);
         }
     }
-    if (key != nullptr) {
 #pragma unroll
-        for (int s = 1; s < R; s <<= 1) {
-            const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, s);
-            best = o > best ? o : best;
-        }
-        if (lane == 0 && best != 0ull) atomicMax(key, best);
-    }
+    for (int s = 16; s >= 1; s >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, s));
+    if (lane == 0) y[row] = acc;
 }
 
-// ggml Q8_0 [rows][nb] blocks of 34 bytes -> the row layout of dense_gemv_q8_0_kernel: [rows][stride][32 B] quants, then
+// ggml Q8_0 [rows][nb] blocks of 34 bytes -> the row layout of dense_product_kernel: [rows][stride][32 B] quants, then
 // [rows][stride] f16 scales. One thread per block.
 __global__ void repack_q8_0_dense_kernel(const uint8_t *src, uint8_t *dst, long long nblocks, int nb) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -295,101 +343,6 @@ __global__ void repack_q8_0_dense_kernel(const uint8_t *src, uint8_t *dst, long 
     uint16_t *d = reinterpret_cast<uint16_t *>(dst + nblocks / nb * stride * 32) + o;
     *d = static_cast<uint16_t>(s[0] | (s[1] << 8));
     for (int j = 0; j < 32; ++j) q[j] = s[2 + j];
-}
-
-// y = W x for a Q8_0 matrix (what every 2-D tensor of a model file that is not Q4_0 becomes: planarize_q4,
-// src/warodecode.cu:1027-1075), same structure and float order as dense_gemv_q4_0_kernel: lane l takes blocks l, l + 32,
-// ..., one fmaf(d_w * d_x, (float)int_dot, acc) per block with the exact integer dot of its 32 values, then the
-// butterfly. A block is two 16-byte loads.
-template <int R, int U>
-__global__ void __launch_bounds__(kDecThreads, 4) dense_gemv_q8_0_kernel(const uint8_t *wp, int rows, int nb, const int8_t *xq,
-                                                                       const float *xd, float *y, unsigned long long *key) {
-    extern __shared__ __align__(16) uint8_t dsm[];
-    grid_dep_launch();
-    uint4 *sq = reinterpret_cast<uint4 *>(dsm);
-    float *sd = reinterpret_cast<float *>(dsm + static_cast<size_t>(nb) * 32);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const uint4 *q_all = reinterpret_cast<const uint4 *>(wp);
-    const int stride = dense_row_stride(nb);
-    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * stride * 32);
-    uint4 wl[R][U], wh[R][U];
-    uint16_t dw[R][U];
-    auto load = [&](int row0, int b0) {
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int b = b0 + 32 * u;
-                if (b < nb && row0 + r < rows) {
-                    const size_t blk = static_cast<size_t>(row0 + r) * stride + b;
-                    wl[r][u] = __ldg(q_all + 2 * blk);
-                    wh[r][u] = __ldg(q_all + 2 * blk + 1);
-                    dw[r][u] = __ldg(d_all + blk);
-                }
-            }
-    };
-    const int row_first = (blockIdx.x * nwarps + warp) * R;
-    if (row_first < rows) load(row_first, lane);     // weights do not depend on the kernel before this one
-    grid_dep_wait();
-    for (int i = threadIdx.x; i < nb * 2; i += blockDim.x) sq[i] = reinterpret_cast<const uint4 *>(xq)[i];
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) sd[i] = xd[i];
-    __syncthreads();
-    unsigned long long best = 0ull;
-    for (int row0 = row_first; row0 < rows; row0 += gridDim.x * nwarps * R) {
-        float acc[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[r] = 0.0f;
-#pragma unroll 1
-        for (int b0 = lane; b0 < nb; b0 += 32 * U) {
-            if (row0 != row_first || b0 != lane) load(row0, b0);
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int b = b0 + 32 * u;
-                if (b < nb) {
-                    const uint4 lo = sq[2 * b], hi = sq[2 * b + 1];
-                    const float dx = sd[b];
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        if (row0 + r < rows) {
-                            int s = dp4a_s8(static_cast<int>(wl[r][u].x), static_cast<int>(lo.x), 0);
-                            s = dp4a_s8(static_cast<int>(wl[r][u].y), static_cast<int>(lo.y), s);
-                            s = dp4a_s8(static_cast<int>(wl[r][u].z), static_cast<int>(lo.z), s);
-                            s = dp4a_s8(static_cast<int>(wl[r][u].w), static_cast<int>(lo.w), s);
-                            s = dp4a_s8(static_cast<int>(wh[r][u].x), static_cast<int>(hi.x), s);
-                            s = dp4a_s8(static_cast<int>(wh[r][u].y), static_cast<int>(hi.y), s);
-                            s = dp4a_s8(static_cast<int>(wh[r][u].z), static_cast<int>(hi.z), s);
-                            s = dp4a_s8(static_cast<int>(wh[r][u].w), static_cast<int>(hi.w), s);
-                            acc[r] = __fmaf_rn(__fmul_rn(half_bits_to_float(dw[r][u]), dx), static_cast<float>(s), acc[r]);
-                        }
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-#pragma unroll
-            for (int s = 16; s >= 1; s >>= 1) acc[r] = __fadd_rn(acc[r], __shfl_xor_sync(0xffffffffu, acc[r], s));
-        }
-        if (lane < R && row0 + lane < rows) {
-            float v = acc[0];
-#pragma unroll
-            for (int r = 1; r < R; ++r) v = lane == r ? acc[r] : v;
-            y[row0 + lane] = v;
-            if (key != nullptr && v == v && fabsf(v) != INFINITY) {
-                const unsigned long long k =
-                    (static_cast<unsigned long long>(order_key(v)) << 32) | (0xffffffffu - static_cast<unsigned>(row0 + lane));
-                best = k > best ? k : best;
-            }
-        }
-    }
-    if (key != nullptr) {
-#pragma unroll
-        for (int s = 1; s < R; s <<= 1) {
-            const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, s);
-            best = o > best ? o : best;
-        }
-        if (lane == 0 && best != 0ull) atomicMax(key, best);
-    }
 }
 
 // The attention of one query head over cache positions 0..pos by one CTA of `nthreads` threads. qs: the rotated q head,
@@ -737,14 +690,111 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
     }
 }
 
-// act = SiLU(g) * u for gate_up = [gate rows | up rows], -> Q8_0; one warp per block of 32 (swiglu_kernel, :1956).
-__global__ void dense_swiglu_quant_kernel(const float *gate_up, int n, int8_t *xq, float *xd) {
+// y = W RMSNorm(hidden + proj) in one kernel: every CTA forms the norm and its Q8_0 form for itself (in shared memory), the
+// first one also stores the sum. The norm is a chain of a load, two reductions and two divisions that one CTA of a kernel of
+// its own took 3.2 us for, launch and hand-over included, while the other SMs waited; here it runs next to the weights that are
+// already on their way (2.2 us from the end of the kernel in front to the first product). CTAs of 512 threads, two per SM, so
+// that an SM reads hidden and proj twice and not four times.
+// Measured, 16 layers of 2048 / 8192 and a 128256-row head, 72 positions: 376 us per token with separate norm, product and
+// SwiGLU kernels, 386 with this kernel, 312 with the later weights asked into L2 (L2Ahead) and the cheaper block term.
+// MODE 0: y[row]; 1: rows are [ffn gate rows | ffn up rows], and a CTA takes 32 of both at once: SiLU(g) * u is quantised to
+// Q8_0 where it is formed (swiglu_kernel, :1956), without a kernel and a pass over memory of its own; 2: y[row] and the
+// arg-max of the finite results (one atomicMax per warp): key = order_key(value) << 32 | ~row, so the largest value wins and
+// ties go to the lowest row (dense_argmax_reduce_kernel, :1603-1632). Rows: R per warp, U blocks per lane and row in flight. Dynamic shared memory:
+// nb * 40 bytes.
+constexpr int kNormProductThreads = 512;
+template <bool Q8, int R, int U, int MODE, int PASSES>
+__global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_kernel(NormInput in, const uint8_t *wp, int rows, float *y,
+                                                                                   unsigned long long *key, int8_t *oq, float *od, L2Ahead ahead) {
+    static_assert(MODE != 1 || R == 4, "two gate rows and two up rows per warp");
+    constexpr int kWarpsHere = kNormProductThreads / 32;
+    extern __shared__ __align__(16) uint8_t dsm[];
+    __shared__ float outs[64];
     grid_dep_launch();
-    grid_dep_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;     // n is a multiple of 32: whole warps leave together
-    const float v = __fmul_rn(silu_ggml(gate_up[i]), gate_up[n + i]);
-    q8_0_block_warp(v, threadIdx.x & 31, xq + (i & ~31), xd + (i >> 5));
+    if (blockIdx.x != 0) in.hidden_out = nullptr;
+    const int nb = in.n >> 5, stride = dense_row_stride(nb), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const BlockInput x(dsm, nb);
+    const uint4 *q_all = reinterpret_cast<const uint4 *>(wp);
+    const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * stride * (Q8 ? 32 : 16));
+    auto row_of = [&](int unit, int r) {
+        if constexpr (MODE == 1) return (r >> 1) * (rows >> 1) + unit * 32 + warp * 2 + (r & 1);
+        return (unit * kWarpsHere + warp) * R + r;
+    };
+    const int units = MODE == 1 ? rows >> 6 : (rows + kWarpsHere * R - 1) / (kWarpsHere * R);
+    RowBlock<Q8> w[R][U];
+    auto load = [&](int unit, int b0) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int b = b0 + 32 * u, row = row_of(unit, r);
+                if (b < nb && (MODE == 1 || row < rows)) w[r][u].load(q_all, d_all, static_cast<size_t>(row) * stride + b);
+            }
+    };
+    int unit = blockIdx.x;
+    load(unit, lane);           // weights do not depend on the kernel before this one
+    ahead.request();
+    dense_norm_quant_body<PASSES>(in, [] { grid_dep_wait(); }, [&](int e, uint32_t packed, float d) {
+        const int b = e >> 5, j = e & 31;
+        *reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>((j & 16) ? x.hi + b : x.lo + b) + (j & 15)) = packed;
+        int sum = dp4a_s8(static_cast<int>(packed), 0x01010101, 0);
+#pragma unroll
+        for (int s = 1; s < 8; s <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+        if (j == 0) x.x[b] = make_int2(__float_as_int(d), -8 * sum);
+    });
+    __syncthreads();
+    unsigned long long best = 0ull;
+    for (; unit < units; unit += gridDim.x) {
+        float acc[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+#pragma unroll 1
+        for (int b0 = lane; b0 < nb; b0 += 32 * U) {
+            if (unit != static_cast<int>(blockIdx.x) || b0 != lane) load(unit, b0);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int b = b0 + 32 * u;
+                if (b < nb) {
+                    const uint4 lo = x.lo[b], hi = x.hi[b];
+                    const int2 d = x.x[b];
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+                        if (MODE == 1 || row_of(unit, r) < rows) acc[r] = w[r][u].term(lo, hi, d, acc[r]);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+            for (int s = 16; s >= 1; s >>= 1) acc[r] = __fadd_rn(acc[r], __shfl_xor_sync(0xffffffffu, acc[r], s));
+        }
+        float v = acc[0];
+#pragma unroll
+        for (int r = 1; r < R; ++r) v = lane == r ? acc[r] : v;
+        if constexpr (MODE == 1) {
+            if (lane < R) outs[(lane >> 1) * 32 + warp * 2 + (lane & 1)] = v;
+            __syncthreads();
+            if (warp == 0) q8_0_block_warp(__fmul_rn(silu_ggml(outs[lane]), outs[32 + lane]), lane, oq + unit * 32, od + unit);
+            __syncthreads();
+        } else {
+            const int row = row_of(unit, lane);
+            if (lane < R && row < rows) {
+                y[row] = v;
+                if (MODE == 2 && v == v && fabsf(v) != INFINITY) {
+                    const unsigned long long k = (static_cast<unsigned long long>(order_key(v)) << 32) | (0xffffffffu - static_cast<unsigned>(row));
+                    best = k > best ? k : best;
+                }
+            }
+        }
+    }
+    if constexpr (MODE == 2) {
+#pragma unroll
+        for (int s = 1; s < R; s <<= 1) {
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, s);
+            best = o > best ? o : best;
+        }
+        if (lane == 0 && best != 0ull) atomicMax(key, best);
+    }
 }
 
 // End of a step: the arg-max key becomes the next token (0 when no logit was finite), is recorded at out[pos + 1],

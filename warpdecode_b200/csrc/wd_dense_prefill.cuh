@@ -18,8 +18,15 @@ __global__ void __launch_bounds__(1024) prefill_norm_quant_kernel(float *hidden,
                                                                  int embd_q8) {
     grid_dep_launch();
     const size_t m = blockIdx.x;
-    dense_norm_quant_body(hidden + m * n, proj != nullptr ? proj + m * n : nullptr, w, n, eps, xq + m * n, xd + m * (n >> 5), embd,
-                          tokens + m, vocab, embd_q8 != 0, [] { grid_dep_wait(); });
+    float *h = hidden + m * n;
+    const NormInput in = {h, proj != nullptr ? proj + m * n : nullptr, w, embd != nullptr || proj != nullptr ? h : nullptr, embd, tokens + m, eps,
+                          n, vocab, embd_q8};
+    xq += m * n;
+    xd += m * (n >> 5);
+    dense_norm_quant_body<1>(in, [] { grid_dep_wait(); }, [&](int e, uint32_t packed, float d) {
+        store_quant4(xq, e, packed);
+        if ((e & 31) == 0) xd[e >> 5] = d;
+    });
 }
 
 // ---- Y[m][row] = W[row] . X[m] for the tokens of a chunk ---------------------------------------------------------------

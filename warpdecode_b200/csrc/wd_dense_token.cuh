@@ -49,7 +49,7 @@ struct DenseTokenParams {
 };
 
 // One row against the Q8_0 activation in shared memory; the row sits in shared memory as [nb * 16 B][nb * 2 B].
-// The order is dense_gemv_q4_0_kernel's: lane l takes blocks l, l + 32, ... ascending, then the butterfly.
+// The order is dense_product_kernel's: lane l takes blocks l, l + 32, ... ascending, then the butterfly.
 __device__ __forceinline__ float dense_row_smem(const uint8_t *row, int nb, const uint4 *sq, const float *sd, int lane) {
     const uint4 *q = reinterpret_cast<const uint4 *>(row);
     const uint16_t *d = reinterpret_cast<const uint16_t *>(row + static_cast<size_t>(nb) * 16);
