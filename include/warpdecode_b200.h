@@ -231,8 +231,8 @@ int wd_dense_decoder_tensor_type(wd_dense_decoder *d, int layer, int which);
 int wd_dense_decoder_get_tensor(wd_dense_decoder *d, int layer, int which, void *host_out, size_t bytes);
 /* Every 2-D tensor drawn N(0, sigma) and quantised to Q4_0 on the device, norms 1 (synthetic models for measurements). */
 int wd_dense_decoder_synth(wd_dense_decoder *d, unsigned long long seed, float sigma);
-/* Greedy decode from position 0: the prompt is fed token by token, then n_gen tokens are generated (Runtime::run,
- * src/warodecode.cu:2120-2150). out_tokens [n_prompt + n_gen] receives the prompt followed by the generated tokens;
+/* Greedy decode from position 0: the prompt in passes of up to 512 positions over the weights, with the results of feeding it token
+ * by token, then n_gen tokens are generated (Runtime::run, src/warodecode.cu:2120-2150). out_tokens [n_prompt + n_gen] receives the prompt followed by the generated tokens;
  * ms_total (optional) the device time of the n_prompt + n_gen - 1 steps. */
 int wd_dense_decoder_decode(wd_dense_decoder *d, const int *prompt, int n_prompt, int n_gen, int *out_tokens, float *ms_total);
 /* Profiling of the token kernel: when WD_DENSE_STAMPS was set at creation, the SM clock counter of one CTA at the twelve
