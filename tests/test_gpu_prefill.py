@@ -81,3 +81,21 @@ def test_norm_and_product_in_one_kernel(wd, oracle, H, hd, F, V, q8):
     assert np.array_equal(ol.fbits(logits), ol.fbits(ref.logits))
     assert np.array_equal(ol.fbits(hidden), ol.fbits(ref.hidden))
     dec.close()
+
+
+@pytest.mark.parametrize("nh,nkv,hd,P,style", [(4, 2, 64, 322, "q4"),           # one position and one chunk beyond the single ring
+                                               (4, 2, 64, 640, "file"), (2, 1, 64, 1090, "q4"),         # values refilled behind the scores
+                                               (3, 1, 96, 500, "q4"), (3, 1, 96, 1350, "q4"), (2, 1, 128, 1400, "q4")])
+def test_attention_over_a_cluster(wd, oracle, nh, nkv, hd, P, style):
+    test_prompt_pass_equals_the_one_token_steps(wd, oracle, 256, nh, nkv, hd, 320, 1, P, 3, style)
+
+
+def test_attention_of_a_long_decoder_at_its_first_positions(wd, oracle):
+    """The cluster form is chosen by the longest context; the first positions leave some of its CTAs without keys."""
+    cfg = dict(hidden=256, n_heads=2, n_kv_heads=1, head_dim=128, ffn=64, vocab=500, n_layers=1, max_ctx=2000, rms_eps=1e-5)
+    dec = wd.DenseDecoder(256, 2, 1, 128, 64, 500, 1, 2000, 1e-5, 500000.0)
+    dec.synth(5, 0.05)
+    got, _ = dec.decode(np.arange(2), 130)
+    ref = _oracle_for(wd, oracle, dec, cfg, 500000.0)
+    assert np.array_equal(got, ref.decode(np.arange(2), 130))
+    dec.close()

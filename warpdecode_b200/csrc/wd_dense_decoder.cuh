@@ -461,17 +461,33 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Geometry of the decode attention for a head dimension: chunks of 64 cache rows (keys or values) in padded rows, so that
-// neighbouring positions start in different banks.
-template <int HD>
+// Cluster of CTAs that share one head: a barrier in two halves, and a store into a peer's shared memory.
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void store_peer(float *p, uint32_t rank, float v) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+
+// Geometry of the decode attention for a head dimension and C CTAs per head: chunks of 64 key rows, and of 64 C value rows of
+// HD / C elements, in padded rows, so that neighbouring positions start in different banks.
+template <int HD, int C>
 struct DecodeAttn {
-    static constexpr int kThreads = 512, kChunk = 64, kRow = HD + 4;
-    static constexpr int kSlotBytes = kChunk * kRow * 4;
+    static constexpr int kThreads = 512, kChunk = 64, kRow = HD + 4, kSlice = HD / C, kChunkV = kChunk * C, kRowV = kSlice + 4;
+    static constexpr int kSlot = kChunk * kRow > kChunkV * kRowV ? kChunk * kRow : kChunkV * kRowV;      // floats
+    static constexpr int kSlotBytes = kSlot * 4;
     static constexpr int kRoom = 190 * 1024;                    // slots and scores together; the rest of an SM is for the product before it
+    static int want(int max_ctx) { return ((max_ctx + kChunk - 1) / kChunk + C - 1) / C + (max_ctx + kChunkV - 1) / kChunkV; }
     // slots of the ring: both caches of the longest context, or what fits beside its scores
     static int slots(int max_ctx) {
-        const int want = 2 * ((max_ctx + kChunk - 1) / kChunk), fit = (kRoom - max_ctx * 4) / kSlotBytes;
-        return want < fit ? want : fit;
+        const int fit = (kRoom - max_ctx * 4) / kSlotBytes, w = want(max_ctx);
+        return w < fit ? w : fit;
     }
 };
 
@@ -486,39 +502,55 @@ struct DecodeAttn {
 // keys and values must be there when they are needed: the cache below pos was written by earlier tokens, and the first
 // chunks of it (all of it up to 320 positions of 64) are copied to shared memory in a ring, keys before values,
 // requested BEFORE the wait for the QKV product; a score is one thread's work, without shuffles.
-// Measured per layer inside the step of the 16-layer model (32 heads of 64), start -> now: 2.1 us at 72 positions (6.6 us
-// before), and at 512 positions 74 us before.
+// Measured per layer inside the step of the 16-layer model (32 heads of 64), before -> now: 6.6 -> 2.1 us at 72 positions; at 500
+// positions 74 -> 7.7 us (8.6 us by one CTA per head).
+//
+// C: CTAs per head, a cluster. One CTA takes in 512 bytes per position through its SM, and once a context is longer than its
+// ring holds, the last values only follow when the first keys have been scored. With C = HD / 32 each CTA scores every C-th
+// chunk of keys, stores the scores into its peers' shared memory too, and sums 32 elements of the values (one Q8_0 block) over
+// all positions: the orders stay, an SM takes in 1 / C of the bytes. For decoders whose longest context does not fit one ring.
 //
 // EXTRAS: the layer has q/k/v biases (Qwen2-style files: added to the QKV product's rows) and / or RMSNorm weights for
 // the q and k heads (Qwen3-style: qk_norm_kernel, src/warodecode.cu:1836), applied in that order before the rotary
 // embedding (emit_step :2069-2075). Layers without them run the instantiation that has none of that code.
 // Dynamic shared memory: `slots` chunks, then max_ctx scores.
-template <int HD, bool EXTRAS>
-__global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kernel(const float *qkv, const float *table, float *kcache,
+template <int HD, bool EXTRAS, int C>
+__global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_kernel(const float *qkv, const float *table, float *kcache,
                                                                                  float *vcache, const int *pos_ptr, int heads,
                                                                                  int kv_heads, int slots, float inv_sqrt, int8_t *oq,
                                                                                  float *od, const float *bqkv, const float *q_norm,
                                                                                  const float *k_norm, float eps) {
-    using A = DecodeAttn<HD>;
+    using A = DecodeAttn<HD, C>;
     constexpr int kNt = A::kThreads, kChunk = A::kChunk, kRow = A::kRow, kHalf = HD / 2, kRow16 = HD / 4;
+    constexpr int kSlice = A::kSlice, kChunkV = A::kChunkV, kRowV = A::kRowV, kSlice16 = kSlice / 4;
     extern __shared__ __align__(16) float vring[];
     __shared__ __align__(16) float qs[HD], kn[HD];
-    __shared__ float vn[HD], outv[HD], wmax[kNt / 32];
-    float *sc = vring + static_cast<size_t>(slots) * kChunk * kRow;
+    __shared__ float vn[HD], outv[kSlice], wmax[kNt / 32];
+    float *sc = vring + static_cast<size_t>(slots) * A::kSlot;
     grid_dep_launch();
-    const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if constexpr (C > 1) cluster_arrive();          // answered before the first store into a peer
+    const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0;
+    const int h = blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int pos = *pos_ptr, kv_dim = kv_heads * HD, kvh = (h * kv_heads) / heads;
     float *kc = kcache + static_cast<size_t>(kvh) * HD, *vc = vcache + static_cast<size_t>(kvh) * HD;
-    const int n_chunks = (pos + kChunk - 1) / kChunk, n_items = 2 * n_chunks;      // positions 0 .. pos - 1: key chunks, then value chunks
-    auto slot_of = [&](int item) { return vring + static_cast<size_t>(item % slots) * kChunk * kRow; };
+    // positions 0 .. pos - 1: this CTA's key chunks (every C-th), then all value chunks of its slice
+    const int n_chunks = ((pos + kChunk - 1) / kChunk - rank + C - 1) / C, n_vchunks = (pos + kChunkV - 1) / kChunkV, n_items = n_chunks + n_vchunks;
+    auto slot_of = [&](int item) { return vring + static_cast<size_t>(item % slots) * A::kSlot; };
     auto request = [&](int item) {
         if (item >= n_items) return;
-        const int c = item < n_chunks ? item : item - n_chunks;
-        const float *src = item < n_chunks ? kc : vc;
         float *dst = slot_of(item);
-        for (int i = tid; i < kChunk * kRow16; i += kNt) {
-            const int r = i / kRow16, e = i - r * kRow16, t = c * kChunk + r;
-            if (t < pos) cp_async16(dst + r * kRow + e * 4, src + static_cast<size_t>(t) * kv_dim + e * 4, true);
+        if (item < n_chunks) {
+            const int t0 = (item * C + rank) * kChunk;
+            for (int i = tid; i < kChunk * kRow16; i += kNt) {
+                const int r = i / kRow16, e = i - r * kRow16;
+                if (t0 + r < pos) cp_async16(dst + r * kRow + e * 4, kc + static_cast<size_t>(t0 + r) * kv_dim + e * 4, true);
+            }
+        } else {
+            const int t0 = (item - n_chunks) * kChunkV;
+            for (int i = tid; i < kChunkV * kSlice16; i += kNt) {
+                const int r = i / kSlice16, e = i - r * kSlice16;
+                if (t0 + r < pos) cp_async16(dst + r * kRowV + e * 4, vc + static_cast<size_t>(t0 + r) * kv_dim + rank * kSlice + e * 4, true);
+            }
         }
     };
     for (int i = 0; i < min(slots, n_chunks); ++i) request(i);
@@ -583,7 +615,7 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
         k_raw = kn_in;
         v_raw = vn_in;
     }
-    const bool writer = h % (heads / kv_heads) == 0;        // the first head of its KV group
+    const bool writer = h % (heads / kv_heads) == 0 && rank == 0;       // the first head of its KV group
     if (tid < kHalf) {
         const float a = q_raw[tid], b = q_raw[tid + kHalf], c = k_raw[tid], d = k_raw[tid + kHalf];
         const float v0 = v_raw[tid], v1 = v_raw[tid + kHalf];
@@ -603,6 +635,7 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
         }
     }
     __syncthreads();
+    if constexpr (C > 1) cluster_wait();        // the peers run
     float m = -INFINITY;
     const int batch = min(kNt / kChunk, slots);         // key chunks scored side by side, one position per thread
 #pragma unroll 1
@@ -610,13 +643,17 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
         if (c0 == 0) cp_async_wait<1>();
         else cp_async_wait<0>();
         __syncthreads();
-        const int c = c0 + tid / kChunk, t = c * kChunk + (tid & (kChunk - 1));
+        const int c = c0 + tid / kChunk, t = (c * C + rank) * kChunk + (tid & (kChunk - 1));
         const bool newest = c0 == 0 && tid == kNt - 1;
         if ((tid < batch * kChunk && c < n_chunks && t < pos) || newest) {
             // the last thread scores the new position, and an old one too when it has one
             if (!newest || (tid < batch * kChunk && t < pos)) {
                 const float v = __fmul_rn(lane_order_dot<HD>(qs, slot_of(c) + (tid & (kChunk - 1)) * kRow), inv_sqrt);
                 sc[t] = v;
+                if constexpr (C > 1) {
+#pragma unroll
+                    for (int r = 1; r < C; ++r) store_peer(sc + t, rank + r < C ? rank + r : rank + r - C, v);
+                }
                 m = v > m ? v : m;          // a NaN score never becomes the maximum
             }
             if (newest) {
@@ -631,6 +668,11 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
             cp_async_commit();
         }
     }
+    if constexpr (C > 1) {          // all scores are here; nothing is stored into a peer after this
+        cluster_arrive();
+        cluster_wait();
+        for (int t = tid; t <= pos; t += kNt) m = sc[t] > m ? sc[t] : m;
+    }
 #pragma unroll
     for (int s = 16; s >= 1; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
     if (lane == 0) wmax[warp] = m;
@@ -643,10 +685,10 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
     __syncthreads();
     float l = 0.0f, acc = 0.0f;
 #pragma unroll 1
-    for (int c = 0; c < n_chunks; ++c) {
-        if (tid < HD) {
-            const float *v = slot_of(n_chunks + c) + tid, *p = sc + c * kChunk;
-            const int n = min(kChunk, pos - c * kChunk);
+    for (int c = 0; c < n_vchunks; ++c) {
+        if (tid < kSlice) {
+            const float *v = slot_of(n_chunks + c) + tid, *p = sc + c * kChunkV;
+            const int n = min(kChunkV, pos - c * kChunkV);
             // the two chains advance four cycles a step; a whole chunk's weights and values are requested well ahead of them
             int r = 0;
             for (; r + 32 <= n; r += 32) {
@@ -655,7 +697,7 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
 #pragma unroll
                 for (int i = 0; i < 8; ++i) p4[i] = *reinterpret_cast<const float4 *>(p + r + 4 * i);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) x[i] = v[(r + i) * kRow];
+                for (int i = 0; i < 32; ++i) x[i] = v[(r + i) * kRowV];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     l = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(l, p4[i].x), p4[i].y), p4[i].z), p4[i].w);
@@ -667,10 +709,10 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
             }
             for (; r < n; ++r) {
                 l = __fadd_rn(l, p[r]);
-                acc = __fmaf_rn(p[r], v[r * kRow], acc);
+                acc = __fmaf_rn(p[r], v[r * kRowV], acc);
             }
         }
-        if (n_chunks > slots) {     // longer than the ring: refill the slot; when a refilled chunk is read, more than three requests are younger
+        if (n_vchunks > slots) {     // longer than the ring: refill the slot; when a refilled chunk is read, more than three requests are younger
             __syncthreads();
             request(n_chunks + c + slots);
             cp_async_commit();
@@ -678,14 +720,14 @@ __global__ void __launch_bounds__(DecodeAttn<HD>::kThreads) dense_attention_kern
             __syncthreads();
         }
     }
-    if (tid < HD) {
+    if (tid < kSlice) {
         l = __fadd_rn(l, sc[pos]);
-        acc = __fmaf_rn(sc[pos], vn[tid], acc);
+        acc = __fmaf_rn(sc[pos], vn[rank * kSlice + tid], acc);
         outv[tid] = __fdiv_rn(acc, l);
     }
     __syncthreads();
-    if (warp < HD / 32) {
-        const int b = (h * HD) / 32 + warp;
+    if (warp < kSlice / 32) {
+        const int b = (h * HD + rank * kSlice) / 32 + warp;
         q8_0_block_warp(outv[warp * 32 + lane], lane, oq + static_cast<size_t>(b) * 32, od + b);
     }
 }
