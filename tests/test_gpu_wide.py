@@ -97,3 +97,24 @@ def test_a_batch_whose_early_picks_do_not_stand_is_decoded_again(oracle, bad):
             assert np.array_equal(bits(out[t]), bits(want[t]["out"])), t
     assert eng.fallbacks() == 3 * len(bad) and eng.device_status() == 0
     eng.close()
+
+
+@pytest.mark.parametrize("E,K,scale", [(8, 3, 1.0), (64, 10, 1000.0), (600, 10, 300.0), (16, 16, 30.0)])
+def test_plain_layout_picks_from_a_threshold_or_the_rungs(oracle, E, K, scale):
+    """Ordinary rows, and activations that push most probabilities to zero, where the k largest logits are not the k rungs."""
+    import warpdecode_b200 as wd
+    H, F, SF = 768, 64, 128
+    m = synth.make_moe_block(E + K, H, F, E, K, SF, 21, 20)
+    x = np.random.Generator(np.random.PCG64(E)).standard_normal((3, H)).astype(np.float32)
+    x[1:] *= np.float32(scale)
+    eng = wd.Engine(H, F, E, K, SF, 1, expert_type=21, down_type=20, max_tokens=3)
+    eng.load_block(0, m)
+    assert eng.kernel_name() == "plain_gate_up_kernel"
+    out = eng.forward_host(0, x)
+    for t in range(3):
+        want = oracle.moe_block(m, x[t])
+        assert np.array_equal(eng.tap("ids", t), want["ids"])
+        assert np.array_equal(bits(eng.tap("weights", t)), bits(want["weights"]))
+        assert np.array_equal(bits(out[t]), bits(want["out"])), t
+    assert eng.device_status() == 0
+    eng.close()
