@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
 // SwiGLU kernels, 386 with this kernel, 312 with the later weights asked into L2 (L2Ahead) and the cheaper block term.
 // MODE 0: y[row]; 1: rows are [ffn gate rows | ffn up rows], and a CTA takes 32 of both at once: SiLU(g) * u is quantised to
 // Q8_0 where it is formed (swiglu_kernel, :1956), without a kernel and a pass over memory of its own; 2: y[row] and the
-// arg-max of the finite results (one atomicMax per warp): key = order_key(value) << 32 | ~row, so the largest value wins and
+// arg-max of the finite results: key = order_key(value) << 32 | ~row, so the largest value wins and
 // ties go to the lowest row (dense_argmax_reduce_kernel, :1603-1632). Rows: R per warp, U blocks per lane and row in flight. Dynamic shared memory:
 // nb * 40 bytes.
 constexpr int kNormProductThreads = 512;
@@ -829,13 +829,24 @@ __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_ker
             }
         }
     }
-    if constexpr (MODE == 2) {
+    if constexpr (MODE == 2) {      // one atomic per CTA
+        __shared__ unsigned long long bests[kWarpsHere];
 #pragma unroll
         for (int s = 1; s < R; s <<= 1) {
             const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, s);
             best = o > best ? o : best;
         }
-        if (lane == 0 && best != 0ull) atomicMax(key, best);
+        if (lane == 0) bests[warp] = best;
+        __syncthreads();
+        if (warp == 0) {
+            best = bests[lane & (kWarpsHere - 1)];
+#pragma unroll
+            for (int s = 1; s < kWarpsHere; s <<= 1) {
+                const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, s);
+                best = o > best ? o : best;
+            }
+            if (lane == 0 && best != 0ull) atomicMax(key, best);
+        }
     }
 }
 
