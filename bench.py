@@ -47,7 +47,7 @@ LAYER_BYTES = 10 * EXPERT_BYTES + REPLICATED_BYTES
 HEAD_BYTES = VOCAB * (CFG["hidden"] // 32) * 34
 # dram__bytes_read + dram__bytes_write of the layer kernel per layer, from an ncu capture of a two-layer
 # launch of the same shape; every layer reads its own weights once, so a launch of n layers moves n times this.
-TRAFFIC_PER_LAYER = 18_137_000
+TRAFFIC_PER_LAYER = 21_045_000
 METRIC = "batch-1 decode tok/s (48L 512-expert IQ3_S MoE)"
 WORKLOAD = ("cfg2/cfg3 MoE stack: 48 layers x (router top-10 of 512 IQ3_S experts + Q8_0 shared expert), "
             "hidden 2048, all experts resident, router bias N(0,1) at every N; per token x=RMSNorm(residual), "
