@@ -100,7 +100,6 @@ __device__ __forceinline__ void q8_0_block_warp(float v, int lane, Quant *q_out,
 }
 
 // Four quants of one thread (values e .. e + 3, e a multiple of four) with one store.
-__device__ __forceinline__ void store_quant4(int8_t *out, int e, uint32_t packed) { *reinterpret_cast<uint32_t *>(out + e) = packed; }
 __device__ __forceinline__ void store_quant4(PairedQuant *out, int e, uint32_t packed) {
     *reinterpret_cast<uint32_t *>(out + (e & ~31) + paired_place(e & 31)) = packed;
 }
