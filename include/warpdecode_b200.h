@@ -269,6 +269,11 @@ int wd_quantize_q8_K_host(const float *x, int n, void *blocks);
  * engine uses. `partials`, if not NULL, receives the int32 sums [rows][cols/256][8] (IQ types). */
 int wd_matvec_host(int type, const void *w, int rows, int cols, const float *x, float *y,
                    int32_t *partials);
+/* The tile tasks of CTA `cta` of `n_cta` in a batch call of n_tokens (<= max_tokens <= 4) on the batch kernel, in the order its sixteen
+ * warps walk them (warp w: tasks w, w + 16, ...): desc and aux as the kernel works them out (csrc/wd_moe_batch.cuh, batch_task).
+ * wide: the last n_tokens CTAs pick and take no tiles. Returns the number of tasks (at most `cap` are written). Host only. */
+int wd_batch_tasks(int hidden, int expert_ffn, int top_k, int n_tokens, int max_tokens, int wide, int n_cta, int cta,
+                   uint32_t *desc, int *aux, int cap);
 /* ---- model load from GGUF ------------------------------------------------------------------ */
 /* Read-only mapping of a GGUF file (v2/v3) with its metadata and tensor directory parsed: the part of
  * GgufFile (src/gguf.hpp) and load_qwen38_runtime (src/qwen38_runtime.cuh:117-265) that the MoE path

@@ -115,3 +115,26 @@ def test_batch_of_four_at_the_model_shape(wd, oracle, batch_kernel, monkeypatch)
         assert np.array_equal(eng.tap("ids", n - 1), ids[n - 1])
     assert eng.device_status() == 0
     eng.close()
+
+
+@pytest.mark.parametrize("H,F,E,K,typ", [(2048, 1024, 16, 8, 22), (1024, 1024, 32, 12, 21), (2048, 512, 32, 12, 21), (512, 1024, 16, 16, 22)])
+def test_more_gate_up_tiles_than_one_round_of_warps(oracle, H, F, E, K, typ):
+    """Runs of down tiles that need many activation superblocks while a CTA's warps still have gate/up tiles to do: the gathers
+    may not stand in front of the tiles they wait for (one token: its gate/up tiles directly precede its down tiles)."""
+    import warpdecode_b200 as wd
+    from warpdecode_b200 import synth
+    m = synth.make_moe_block(H + F + K, H, F, E, K, 128, typ, typ)
+    rng = np.random.Generator(np.random.PCG64(K))
+    m["gate"], m["up"] = (synth.random_blocks(rng, typ, E * F * H // 256) for _ in range(2))
+    m["down"] = synth.random_blocks(rng, typ, E * H * F // 256)
+    eng = wd.Engine(H, F, E, K, 128, 1, expert_type=typ, down_type=typ, max_tokens=4)
+    eng.load_block(0, m)
+    assert eng.batch_kernel_name() == "moe_batch_kernel"
+    x = rng.standard_normal((4, H)).astype(np.float32)
+    want = [oracle.moe_block(m, v)["out"] for v in x]
+    for T in (1, 2, 4, 1):
+        out = eng.forward_host(0, x[:T])
+        assert eng.device_status() == 0
+        for t in range(T):
+            assert np.array_equal(ol.fbits(out).reshape(T, H)[t], ol.fbits(want[t])), (T, t)
+    eng.close()

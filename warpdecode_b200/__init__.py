@@ -111,6 +111,7 @@ def lib():
         L.wd_batch_kernel_name.restype = C.c_char_p
         L.wd_last_kernel_name.argtypes = [vp]
         L.wd_last_kernel_name.restype = C.c_char_p
+        L.wd_batch_tasks.argtypes = [C.c_int] * 8 + [vp, vp, C.c_int]
         L.wd_measure_tile_decoder.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_double)]
         L.wd_dense_decoder_create.argtypes = [C.POINTER(DenseConfig), C.POINTER(C.c_void_p)]
         L.wd_dense_decoder_set_tensor_typed.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
@@ -558,6 +559,16 @@ def measure_tile_decoder(nsb=8, warps=16, unroll=1, device=0):
     c = C.c_double()
     _check(lib().wd_measure_tile_decoder(device, nsb, warps, unroll, C.byref(c)))
     return c.value
+
+
+def batch_tasks(hidden, expert_ffn, top_k, n_tokens, max_tokens, wide, n_cta, cta):
+    """Descriptions and aux words of one CTA's tile tasks in a batch call (host only)."""
+    cap = 4096
+    desc, aux = np.zeros(cap, np.uint32), np.zeros(cap, np.int32)
+    n = lib().wd_batch_tasks(hidden, expert_ffn, top_k, n_tokens, max_tokens, int(wide), n_cta, cta, _ptr(desc), _ptr(aux), cap)
+    if n < 0 or n > cap:
+        _check(n if n < 0 else -1)
+    return desc[:n], aux[:n]
 
 
 def embed_q8_0(table_dev_ptr, rows, cols, token_ptr, out_ptr, stream=None):

@@ -491,9 +491,7 @@ void plan_batch(wd_engine *e) {
         p.off_tasks = take(static_cast<size_t>(p.max_tasks) * 16);
     }
     p.off_pairbuf = take(static_cast<size_t>(32) * 2 * r_h * 4);
-    const int t3 = H / r_f;                                  // down tiles per pair
-    const int max3 = (K * t3 + wcta - 1) / wcta;             // longest run of one token's down tiles in one CTA
-    const int n_exp_tok = std::min(K, (max3 - 1) / t3 + 2);  // pairs such a run can touch
+    const int n_exp_tok = wd::batch_run_pairs(K, H / r_f, wcta);
     p.n_act = static_cast<unsigned>(wd::kMaxTokens * n_exp_tok * m.nsb_f);
     if (p.n_act > 62) return;
     p.off_actk = take(static_cast<size_t>(p.n_act) * wd::kActSbStride);
@@ -1745,6 +1743,25 @@ int wd_measure_tile_decoder(int device, int nsb, int warps, int unroll, double *
     std::sort(h.begin(), h.end());
     *cycles_per_round = static_cast<double>(h[h.size() / 2]) / iters;
     return WD_OK;
+}
+
+int wd_batch_tasks(int hidden, int expert_ffn, int top_k, int n_tokens, int max_tokens, int wide, int n_cta, int cta, uint32_t *desc, int *aux,
+                   int cap) {
+    if (!desc || !aux || !pow2(hidden) || !pow2(expert_ffn) || hidden < 256 || expert_ffn < 256 || hidden > 8192 || expert_ffn > 2048 || top_k < 1 ||
+        top_k > wd::kMaxK || n_tokens < 1 || n_tokens > max_tokens || max_tokens > wd::kMaxTokens || cta < 0 || cta >= n_cta || n_cta <= max_tokens)
+        return fail(WD_E_INVALID, "wd_batch_tasks: bad geometry");
+    const int nsb_h = hidden / 256, nsb_f = expert_ffn / 256, t2 = expert_ffn * nsb_h / 32, t3 = hidden * nsb_f / 32;
+    int t2_log2 = 0, t3_log2 = 0, ints[wd::BatchList::kInts] = {};
+    while ((1 << t2_log2) < t2) ++t2_log2;
+    while ((1 << t3_log2) < t3) ++t3_log2;
+    const int wcta = wide ? n_cta - n_tokens : n_cta;
+    const int act_per_tok = wd::batch_run_pairs(top_k, t3, wide ? n_cta - max_tokens : n_cta) * nsb_f;
+    const wd::BatchList list(ints);
+    wd::batch_lay_out(list, n_tokens, top_k, t2_log2, t3_log2, nsb_f, cta, wcta);
+    const int n = list.begin[2 * n_tokens];
+    for (int i = 0; i < std::min(n, cap); ++i)
+        desc[i] = wd::batch_task(list, i, n_tokens, top_k, t2_log2, t3_log2, nsb_f, act_per_tok, wcta, aux[i]);
+    return n;
 }
 
 const char *wd_kernel_name(const wd_engine *e) {

@@ -80,6 +80,93 @@ struct BatchParams {
     unsigned n1r, n1s, nsd, n_act;   // router tasks, shared gate/up tasks, shared-down tasks, activation superblocks per CTA (maxima)
 };
 
+// ---- the task list of a CTA (host and device: a CPU test walks the lists of a whole grid) ----
+// The tile tasks of a CTA form one list of segments: gate/up(token 0), gate/up(1), then for every token t gate/up(t + 2) (while
+// there is one) followed by down(t). The down tiles of a token thus come two segments after its gate/up tiles, when the
+// activations they need have long been published, and nobody waits for them. Per token the gate/up units go round the CTAs
+// (rotated by token, so that the odd units even out) and the down tiles are cut into one contiguous run per CTA (a run needs the
+// activations of one or two pairs only).
+struct BatchList {              // ints of the list in shared memory
+    static constexpr int kBegin = 0, kInfo = 9, kCta = 17, kVb = 21, kJl0 = 25, kNg = 29, kGuEnd = 33, kInts = 37;
+    int *begin, *info;          // [2T + 1] first task of every segment; [2T] token * 2 + (1: down tiles)
+    int *cta, *vb, *jl0, *ng;   // per token: the CTA's place in the rotation, first down tile, first pair and activation superblocks of the run
+    int *gu_end;                // per token: the end of its gate/up segment
+    __host__ __device__ explicit BatchList(int *m)
+        : begin(m + kBegin), info(m + kInfo), cta(m + kCta), vb(m + kVb), jl0(m + kJl0), ng(m + kNg), gu_end(m + kGuEnd) {}
+};
+// pairs that one CTA's run of a token's down tiles can touch (t3: down tiles per pair)
+__host__ __device__ inline int batch_run_pairs(int K, int t3, int wcta) {
+    const int longest = (K * t3 + wcta - 1) / wcta, n = (longest - 1) / t3 + 2;
+    return n < K ? n : K;
+}
+__host__ __device__ inline void batch_lay_out(const BatchList &L, int T, int K, int t2_log2, int t3_log2, int nsb_f, int cta, int wcta) {
+    const int u_tok = K << t2_log2, v_tok = K << t3_log2;       // gate/up units and down tiles of one token
+    int c2[kMaxTokens], c3[kMaxTokens];
+    for (int t = 0; t < T; ++t) {
+        int ct = cta + t * (wcta / kMaxTokens);
+        if (ct >= wcta) ct -= wcta;
+        L.cta[t] = ct;
+        c2[t] = cta < wcta && u_tok > ct ? (u_tok - ct + wcta - 1) / wcta : 0;
+        const int vb = static_cast<int>(static_cast<unsigned>(ct) * static_cast<unsigned>(v_tok) / static_cast<unsigned>(wcta));
+        const int ve = cta < wcta ? static_cast<int>(static_cast<unsigned>(ct + 1) * static_cast<unsigned>(v_tok) / static_cast<unsigned>(wcta)) : vb;
+        L.vb[t] = vb;
+        L.jl0[t] = vb >> t3_log2;
+        c3[t] = ve - vb;
+        L.ng[t] = ve > vb ? (((ve - 1) >> t3_log2) - (vb >> t3_log2) + 1) * nsb_f : 0;
+    }
+    int at = 0, k = 0;
+    auto add = [&](int t, int down) {
+        L.begin[k] = at;
+        L.info[k] = t * 2 + down;
+        at += down ? c3[t] : 2 * c2[t];
+        if (!down) L.gu_end[t] = at;
+        ++k;
+    };
+    add(0, 0);
+    if (T > 1) add(1, 0);
+    for (int t = 0; t < T; ++t) {
+        if (t + 2 < T) add(t + 2, 0);
+        add(t, 1);
+    }
+    L.begin[k] = at;
+}
+// Task i:
+//   desc: bit 0 down tile, 1-2 token, 3-8 pair, 9-20 tile inside the pair's matrix, 21 up tile (else gate),
+//         22-27 one more than the activation superblock this task's warp gathers afterwards (0: none)
+//   aux : gate/up tile: entry of the pair buffer; down tile: first activation superblock of its pair
+// The gathers of a down segment are handed to the tasks that end a round (kWarps tasks) before it starts, one each. A gather
+// waits for gate/up tiles of all CTAs, so the warp that does it may not have a gate/up tile of that token (or an earlier one) still in
+// front of it, or it waits for itself: its next task, i + kWarps, lies behind the token's gate/up segment. Gate/up tiles then wait for
+// earlier tokens only, and by induction over the tokens every wait ends. A gather nobody was handed is done by the first
+// tile that needs it.
+__host__ __device__ inline uint32_t batch_task(const BatchList &L, int i, int T, int K, int t2_log2, int t3_log2, int nsb_f, int act_per_tok, int wcta,
+                                               int &aux) {
+    int k = 0;
+    while (k + 1 < 2 * T && i >= L.begin[k + 1]) ++k;
+    const int t = L.info[k] >> 1, down = L.info[k] & 1, li = i - L.begin[k];
+    uint32_t d;
+    if (!down) {
+        const int u = L.cta[t] + (li >> 1) * wcta;
+        d = static_cast<uint32_t>(t << 1) | static_cast<uint32_t>((t * K + (u >> t2_log2)) << 3) |
+            static_cast<uint32_t>((u & ((1 << t2_log2) - 1)) << 9) | static_cast<uint32_t>((li & 1) << 21);
+        aux = ((i - (li & 1)) >> 1) & 31;
+    } else {
+        const int v = L.vb[t] + li, pl = v >> t3_log2;
+        d = 1u | static_cast<uint32_t>(t << 1) | static_cast<uint32_t>((t * K + pl) << 3) | static_cast<uint32_t>((v & ((1 << t3_log2) - 1)) << 9);
+        aux = t * act_per_tok + (pl - L.jl0[t]) * nsb_f;
+    }
+    for (int kd = 0; kd < 2 * T; ++kd) {
+        if (!(L.info[kd] & 1)) continue;
+        const int td = L.info[kd] >> 1;
+        int base = L.begin[kd] - kWarps - L.ng[td];
+        if (base < L.gu_end[td] - kWarps) base = L.gu_end[td] - kWarps;
+        if (base < 0) base = 0;
+        // at most one per task (short segments overlap)
+        if (i >= base && i < base + L.ng[td] && (d >> 22) == 0u) d |= static_cast<uint32_t>(td * act_per_tok + (i - base) + 1) << 22;
+    }
+    return d;
+}
+
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
@@ -157,45 +244,9 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
         for (int b = lane; b < static_cast<int>(P.n_act); b += 32) act_state[b] = 0;
     }
     if (cta == 0 && tid == 0) P.sync[5] = smem_u32(bars);
-    const int u_tok = P.K << P.t2_log2, v_tok = P.K << P.t3_log2;      // gate/up units and down tiles of one token
     const int n_exp_tok = static_cast<int>(P.n_act) / (kMaxTokens * P.nsb_f);     // pairs a run may touch (planned maximum)
-    // The tile tasks of a CTA form one list of segments: gate/up(token 0), gate/up(1), then for every token t
-    // gate/up(t + 2) (while there is one) followed by down(t). The down tiles of a token thus come two segments after
-    // its gate/up tiles, when the activations they need have long been published, and nobody waits for them.
-    // Per token the gate/up units go round the CTAs (rotated by token, so that the odd units even out) and the down
-    // tiles are cut into one contiguous run per CTA (a run needs the activations of one or two pairs only).
-    int *seg_begin = reinterpret_cast<int *>(sm + P.off_seg);          // [2T + 1] first task of every segment
-    int *seg_info = seg_begin + 9;                                     // [2T] token * 2 + (1: down tiles)
-    int *tok_cta = seg_begin + 17, *tok_vb = seg_begin + 21, *tok_jl0 = seg_begin + 25, *tok_ng = seg_begin + 29;
-    if (tid == 64) {         // the list does not depend on the picks: laid out while the front's copies travel
-        int c2[kMaxTokens], c3[kMaxTokens];
-        for (int t = 0; t < T; ++t) {
-            int ct = cta + t * (wcta / kMaxTokens);
-            if (ct >= wcta) ct -= wcta;
-            tok_cta[t] = ct;
-            c2[t] = cta < wcta && u_tok > ct ? (u_tok - ct + wcta - 1) / wcta : 0;
-            const int vb = static_cast<int>(static_cast<unsigned>(ct) * static_cast<unsigned>(v_tok) / static_cast<unsigned>(wcta));
-            const int ve = cta < wcta ? static_cast<int>(static_cast<unsigned>(ct + 1) * static_cast<unsigned>(v_tok) / static_cast<unsigned>(wcta)) : vb;
-            tok_vb[t] = vb;
-            tok_jl0[t] = vb >> P.t3_log2;
-            c3[t] = ve - vb;
-            tok_ng[t] = ve > vb ? (((ve - 1) >> P.t3_log2) - (vb >> P.t3_log2) + 1) * P.nsb_f : 0;   // activation superblocks of the run
-        }
-        int at = 0, k = 0;
-        auto add = [&](int t, int down) {
-            seg_begin[k] = at;
-            seg_info[k] = t * 2 + down;
-            at += down ? c3[t] : 2 * c2[t];
-            ++k;
-        };
-        add(0, 0);
-        if (T > 1) add(1, 0);
-        for (int t = 0; t < T; ++t) {
-            if (t + 2 < T) add(t + 2, 0);
-            add(t, 1);
-        }
-        seg_begin[k] = at;
-    }
+    const BatchList list(reinterpret_cast<int *>(sm + P.off_seg));
+    if (tid == 64) batch_lay_out(list, T, P.K, P.t2_log2, P.t3_log2, P.nsb_f, cta, wcta);   // does not depend on the picks: laid out while the front's copies travel
     // ---- the copies of the front (into the ring's memory): the T activations, the router tasks and shared gate/up
     // tasks of this CTA, the slot table, the shared gate vector (one CTA) ----
     const int n_rt = P.E >> 2, n_st = P.SF >> 2;
@@ -372,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
             __syncthreads();
         }
     }
-    int n_tiles = seg_begin[2 * T];
+    int n_tiles = list.begin[2 * T];
     const int n_sd = P.SF > 0 ? (P.H >> 2) : 0;
     int my_sd = n_sd > cta ? (n_sd - cta + ncta - 1) / ncta : 0;
     bool stopped = false;
@@ -380,11 +431,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     const int ns = static_cast<int>(P.ring);
     const int act_per_tok = n_exp_tok * P.nsb_f;
     // Every task's description, worked out once (the walk further down runs while the integer pipes are saturated by
-    // the decoders, so it must be short), here while the picks travel: the offset of its tile inside an expert's
-    // slot (the slot's address is added once the picks are known), and
-    //   desc: bit 0 down tile, 1-2 token, 3-8 pair, 9-20 tile inside the pair's matrix, 21 up tile (else gate),
-    //         22-27 one more than the activation superblock this task's warp gathers afterwards (0: none)
-    //   aux : gate/up tile: entry of the pair buffer; down tile: first activation superblock of its pair
+    // the decoders, so it must be short), here while the picks travel, and the offset of its tile inside an expert's
+    // slot (the slot's address is added once the picks are known)
 #pragma unroll 1
     for (int attempt = 0;; ++attempt) {         // a second time only when a proof replaced picked ids (WIDE)
     uint64_t *tbars = bars + (attempt ? kBatchMaxBars : 0);       // ring slots and activations
@@ -394,37 +442,11 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
     int *task_aux = reinterpret_cast<int *>(task_desc + P.max_tasks);
 #pragma unroll 1
     for (int i = tid; i < n_tiles; i += kThreads) {
-        int k = 0;
-        while (k + 1 < 2 * T && i >= seg_begin[k + 1]) ++k;
-        const int t = seg_info[k] >> 1, down = seg_info[k] & 1, li = i - seg_begin[k];
-        uint32_t d;
-        unsigned long long src;
         int aux;
-        if (!down) {
-            const int u = tok_cta[t] + (li >> 1) * wcta;
-            const int pair = t * P.K + (u >> P.t2_log2), tile = u & ((1 << P.t2_log2) - 1);
-            src = ((li & 1) ? P.up_off : P.gate_off) + static_cast<unsigned long long>(tile) * P.gu_tile;
-            d = static_cast<uint32_t>(t << 1) | static_cast<uint32_t>(pair << 3) | static_cast<uint32_t>(tile << 9) |
-                static_cast<uint32_t>((li & 1) << 21);
-            aux = ((i - (li & 1)) >> 1) & 31;
-        } else {
-            const int v = tok_vb[t] + li;
-            const int pl = v >> P.t3_log2, tile = v & ((1 << P.t3_log2) - 1);
-            const int pair = t * P.K + pl;
-            src = P.down_off + static_cast<unsigned long long>(tile) * P.d_tile;
-            d = 1u | static_cast<uint32_t>(t << 1) | static_cast<uint32_t>(pair << 3) | static_cast<uint32_t>(tile << 9);
-            aux = t * act_per_tok + (pl - tok_jl0[t]) * P.nsb_f;
-        }
-        // the gathers of a down segment are handed to the tasks that end a round (16 tasks) before it starts
-#pragma unroll 1
-        for (int kd = 0; kd < 2 * T; ++kd) {
-            if (!(seg_info[kd] & 1)) continue;
-            const int td = seg_info[kd] >> 1;
-            const int base = max(0, seg_begin[kd] - kWarps - tok_ng[td]);
-            // at most one per task (short segments overlap); a gather nobody was handed is done by the first tile that needs it
-            if (i >= base && i < base + tok_ng[td] && (d >> 22) == 0u) d |= static_cast<uint32_t>(td * act_per_tok + (i - base) + 1) << 22;
-        }
-        task_src[i] = src;
+        const uint32_t d = batch_task(list, i, T, P.K, P.t2_log2, P.t3_log2, P.nsb_f, act_per_tok, wcta, aux);
+        const unsigned tile = (d >> 9) & 4095u;
+        task_src[i] = (d & 1u) ? P.down_off + static_cast<unsigned long long>(tile) * P.d_tile
+                               : (((d >> 21) & 1u) ? P.up_off : P.gate_off) + static_cast<unsigned long long>(tile) * P.gu_tile;
         task_desc[i] = d;
         task_aux[i] = aux;
     }
@@ -541,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
         const int t = g / act_per_tok, r = g - t * act_per_tok;
         const int pl = r / P.nsb_f, sbk = r - pl * P.nsb_f;
         float av[8];
-        wait_tagged<8>(t_act + static_cast<size_t>(t * P.K + tok_jl0[t] + pl) * P.F + sbk * 256 + lane, 32, 8, tag, av, err);
+        wait_tagged<8>(t_act + static_cast<size_t>(t * P.K + list.jl0[t] + pl) * P.F + sbk * 256 + lane, 32, 8, tag, av, err);
 #pragma unroll
         for (int k = 0; k < 8; ++k) scr[lane + 32 * k] = av[k];
         __syncwarp();
