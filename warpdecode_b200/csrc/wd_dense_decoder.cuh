@@ -221,25 +221,6 @@ struct BlockInput {
     static constexpr int kBlockBytes = 40;
 };
 
-// Weights that a later kernel of the step reads, asked into L2 by one that has its own loads under way: left to themselves they
-// cross DRAM only while the kernel that needs them runs, which is half of the step. Up to two ranges, in pieces of 4 KB, one lane per
-// piece. The qkv product asks for the layer's gate/up matrix, wo for w_down, gate/up for the next layer's qkv and wo.
-struct L2Ahead {
-    const uint8_t *p[2];
-    unsigned bytes[2];          // multiples of 16
-    __device__ __forceinline__ void request() const {
-        constexpr unsigned kPiece = 4096;
-        if ((threadIdx.x & 31) != 0) return;
-        const unsigned warp = threadIdx.x >> 5, first = warp * gridDim.x + blockIdx.x, step = (blockDim.x >> 5) * gridDim.x;
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-            for (unsigned i = first; i < (bytes[k] + kPiece - 1) / kPiece; i += step) {
-                const unsigned n = min(kPiece, bytes[k] - i * kPiece);
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p[k] + static_cast<size_t>(i) * kPiece), "r"(n) : "memory");
-            }
-    }
-};
-
 // A block of 32 weights of a packed matrix, and its term of a row's chain: fmaf(d_w * d_x, (float)int_dot, acc).
 template <bool Q8>
 struct RowBlock {
@@ -249,6 +230,19 @@ struct RowBlock {
 #pragma unroll
         for (int i = 0; i < (Q8 ? 2 : 1); ++i) q[i] = __ldg(quants + (Q8 ? 2 : 1) * blk + i);
         d = __ldg(scales + blk);
+    }
+    // The same in front of grid_dep_wait(), by ordinary loads that the wait's memory clobber holds in place: read-only (nc) loads, volatile
+    // or not, end up behind it, where their values are first used, and the weights then set out only when the kernel in front has ended.
+    // us per token, nc / ordinary / ordinary past L1 (this): 342 / 304 / 303 with 16 layers of 2048 / 8192 and a 128256-row head, 180 / 165 /
+    // 163 with 12 of 1024 / 2816, 215 / 197 / 199 with 8 Q8_0 layers of 2048 / 8192.
+    __device__ __forceinline__ void load_early(const uint4 *quants, const uint16_t *scales, size_t blk) {
+#pragma unroll
+        for (int i = 0; i < (Q8 ? 2 : 1); ++i)
+            asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(q[i].x), "=r"(q[i].y), "=r"(q[i].z), "=r"(q[i].w)
+                         : "l"(quants + (Q8 ? 2 : 1) * blk + i)
+                         : "memory");
+        asm volatile("ld.global.L1::no_allocate.u16 %0, [%1];" : "=h"(d) : "l"(scales + blk) : "memory");
     }
     // lo, hi: quants 0 .. 15 and 16 .. 31 of the activation's block; x: its scale (as bits) and -8 times the sum of its quants
     __device__ __forceinline__ float term(const uint4 &lo, const uint4 &hi, const int2 &x, float acc) const {
@@ -283,7 +277,7 @@ struct RowBlock {
 // bytes. U blocks per lane in flight: with one warp per row every byte of the matrix is requested at once.
 template <bool Q8, int U>
 __global__ void __launch_bounds__(kDecThreads, 4) dense_product_kernel(const uint8_t *wp, int rows, int nb, const int8_t *xq, const float *xd,
-                                                                      float *y, L2Ahead ahead) {
+                                                                      float *y) {
     extern __shared__ __align__(16) uint8_t dsm[];
     grid_dep_launch();
     const BlockInput in(dsm, nb);
@@ -291,15 +285,11 @@ __global__ void __launch_bounds__(kDecThreads, 4) dense_product_kernel(const uin
     const uint4 *q_all = reinterpret_cast<const uint4 *>(wp);
     const uint16_t *d_all = reinterpret_cast<const uint16_t *>(wp + static_cast<size_t>(rows) * stride * (Q8 ? 32 : 16));
     RowBlock<Q8> w[U];
-    auto load = [&](int b0) {
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (b0 + 32 * u < nb && row < rows) w[u].load(q_all, d_all, static_cast<size_t>(row) * stride + b0 + 32 * u);
-    };
     // The weights do not depend on the kernel before this one: the first loads leave before the wait for it, and the
     // activation (its output) is fetched after.
-    load(lane);
-    ahead.request();
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (lane + 32 * u < nb && row < rows) w[u].load_early(q_all, d_all, static_cast<size_t>(row) * stride + lane + 32 * u);
     grid_dep_wait();
 #pragma unroll 2
     for (int i = threadIdx.x; i < ((nb * 2 + 31) & ~31); i += kDecThreads) {        // half a block per thread; whole warps
@@ -319,7 +309,11 @@ __global__ void __launch_bounds__(kDecThreads, 4) dense_product_kernel(const uin
     float acc = 0.0f;
 #pragma unroll 1
     for (int b0 = lane; b0 < nb; b0 += 32 * U) {
-        if (b0 != lane) load(b0);
+        if (b0 != lane) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (b0 + 32 * u < nb) w[u].load(q_all, d_all, static_cast<size_t>(row) * stride + b0 + 32 * u);
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int b = b0 + 32 * u;
@@ -737,7 +731,9 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
 // already on their way (2.2 us from the end of the kernel in front to the first product). CTAs of 512 threads, two per SM, so
 // that an SM reads hidden and proj twice and not four times.
 // Measured, 16 layers of 2048 / 8192 and a 128256-row head, 72 positions: 376 us per token with separate norm, product and
-// SwiGLU kernels, 386 with this kernel, 312 with the later weights asked into L2 (L2Ahead) and the cheaper block term.
+// SwiGLU kernels, 303 with this kernel and its first weight loads in front of the wait (RowBlock::load_early; 342 behind it). Matrices of
+// later kernels asked into L2 ahead of them gain nothing beside that: 305 us here, and where a layer's matrices approach the size of L2
+// they cost 6 to 25 % (4096 / 16384: 220 -> 245 us with 5 Q4_0 layers, 188 -> 235 with 3 Q8_0 layers).
 // MODE 0: y[row]; 1: rows are [ffn gate rows | ffn up rows], and a CTA takes 32 of both at once: SiLU(g) * u is quantised to
 // Q8_0 where it is formed (swiglu_kernel, :1956), without a kernel and a pass over memory of its own; 2: y[row] and the
 // arg-max of the finite results: key = order_key(value) << 32 | ~row, so the largest value wins and
@@ -746,7 +742,7 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
 constexpr int kNormProductThreads = 512;
 template <bool Q8, int R, int U, int MODE, int PASSES>
 __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_kernel(NormInput in, const uint8_t *wp, int rows, float *y,
-                                                                                   unsigned long long *key, int8_t *oq, float *od, L2Ahead ahead) {
+                                                                                   unsigned long long *key, int8_t *oq, float *od) {
     static_assert(MODE != 1 || R == 4, "two gate rows and two up rows per warp");
     constexpr int kWarpsHere = kNormProductThreads / 32;
     extern __shared__ __align__(16) uint8_t dsm[];
@@ -763,18 +759,21 @@ __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_ker
     };
     const int units = MODE == 1 ? rows >> 6 : (rows + kWarpsHere * R - 1) / (kWarpsHere * R);
     RowBlock<Q8> w[R][U];
-    auto load = [&](int unit, int b0) {
+    auto load = [&](int unit, int b0, bool early) {
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int b = b0 + 32 * u, row = row_of(unit, r);
-                if (b < nb && (MODE == 1 || row < rows)) w[r][u].load(q_all, d_all, static_cast<size_t>(row) * stride + b);
+                if (b < nb && (MODE == 1 || row < rows)) {
+                    const size_t blk = static_cast<size_t>(row) * stride + b;
+                    if (early) w[r][u].load_early(q_all, d_all, blk);
+                    else w[r][u].load(q_all, d_all, blk);
+                }
             }
     };
     int unit = blockIdx.x;
-    load(unit, lane);           // weights do not depend on the kernel before this one
-    ahead.request();
+    load(unit, lane, true);           // weights do not depend on the kernel before this one
     dense_norm_quant_body<PASSES>(in, [] { grid_dep_wait(); }, [&](int e, uint32_t packed, float d) {
         const int b = e >> 5, j = e & 31;
         *reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>((j & 16) ? x.hi + b : x.lo + b) + (j & 15)) = packed;
@@ -791,7 +790,7 @@ __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_ker
         for (int r = 0; r < R; ++r) acc[r] = 0.0f;
 #pragma unroll 1
         for (int b0 = lane; b0 < nb; b0 += 32 * U) {
-            if (unit != static_cast<int>(blockIdx.x) || b0 != lane) load(unit, b0);
+            if (unit != static_cast<int>(blockIdx.x) || b0 != lane) load(unit, b0, false);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int b = b0 + 32 * u;
