@@ -192,12 +192,13 @@ __device__ __forceinline__ void iq_tile_rows(const int partial[8], float scale, 
     __syncwarp();
 }
 
-// The same for the two row lengths of the 48-layer model (eight superblocks: gate/up rows, two: down rows), without loops:
-// every value and scale of a chain is requested before the first step. Used by the wide decoders, whose integer side is
-// short enough for the dependent loads of the general form to show.
+// The same for rows of NSB = 1, 2, 4 or 8 superblocks (of the admissible lengths all but hidden 4096 and 8192), without loops: every
+// value and scale of a chain is requested before the first step. Used by the wide decoders, whose integer side is short
+// enough for the dependent loads of the general form to show. Fixed forms of 16 and 32 gain nothing (hidden 4096: 28.2 us per layer either way).
 template <int NSB>
 __device__ __forceinline__ void iq_tile_rows_fixed(const int partial[8], float scale, int lane, float *scr, float *rows_out, float post) {
     constexpr int R = 32 / NSB, kStripe = NSB * 8 + 8;
+    static_assert(R % 4 == 0, "four rows of chunk-lanes per step");
     float *dst = scr + (lane / NSB) * kStripe + (lane % NSB) * 8;
     *reinterpret_cast<float4 *>(dst) = make_float4(static_cast<float>(partial[0]), static_cast<float>(partial[1]),
                                                    static_cast<float>(partial[2]), static_cast<float>(partial[3]));
@@ -270,27 +271,44 @@ __device__ __forceinline__ void wide_partials(int kind, const uint8_t *tile, int
     if (kind == kWide + kTypeIq2s) wide2_partials<UNROLL>(tile, lane, a, p, i0, i1);
     else wide3_partials<UNROLL>(tile, lane, a, p, i0, i1);
 }
-// float side of a wide tile whose integer sums are known
+// float side of a wide tile whose integer sums are known. A, B: the superblocks per row that occur, A <= B, 0 for those beyond 8; or
+// kAnyRows for both. The layer kernel is compiled for the pair of its engine: a layer's code runs once and is fetched cold, and with all
+// four fixed forms in it a stack step of the 48-layer model takes 19.9 us per layer instead of 18.4. us per layer with fixed forms of 8 and 2 alone
+// in every kernel -> the engine's own pair: 2048 / 512 19.2 -> 18.4, 1024 / 512 17.6 -> 16.3, 1024 / 1024 19.8 -> 19.0, 512 / 256 15.2 ->
+// 14.1, 256 / 256 15.9 -> 14.1, 4096 / 512 29.8 -> 29.9. The batch kernel, whose decoder loops over many tiles, holds them all: four-token
+// calls at 1024 / 1024 29.3 -> 28.3 us, 2048 / 512 unchanged.
+constexpr int kAnyRows = -1;
+template <int A, int B>
 __device__ __forceinline__ void wide_rows(int kind, const uint8_t *tile, const int p[8], float dx, int nsb, int lane, float *scr, float *rows_out) {
     const float dw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(tile + wide_tile_off_d(kind - kWide) + lane * 2));
     const float scale = __fmul_rn(dw, dx), post = iq_row_post(kind - kWide);
-    if (nsb == 8) iq_tile_rows_fixed<8>(p, scale, lane, scr, rows_out, post);
-    else if (nsb == 2) iq_tile_rows_fixed<2>(p, scale, lane, scr, rows_out, post);
-    else iq_tile_rows(p, scale, nsb, lane, scr, rows_out, post);
+    if constexpr (A == kAnyRows) {
+        if (nsb == 8) iq_tile_rows_fixed<8>(p, scale, lane, scr, rows_out, post);
+        else if (nsb == 4) iq_tile_rows_fixed<4>(p, scale, lane, scr, rows_out, post);
+        else if (nsb == 2) iq_tile_rows_fixed<2>(p, scale, lane, scr, rows_out, post);
+        else if (nsb == 1) iq_tile_rows_fixed<1>(p, scale, lane, scr, rows_out, post);
+        else iq_tile_rows(p, scale, nsb, lane, scr, rows_out, post);
+    } else if constexpr (A == 0) {
+        if (B != 0 && nsb == B) iq_tile_rows_fixed<B == 0 ? 1 : B>(p, scale, lane, scr, rows_out, post);
+        else iq_tile_rows(p, scale, nsb, lane, scr, rows_out, post);
+    } else {
+        if (A == B || nsb == B) iq_tile_rows_fixed<B>(p, scale, lane, scr, rows_out, post);
+        else iq_tile_rows_fixed<A>(p, scale, lane, scr, rows_out, post);
+    }
 }
-template <int UNROLL>
+template <int UNROLL, int A, int B>
 __device__ __noinline__ void wide_tile_to_rows(int kind, const uint8_t *tile, const uint8_t *a, float dx, int nsb, int lane, float *scr,
                                                float *rows_out) {
     int p[8];
     wide_partials<UNROLL>(kind, tile, lane, a, p, 0, 8);
-    wide_rows(kind, tile, p, dx, nsb, lane, scr, rows_out);
+    wide_rows<A, B>(kind, tile, p, dx, nsb, lane, scr, rows_out);
 }
 
 // What a layer kernel calls: the decoder of its pool's form. UNROLL: sub-blocks per loop iteration of the compact decoder.
-template <bool WIDE, int UNROLL>
+template <bool WIDE, int UNROLL, int A = kAnyRows, int B = kAnyRows>
 __device__ __forceinline__ void tile_to_rows(int kind, const uint8_t *tile, const uint8_t *a, float dx, int nsb, int lane, uint32_t lane4x2,
                                              const uint8_t *tab3, const uint8_t *tab2, float *scr, float *rows_out) {
-    if constexpr (WIDE) wide_tile_to_rows<8>(kind, tile, a, dx, nsb, lane, scr, rows_out);
+    if constexpr (WIDE) wide_tile_to_rows<8, A, B>(kind, tile, a, dx, nsb, lane, scr, rows_out);
     else iq_tile_to_rows_any<UNROLL>(kind, tile, a, dx, nsb, lane, lane4x2, tab3, tab2, scr, rows_out, nullptr);
 }
 // integer sums of sub-blocks [i0, i1)
@@ -301,10 +319,10 @@ __device__ __forceinline__ void tile_partials(int kind, const uint8_t *tile, con
     else if (kind == kTypeIq2s) iq2_block_partials_range(tile, lane, a, tab2, p, i0, i1);
     else iq3_block_partials_range(tile, lane, a, lane4x2, tab3, p, i0, i1);
 }
-template <bool WIDE>
+template <bool WIDE, int A = kAnyRows, int B = kAnyRows>
 __device__ __forceinline__ void tile_rows(int kind, const uint8_t *tile, const int p[8], float dx, int nsb, int lane, float *scr, float *rows_out) {
     if constexpr (WIDE) {
-        wide_rows(kind, tile, p, dx, nsb, lane, scr, rows_out);
+        wide_rows<A, B>(kind, tile, p, dx, nsb, lane, scr, rows_out);
     } else {
         const float dw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(tile + iq_tile_off_d(kind) + lane * 2));
         iq_tile_rows(p, __fmul_rn(dw, dx), nsb, lane, scr, rows_out, iq_row_post(kind));

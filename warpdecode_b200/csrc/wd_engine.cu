@@ -596,8 +596,29 @@ int sync_layer_table(wd_engine *e, cudaStream_t s) {
     return WD_OK;
 }
 
+// The layer kernel for the engine's two row lengths (gate/up and down rows), the shorter one first, 0 for those beyond 8 superblocks.
+template <int A, int B>
+const void *wide_layer_kernel() { return reinterpret_cast<const void *>(wd::moe_layer_kernel<true, A, B>); }
 const void *layer_kernel(const wd_engine *e) {
-    return e->wide ? reinterpret_cast<const void *>(wd::moe_layer_kernel<true>) : reinterpret_cast<const void *>(wd::moe_layer_kernel<false>);
+    if (!e->wide) return reinterpret_cast<const void *>(wd::moe_layer_kernel<false, 0, 0>);
+    const auto count = [](int nsb) { return nsb <= 8 ? nsb : 0; };
+    const int a = std::min(count(e->nsb_h), count(e->nsb_f)), b = std::max(count(e->nsb_h), count(e->nsb_f));
+    switch (a * 16 + b) {
+        case 0x11: return wide_layer_kernel<1, 1>();
+        case 0x12: return wide_layer_kernel<1, 2>();
+        case 0x14: return wide_layer_kernel<1, 4>();
+        case 0x18: return wide_layer_kernel<1, 8>();
+        case 0x22: return wide_layer_kernel<2, 2>();
+        case 0x24: return wide_layer_kernel<2, 4>();
+        case 0x28: return wide_layer_kernel<2, 8>();
+        case 0x44: return wide_layer_kernel<4, 4>();
+        case 0x48: return wide_layer_kernel<4, 8>();
+        case 0x88: return wide_layer_kernel<8, 8>();
+        case 0x01: return wide_layer_kernel<0, 1>();
+        case 0x02: return wide_layer_kernel<0, 2>();
+        case 0x04: return wide_layer_kernel<0, 4>();
+        default: return wide_layer_kernel<0, 8>();
+    }
 }
 const void *batch_kernel(const wd_engine *e) {
     return e->wide ? reinterpret_cast<const void *>(wd::moe_batch_kernel<true>) : reinterpret_cast<const void *>(wd::moe_batch_kernel<false>);

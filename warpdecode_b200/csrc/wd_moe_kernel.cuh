@@ -223,7 +223,8 @@ __device__ __forceinline__ void issue_phase1_copies(const MoeParams &P, const La
 extern __shared__ __align__(128) uint8_t wd_smem[];
 
 // WIDE: the pool holds wide tiles (wd_formats.cuh), gu_type / d_type are their kinds and no codebook is needed.
-template <bool WIDE>
+// A, B: the superblocks per row of its gate/up and down tiles, the smaller first (wide_rows; 0, 0 with compact tiles).
+template <bool WIDE, int A, int B>
 __global__ void __launch_bounds__(kThreads, 1) moe_layer_kernel(const __grid_constant__ MoeParams P) {
     uint8_t *sm = wd_smem;
     uint8_t *tab = sm + P.off_tab;                                   // IQ3_S codebook, lane-private copies
