@@ -99,3 +99,20 @@ def test_attention_of_a_long_decoder_at_its_first_positions(wd, oracle):
     ref = _oracle_for(wd, oracle, dec, cfg, 500000.0)
     assert np.array_equal(got, ref.decode(np.arange(2), 130))
     dec.close()
+
+
+@pytest.mark.parametrize("P", [1021, 1100, 8186])
+def test_attention_with_the_fewest_slots(wd, oracle, P):
+    """Heads of 128 and the longest context leave four slots of 256 positions per CTA: the first refilled chunk, the one behind
+    it, and the end of the range."""
+    cfg = dict(hidden=256, n_heads=1, n_kv_heads=1, head_dim=128, ffn=64, vocab=500, n_layers=1, max_ctx=8192, rms_eps=1e-5)
+    dec = wd.DenseDecoder(256, 1, 1, 128, 64, 500, 1, 8192, 1e-5, 500000.0)
+    dec.synth(11, 0.05)
+    prompt = np.random.Generator(np.random.PCG64(P)).integers(0, 500, P)
+    got, _ = dec.decode(prompt, 6)
+    logits, hidden = dec.read()
+    ref = _oracle_for(wd, oracle, dec, cfg, 500000.0)
+    assert np.array_equal(got, ref.decode(prompt, 6))
+    assert np.array_equal(ol.fbits(logits), ol.fbits(ref.logits))
+    assert np.array_equal(ol.fbits(hidden), ol.fbits(ref.hidden))
+    dec.close()

@@ -19,6 +19,7 @@
 namespace wd {
 
 constexpr int kDecThreads = 256;
+constexpr int kDenseMaxCtx = 8192;      // longest context a decoder may be created for
 
 // Blocks per row in the packed layouts: rounded up, so that a row's scales start on 8 bytes (the prompt pass copies four).
 // The blocks behind a row's end are never read.
@@ -476,6 +477,10 @@ struct DecodeAttn {
     static constexpr int kSlot = kChunk * kRow > kChunkV * kRowV ? kChunk * kRow : kChunkV * kRowV;      // floats
     static constexpr int kSlotBytes = kSlot * 4;
     static constexpr int kRoom = 190 * 1024;                    // slots and scores together; the rest of an SM is for the product before it
+    // Values longer than the ring are refilled: after chunk c is consumed, chunk c + slots is requested, and chunk c + 1 is read once
+    // all but the kInFlight youngest requests have landed. It was requested `slots` - 1 requests before the youngest.
+    static constexpr int kInFlight = 3;
+    static_assert((kRoom - kDenseMaxCtx * 4) / kSlotBytes > kInFlight, "a refilled chunk would be read before it has landed");
     static int want(int max_ctx) { return ((max_ctx + kChunk - 1) / kChunk + C - 1) / C + (max_ctx + kChunkV - 1) / kChunkV; }
     // slots of the ring: both caches of the longest context, or what fits beside its scores
     static int slots(int max_ctx) {
@@ -705,11 +710,11 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
                 acc = __fmaf_rn(p[r], v[r * kRowV], acc);
             }
         }
-        if (n_vchunks > slots) {     // longer than the ring: refill the slot; when a refilled chunk is read, more than three requests are younger
+        if (n_vchunks > slots) {     // longer than the ring: refill the slot
             __syncthreads();
             request(n_chunks + c + slots);
             cp_async_commit();
-            cp_async_wait<3>();
+            cp_async_wait<A::kInFlight>();
             __syncthreads();
         }
     }
