@@ -529,7 +529,11 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
     if constexpr (C > 1) cluster_arrive();          // answered before the first store into a peer
     const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0;
     const int h = blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int pos = *pos_ptr, kv_dim = kv_heads * HD, kvh = (h * kv_heads) / heads;
+    // The position comes from the finish kernel of the token before. That kernel has ended (it releases nothing early), but this is in
+    // front of the wait, so its store is ordered by the fence behind it and read past L1.
+    int pos;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(pos) : "l"(pos_ptr) : "memory");
+    const int kv_dim = kv_heads * HD, kvh = (h * kv_heads) / heads;
     float *kc = kcache + static_cast<size_t>(kvh) * HD, *vc = vcache + static_cast<size_t>(kvh) * HD;
     // positions 0 .. pos - 1: this CTA's key chunks (every C-th), then all value chunks of its slice
     const int n_chunks = ((pos + kChunk - 1) / kChunk - rank + C - 1) / C, n_vchunks = (pos + kChunkV - 1) / kChunkV, n_items = n_chunks + n_vchunks;
@@ -866,6 +870,7 @@ __global__ void dense_finish_kernel(unsigned long long *key, int *token, int *po
     *token = t;
     *pos = p;
     *key = 0ull;
+    __threadfence();        // the next token's attention reads the position in front of its wait
 }
 
 }  // namespace wd
