@@ -116,3 +116,54 @@ def test_attention_with_the_fewest_slots(wd, oracle, P):
     assert np.array_equal(ol.fbits(logits), ol.fbits(ref.logits))
     assert np.array_equal(ol.fbits(hidden), ol.fbits(ref.hidden))
     dec.close()
+
+
+def test_a_decoder_without_room_for_the_prompt_workspace(wd):
+    """The prompt pass wants 78 MB beside this decoder's tensors. With less left it reads fewer positions at a time, with nearly
+    nothing the steps read the prompt: tokens and logits are the same, and so they are after tensors have changed their type."""
+    import gc
+    import torch
+    from warpdecode_b200 import synth
+    P, G, V, F = 400, 40, 500, 16384
+    prompt = np.random.Generator(np.random.PCG64(1)).integers(0, V, P)
+    q8 = synth.quantize_q8_0((np.random.Generator(np.random.PCG64(2)).standard_normal((256, F)) * 0.05).astype(np.float32)).reshape(-1)
+
+    def run(dec):
+        dec.synth(4, 0.05)
+        a = dec.decode(prompt, G)[0].copy(), dec.read()[0].copy()
+        dec.close()
+        return a
+
+    def create():
+        return wd.DenseDecoder(256, 2, 1, 64, F, V, 1, 512, 1e-5, 500000.0)
+
+    def run_q8(dec):
+        dec.synth(4, 0.05)
+        dec.set_tensor(0, wd.DT_W_DOWN, q8, wd.TYPE_Q8_0)
+        a = dec.decode(prompt, G)[0].copy(), dec.read()[0].copy()
+        dec.close()
+        return a
+    want, want8 = run(create()), run_q8(create())
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    least = None
+    for left in list(range(12, 64, 2)):                     # the least memory this decoder can be created in
+        hog = torch.empty(free - (left << 20), dtype=torch.uint8, device="cuda")
+        try:
+            create().close()
+            least = left
+        except wd.WdError:
+            pass
+        del hog
+        gc.collect()
+        torch.cuda.empty_cache()
+        if least is not None:
+            break
+    assert least is not None
+    for more in (16, 90, 110, 200):
+        hog = torch.empty(free - ((least + more) << 20), dtype=torch.uint8, device="cuda")
+        for got, ref in ((run(create()), want), (run_q8(create()), want8)):
+            assert np.array_equal(got[0], ref[0]) and np.array_equal(ol.fbits(got[1]), ol.fbits(ref[1])), more
+        del hog
+        gc.collect()
+        torch.cuda.empty_cache()
