@@ -118,3 +118,71 @@ def test_plain_layout_picks_from_a_threshold_or_the_rungs(oracle, E, K, scale):
         assert np.array_equal(bits(out[t]), bits(want["out"])), t
     assert eng.device_status() == 0
     eng.close()
+
+
+@pytest.mark.parametrize("H,F,gate,down,f32", [(2048, 512, 22, 22, False), (2560, 640, 22, 20, True)])
+def test_the_wide_form_leaves_the_program_its_memory(monkeypatch, H, F, gate, down, f32):
+    """What the wide form takes beyond the file's form is at most a quarter of the memory that one would leave; an engine
+    in the file's form serves where the wide one does not fit."""
+    import gc
+    import torch
+    import warpdecode_b200 as wd
+    monkeypatch.delenv("WD_WIDE_TILES", raising=False)
+    E, L, GB = 512, 12, 1 << 30
+    compact = L * E * (2 * F * (H // 256) * 82 + (H * (F // 32) * 18 if down == 20 else H * (F // 256) * 82))
+    if f32:
+        wide = L * E * 3 * H * F // 64 * 36
+    else:
+        wide = L * E * 3 * (F * (H // 256) // 32) * 4416
+
+    def wide_engine(left):
+        gc.collect()
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+        before = torch.cuda.mem_get_info()[0]
+        eng = wd.Engine(H, F, E, 8, 128, L, expert_type=gate, down_type=down, router_f32=f32)
+        # the plain-layout path allocates the file's form when the tensors are set, the wide one at creation
+        took = before - torch.cuda.mem_get_info()[0]
+        eng.close()
+        del hog
+        return took > (wide + compact) // 2 if not f32 else took > wide // 2
+    wd.Engine(H, F, E, 8, 128, 1, expert_type=gate, down_type=down, router_f32=f32).close()        # context, modules
+    need = compact + 4 * (wide - compact)
+    assert need > wide + 4 * GB                             # the quarter is the tighter bound at this size
+    assert wide_engine(need + GB // 2)
+    assert not wide_engine(need - GB)
+    assert not wide_engine(wide + 4 * GB + GB // 2)         # fits, and would leave 4 GiB, but too little of the rest
+    assert not wide_engine(compact + GB)
+
+
+def test_two_plain_engines_created_before_their_tensors_are_set(oracle):
+    """Each engine has its buffers when the next one looks at the free memory."""
+    import warpdecode_b200 as wd
+    H, F, E, K, SF = 768, 192, 16, 3, 128
+    ms = [synth.make_moe_block(50 + i, H, F, E, K, SF, 21, 20) for i in range(2)]
+    engs = [wd.Engine(H, F, E, K, SF, 1, expert_type=21, down_type=20) for _ in ms]
+    x = np.random.Generator(np.random.PCG64(9)).standard_normal(H).astype(np.float32)
+    for e, m in zip(engs, ms):
+        e.load_block(0, m)
+    for e, m in zip(engs, ms):
+        assert np.array_equal(bits(e.forward_host(0, x)), bits(oracle.moe_block(m, x)["out"]))
+        e.close()
+
+
+def test_a_fused_gate_up_tensor_in_several_parts(oracle):
+    """Three experts fit the staging buffer at this shape: eight go through it as 3 + 3 + 2 (down rows in ragged parts likewise)."""
+    import warpdecode_b200 as wd
+    H, F, E, K = 768, 576, 8, 4
+    m = synth.make_moe_block(61, H, F, E, K, 128, 21, 20)
+    eng = wd.Engine(H, F, E, K, 128, 1, expert_type=21, down_type=20)
+    eng.load_block(0, m)
+    x = np.random.Generator(np.random.PCG64(3)).standard_normal(H).astype(np.float32)
+    want = bits(oracle.moe_block(m, x)["out"])
+    assert np.array_equal(bits(eng.forward_host(0, x)), want)
+    rng = np.random.Generator(np.random.PCG64(4))
+    m2 = dict(m, gate=synth.random_blocks(rng, 21, E * F * H // 256), up=synth.random_blocks(rng, 21, E * F * H // 256))
+    fused = np.concatenate([np.asarray(m2[k]).reshape(E, -1) for k in ("gate", "up")], axis=1).copy()
+    down = np.ascontiguousarray(m2["down"])
+    wd._check(wd.lib().wd_set_experts_fused(eng.h, 0, fused.ctypes.data, 21, down.ctypes.data, 20))
+    assert np.array_equal(bits(eng.forward_host(0, x)), bits(oracle.moe_block(m2, x)["out"]))
+    eng.close()

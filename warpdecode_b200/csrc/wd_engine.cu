@@ -410,21 +410,27 @@ int plan_shared_memory(wd_engine *e) {
     return WD_OK;
 }
 
-// Wide tiles (wd_formats.cuh) are the faster form wherever they can be kept: every owned expert resident, the larger pool
-// within the caller's cache_mib or (when that is open) within the free memory less 4 GiB for everything else of the
-// program, the tiles of a CTA's share within shared memory, and the generic kernels running. Otherwise compact tiles.
+// Room for the wide form of the experts: `wide` bytes where the compact form takes `compact`. A program that creates its engine
+// first and allocates afterwards counts on what the compact form leaves, so the wide form takes at most a quarter of that on top, leaves 4 GiB in
+// any case, and stays within the caller's cache_mib where that is given. WD_WIDE_TILES=0: never.
+bool wide_fits(const wd_config &c, size_t compact, size_t wide) {
+    if (const char *v = std::getenv("WD_WIDE_TILES"))
+        if (v[0] == '0') return false;
+    if (c.cache_mib > 0 && wide > static_cast<size_t>(c.cache_mib) << 20) return false;
+    size_t room = 0, total = 0;
+    if (cudaMemGetInfo(&room, &total) != cudaSuccess) return false;
+    return room > compact && wide + (4ull << 30) <= room && wide - std::min(compact, wide) <= (room - compact) / 4;
+}
+
+// Wide tiles (wd_formats.cuh) are the faster form wherever they can be kept: every owned expert resident, room for the
+// larger pool, the tiles of a CTA's share within shared memory, and the generic kernels running. Otherwise compact tiles.
 void choose_slot_form(wd_engine *e) {
     const wd_config &c = e->cfg;
     if (!e->resident || (c.shared_ffn > 0 && find_fast_kernel(c))) return;
-    if (const char *v = std::getenv("WD_WIDE_TILES"))
-        if (v[0] == '0') return;
+    const size_t compact = static_cast<size_t>(e->n_slots) * e->slot_bytes;
     set_slot_form(e, true);
-    const size_t pool = static_cast<size_t>(e->n_slots) * e->slot_bytes;
-    size_t room = 0, total = 0;
-    if (c.cache_mib > 0) room = static_cast<size_t>(c.cache_mib) << 20;
-    else if (cudaMemGetInfo(&room, &total) == cudaSuccess) room -= std::min<size_t>(room, 4ull << 30);
     set_tile_form(e);
-    if (pool > room || plan_shared_memory(e) != WD_OK) set_slot_form(e, false);
+    if (!wide_fits(c, compact, static_cast<size_t>(e->n_slots) * e->slot_bytes) || plan_shared_memory(e) != WD_OK) set_slot_form(e, false);
 }
 
 // Shared-memory plan of the batch kernel for up to cfg.max_tokens tokens. Leaves e->batch_ok false (and the batch on
@@ -1028,7 +1034,13 @@ int wd_engine_create(const wd_config *cfg, wd_engine **out) {
         return bail(WD_E_CUDA);                                                       \
     }
     WD_TRY(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
-    WD_TRY(cudaMalloc(&e->pool, static_cast<size_t>(e->n_slots) * e->slot_bytes));
+    ce = cudaMalloc(&e->pool, static_cast<size_t>(e->n_slots) * e->slot_bytes);
+    if (ce != cudaSuccess && e->wide) {
+        cudaGetLastError();
+        set_slot_form(e, false);
+        ce = cudaMalloc(&e->pool, static_cast<size_t>(e->n_slots) * e->slot_bytes);
+    }
+    WD_TRY(ce);
     e->layers.resize(c.n_layers);
     for (Layer &L : e->layers) {
         L.h_slot.assign(c.n_experts, -1);
