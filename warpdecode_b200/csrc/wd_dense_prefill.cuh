@@ -2,8 +2,8 @@
 // the float order of the one-token step (wd_dense_decoder.cuh) kept per token, so that caches, logits and tokens are
 // bit-identical to feeding the prompt token by token.
 //
-// What the step spends per prompt token is one read of every matrix and about 130 dependent launches (540 us on the
-// 16-layer benchmark model, 1.2 ms with 500 positions in the cache). Here a chunk of up to 512 tokens shares both.
+// What the step spends per prompt token is one read of every matrix and 82 dependent launches (300 us on the
+// 16-layer benchmark model, 400 with 500 positions in the cache). Here a chunk of up to 512 tokens shares both.
 #pragma once
 
 #include "wd_dense_decoder.cuh"

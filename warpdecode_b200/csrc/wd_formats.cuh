@@ -29,10 +29,12 @@
 // on four weights (index bits, codebook lookup, sign mask, negate, select, dp4a, scale); with one 4-bit code per weight the
 // codebooks are gone and four weights take 3.5. An IQ3_S weight is +-(2 m + 1), m = 0..7: with n = m or -m - 1 it is
 // 2 n + 1, so the nibble n at the top of its byte with 8 below it IS 8 * weight as an int8. An IQ2_S weight is one of
-// six values, which one prmt selects for four nibbles at once. Measured (one SM, tiles in shared memory): see
-// wide_tile_to_rows. The price is HBM bytes: 134 instead of 110 per 256 weights (IQ3_S), 138 instead of 82 (IQ2_S); the
-// expert products of a token are bound by instruction issue, not by these bytes. A capped cache keeps the compact tiles
-// (a slot then holds the most experts per byte, and a miss costs a repack of the bytes it streams).
+// six values, which one prmt selects for four nibbles at once. The price is HBM bytes: 134 instead of 110 per 256 weights (IQ3_S),
+// 138 instead of 82 (IQ2_S). us per pass of the per-layer call, compact -> wide, with the weights where the last pass left them and with L2
+// flushed before the pass: eight one-token calls at 2048 / 512 IQ3_S 205 -> 178 and 218 -> 192, eight four-token calls 331 -> 263 and 339 ->
+// 269, six two-token calls at 1024 / 512 IQ2_S 184 -> 159 and 187 -> 165 (the choice of CTAs that prove the picks is part of the
+// wide kernels). A capped cache keeps the compact tiles, because its slots then hold the most experts; what crosses the host link at a miss
+// is the file's bytes in either form, and which form serves which hit rate better has not been measured.
 //   Q   off    0: [sub-block i=0..7][lane][16 B] word k (0..3) holds chunks k and k + 4: IQ3_S in the low and the high nibbles
 //                                                of its bytes, IQ2_S in its low and its high 16 bits (nibble j = value j)
 //   SC  off 4096: [lane][4 B or 8 B]             scale nibbles as in the compact tile

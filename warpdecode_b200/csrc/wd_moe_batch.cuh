@@ -19,10 +19,10 @@
 // Arithmetic is the single-token kernel's (same decoders, same quantisers, same router), so every token's ids,
 // weights and output are bit-identical to a single-token call. Single GPU, every expert resident.
 //
-// Bound: the chain activations -> row tasks -> picks -> tiles -> activations -> down tiles -> combine, and with four tokens
-// instruction issue in the tile decoder. Measured per call at the 48-layer model's block, compact tiles -> wide tiles -> picks
-// that travel before their proof -> nothing left for the launch's end: one token 30.5 -> 25 -> 24 -> 22.5 us, four tokens
-// 43 -> 35 -> 34 -> 32.6 us.
+// Bound: the chain activations -> row tasks -> picks -> tiles -> activations -> down tiles -> combine, run once per launch by code that
+// is fetched cold; with four tokens the tile walk is 15 of 27 us, the issue slots 37 % busy over the launch. Measured per call at the 48-layer model's
+// block, compact tiles -> wide tiles -> picks that travel before their proof -> nothing left for the launch's end -> gathers behind
+// their tiles: one token 30.5 -> 25 -> 24 -> 22.5 -> 21.7 us, four tokens 43 -> 35 -> 34 -> 32.6 -> 32.9 us.
 #pragma once
 
 #include "wd_moe_kernel.cuh"
