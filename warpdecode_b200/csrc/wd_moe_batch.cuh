@@ -102,6 +102,7 @@ __host__ __device__ inline int batch_run_pairs(int K, int t3, int wcta) {
 __host__ __device__ inline void batch_lay_out(const BatchList &L, int T, int K, int t2_log2, int t3_log2, int nsb_f, int cta, int wcta) {
     const int u_tok = K << t2_log2, v_tok = K << t3_log2;       // gate/up units and down tiles of one token
     int c2[kMaxTokens], c3[kMaxTokens];
+#pragma unroll 1
     for (int t = 0; t < T; ++t) {
         int ct = cta + t * (wcta / kMaxTokens);
         if (ct >= wcta) ct -= wcta;
@@ -124,6 +125,7 @@ __host__ __device__ inline void batch_lay_out(const BatchList &L, int T, int K, 
     };
     add(0, 0);
     if (T > 1) add(1, 0);
+#pragma unroll 1
     for (int t = 0; t < T; ++t) {
         if (t + 2 < T) add(t + 2, 0);
         add(t, 1);
@@ -142,6 +144,7 @@ __host__ __device__ inline void batch_lay_out(const BatchList &L, int T, int K, 
 __host__ __device__ inline uint32_t batch_task(const BatchList &L, int i, int T, int K, int t2_log2, int t3_log2, int nsb_f, int act_per_tok, int wcta,
                                                int &aux) {
     int k = 0;
+#pragma unroll 1
     while (k + 1 < 2 * T && i >= L.begin[k + 1]) ++k;
     const int t = L.info[k] >> 1, down = L.info[k] & 1, li = i - L.begin[k];
     uint32_t d;
@@ -155,6 +158,7 @@ __host__ __device__ inline uint32_t batch_task(const BatchList &L, int i, int T,
         d = 1u | static_cast<uint32_t>(t << 1) | static_cast<uint32_t>((t * K + pl) << 3) | static_cast<uint32_t>((v & ((1 << t3_log2) - 1)) << 9);
         aux = t * act_per_tok + (pl - L.jl0[t]) * nsb_f;
     }
+#pragma unroll 1
     for (int kd = 0; kd < 2 * T; ++kd) {
         if (!(L.info[kd] & 1)) continue;
         const int td = L.info[kd] >> 1;
