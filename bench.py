@@ -45,9 +45,9 @@ EXPERT_BYTES = 3 * 450560
 REPLICATED_BYTES = 3 * 1114112 + 8192 + 1114112                      # shared expert + gate vector + router
 LAYER_BYTES = 10 * EXPERT_BYTES + REPLICATED_BYTES
 HEAD_BYTES = VOCAB * (CFG["hidden"] // 32) * 34
-# dram__bytes_read + dram__bytes_write of the layer kernel per layer, from an ncu capture of a two-layer
-# launch of the same shape; every layer reads its own weights once, so a launch of n layers moves n times this.
-TRAFFIC_PER_LAYER = 21_045_000
+# dram__bytes_read of the layer kernel per layer, from ncu captures of a two-layer launch of the same shape (wide tiles,
+# and the compact tiles of a capped cache); every layer reads its own weights once, so a launch of n layers moves n times this.
+TRAFFIC_PER_LAYER, TRAFFIC_PER_LAYER_COMPACT = 21_040_000, 18_090_000
 METRIC = "batch-1 decode tok/s (48L 512-expert IQ3_S MoE)"
 WORKLOAD = ("cfg2/cfg3 MoE stack: 48 layers x (router top-10 of 512 IQ3_S experts + Q8_0 shared expert), "
             "hidden 2048, all experts resident, router bias N(0,1) at every N; per token x=RMSNorm(residual), "
@@ -515,7 +515,7 @@ def run_ours(args, rank, world, local_rank):
                 "d2h_bytes_per_step": H * 4},
         "gpu_launches": launches,
         "roofline": {"bound": "hbm", "kernel": eng.kernel_name(), "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": TRAFFIC_PER_LAYER * args.layers if world == 1 else None,
+                     "frac": achieved / peak, "traffic": (TRAFFIC_PER_LAYER if eng.slot_bytes() > EXPERT_BYTES else TRAFFIC_PER_LAYER_COMPACT) * args.layers if world == 1 else None,
                      "peak_source": "measured" if peaks else "fallback",
                      "bytes_per_launch": token_bytes, "us_per_launch": launch_s * 1e6,
                      "us_per_layer": launch_s * 1e6 / args.layers,
