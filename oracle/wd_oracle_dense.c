@@ -277,7 +277,7 @@ static void attention_head(const float *q, const float *kc, const float *vc, siz
 int wdo_dense_step(const wdo_dense_model *m, float *kcache, float *vcache, int token, int pos, float *logits_out) {
     const int H = m->hidden, hd = m->head_dim, nh = m->n_heads, nkv = m->n_kv_heads, F = m->ffn, V = m->vocab;
     const int qdim = nh * hd, kvdim = nkv * hd, qkv_rows = qdim + 2 * kvdim;
-    const int maxn = H > F ? H : F;
+    const int maxn = (H > F ? H : F) > qdim ? (H > F ? H : F) : qdim;
     float *hidden = (float *)malloc(sizeof(float) * H);
     float *norm = (float *)malloc(sizeof(float) * maxn);
     float *qkv = (float *)malloc(sizeof(float) * qkv_rows);

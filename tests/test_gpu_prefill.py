@@ -167,3 +167,9 @@ def test_a_decoder_without_room_for_the_prompt_workspace(wd):
         del hog
         gc.collect()
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("H,nh,nkv,hd,F", [(256, 16, 4, 128, 320), (512, 9, 3, 96, 32)])
+def test_more_head_elements_than_hidden_or_ffn(wd, oracle, H, nh, nkv, hd, F):
+    """The output product's input is the longest row of the model."""
+    test_prompt_pass_equals_the_one_token_steps(wd, oracle, H, nh, nkv, hd, F, 2, 19, 6, "file")
