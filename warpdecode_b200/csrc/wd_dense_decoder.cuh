@@ -860,17 +860,25 @@ __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_ker
 // End of a step: the arg-max key becomes the next token (0 when no logit was finite), is recorded at out[pos + 1],
 // the position advances, the key is cleared for the next step (dense_argmax_finish_kernel + increment_pos_kernel).
 // `forced` (nullable): forced[pos + 1] >= 0 replaces the generated token (prompt tokens).
-__global__ void dense_finish_kernel(unsigned long long *key, int *token, int *pos, int *out, const int *forced) {
+// The next token's attention reads the position in front of its wait, so its store is followed by a fence; a second warp does that beside the
+// token's own chain (in the same thread it costs 0.6 us per token, 1.2 % of a four-layer model's).
+constexpr int kFinishThreads = 64;
+__global__ void __launch_bounds__(kFinishThreads) dense_finish_kernel(unsigned long long *key, int *token, int *pos, int *out, const int *forced) {
     grid_dep_wait();
-    const unsigned long long k = *key;
-    int t = k == 0ull ? 0 : static_cast<int>(0xffffffffu - static_cast<unsigned>(k & 0xffffffffull));
     const int p = *pos + 1;
-    if (forced != nullptr && forced[p] >= 0) t = forced[p];
-    out[p] = t;
-    *token = t;
-    *pos = p;
-    *key = 0ull;
-    __threadfence();        // the next token's attention reads the position in front of its wait
+    __syncthreads();            // both warps have the old position
+    if (threadIdx.x == 32) {
+        *pos = p;
+        __threadfence();
+    }
+    if (threadIdx.x == 0) {
+        const unsigned long long k = *key;
+        int t = k == 0ull ? 0 : static_cast<int>(0xffffffffu - static_cast<unsigned>(k & 0xffffffffull));
+        if (forced != nullptr && forced[p] >= 0) t = forced[p];
+        out[p] = t;
+        *token = t;
+        *key = 0ull;
+    }
 }
 
 }  // namespace wd
