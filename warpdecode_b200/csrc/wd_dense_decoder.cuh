@@ -83,11 +83,14 @@ struct PairedQuant {
 };
 __device__ __forceinline__ int paired_place(int v) { return ((v >> 2) & 3) * 8 + (v >> 4) * 4 + (v & 3); }
 __device__ __forceinline__ void store_quant(int8_t *out, int e, int q) { out[e] = static_cast<int8_t>(q); }
-__device__ __forceinline__ void store_quant(PairedQuant *out, int e, int q) { out[(e & ~31) + paired_place(e & 31)].v = static_cast<int8_t>(q); }
+struct QuantAt {        // four neighbouring quants
+    uint8_t *quad;
+};
+__device__ __forceinline__ void store_quant(const QuantAt &out, int e, int q) { out.quad[e & 3] = static_cast<uint8_t>(q); }
 
 // Q8_0 of 32 floats held one per lane: quant byte and the f16-rounded scale (ggml's rule, as quantize_q8_0_cta).
 template <class Quant>
-__device__ __forceinline__ void q8_0_block_warp(float v, int lane, Quant *q_out, float *d_out) {
+__device__ __forceinline__ void q8_0_block_warp(float v, int lane, Quant q_out, float *d_out) {
     float amax = fabsf(v);
 #pragma unroll
     for (int s = 16; s >= 1; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
@@ -98,11 +101,6 @@ __device__ __forceinline__ void q8_0_block_warp(float v, int lane, Quant *q_out,
     }
     store_quant(q_out, lane, q);
     if (lane == 0) *d_out = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
-}
-
-// Four quants of one thread (values e .. e + 3, e a multiple of four) with one store.
-__device__ __forceinline__ void store_quant4(PairedQuant *out, int e, uint32_t packed) {
-    *reinterpret_cast<uint32_t *>(out + (e & ~31) + paired_place(e & 31)) = packed;
 }
 
 // hidden_out = hidden + proj (proj: when given; hidden_out: when given); y = RMSNorm(that) * w -> Q8_0 (int8 [n], float scale per

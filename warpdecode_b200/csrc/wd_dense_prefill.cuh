@@ -12,24 +12,45 @@ namespace wd {
 
 constexpr int kPrefillChunk = 512;      // tokens per pass at most (workspace: about 100 KB per token at ffn 8192)
 
+// The quantised activations [token][n] of a chunk, in one of two orders. tile = 0: rows of PairedQuant, scales [token][n / 32]
+// (prefill_gemm_kernel). tile > 0: the B operand of prompt_tc_gemm_kernel: per `tile` tokens and block (in entry order: block 32 t + l at
+// bitrev(l) * n_t + t) a record of 8-token x 16-byte matrices, the first half of the block and then the second, and the tokens' scales.
+struct PromptAct {
+    uint8_t *q;
+    float *d;
+    int n, tile;
+    __device__ __forceinline__ uint8_t *record(int m, int b) const {
+        const int n_t = (n + 1023) >> 10, e = static_cast<int>(__brev(static_cast<unsigned>(b) & 31u) >> 27) * n_t + (b >> 5);
+        return q + (static_cast<size_t>(m / tile) * 32 * n_t + e) * (tile * 36);
+    }
+    // where value e (a multiple of four) of token m goes, with the three behind it
+    __device__ __forceinline__ uint8_t *quad(int m, int e) const {
+        if (tile == 0) return q + static_cast<size_t>(m) * n + (e & ~31) + paired_place(e & 31);
+        const int c = m % tile;
+        return record(m, e >> 5) + (e >> 4 & 1) * (tile * 16) + (c >> 3) * 128 + (c & 7) * 16 + (e & 15);
+    }
+    __device__ __forceinline__ float *scale(int m, int b) const {
+        if (tile == 0) return d + static_cast<size_t>(m) * (n >> 5) + b;
+        return reinterpret_cast<float *>(record(m, b) + tile * 32) + m % tile;
+    }
+};
+
 // RMSNorm + Q8_0 of every token of the chunk, one CTA per token; the body is the one-token kernel's.
 __global__ void __launch_bounds__(1024) prefill_norm_quant_kernel(float *hidden, const float *proj, const float *w, int n, float eps,
-                                                                 PairedQuant *xq, float *xd, const uint8_t *embd, const int *tokens, int vocab,
+                                                                 PromptAct x, const uint8_t *embd, const int *tokens, int vocab,
                                                                  int embd_q8) {
     grid_dep_launch();
     const size_t m = blockIdx.x;
     float *h = hidden + m * n;
     const NormInput in = {h, proj != nullptr ? proj + m * n : nullptr, w, embd != nullptr || proj != nullptr ? h : nullptr, embd, tokens + m, eps,
                           n, vocab, embd_q8};
-    xq += m * n;
-    xd += m * (n >> 5);
     dense_norm_quant_body<1>(in, [] { grid_dep_wait(); }, [&](int e, uint32_t packed, float d) {
-        store_quant4(xq, e, packed);
-        if ((e & 31) == 0) xd[e >> 5] = d;
+        *reinterpret_cast<uint32_t *>(x.quad(blockIdx.x, e)) = packed;
+        if ((e & 31) == 0) *x.scale(blockIdx.x, e >> 5) = d;
     });
 }
 
-// ---- Y[m][row] = W[row] . X[m] for the tokens of a chunk ---------------------------------------------------------------
+// ---- Y[m][row] = W[row] . X[m] for the tokens of a chunk: short prompts, short rows (the others: wd_dense_prompt_tc.cuh) ----
 // The one-token order is: lane l of 32 runs one fmaf(d_w * d_x, (float)int_dot, acc) per block b = l, l + 32, ... ascending,
 // then the butterfly ^16 ^8 ^4 ^2 ^1. The integer dot of one block is a contraction of depth 32, i.e. exactly one
 // mma.m16n8k32 (s8) for 16 rows x 8 tokens; it cannot be accumulated over blocks, because every block is scaled by its own
@@ -384,7 +405,7 @@ constexpr int kPrefillAttnThreads = 288;    // eight warps on scores and values,
 template <int HD, int QT>
 __global__ void __launch_bounds__(kPrefillAttnThreads, HD <= 64 ? 2 : 1) prefill_attention_kernel(const float *qrot, const float *kcache, const float *vcache,
                                                                               int pos0, int m_tokens, int heads, int kv_heads,
-                                                                              float inv_sqrt, PairedQuant *oq, float *od) {
+                                                                              float inv_sqrt, PromptAct o) {
     extern __shared__ __align__(16) float asm_[];
     __shared__ float mx[QT], lsum[QT], part[QT * 16];
     grid_dep_launch();
@@ -501,14 +522,17 @@ __global__ void __launch_bounds__(kPrefillAttnThreads, HD <= 64 ? 2 : 1) prefill
     }
     __syncthreads();
     for (int b = warp; b < n_tok * (HD / 32); b += kPrefillAttnThreads / 32) {
-        const int r = b / (HD / 32), k = b - r * (HD / 32);
-        const size_t blk = (static_cast<size_t>(tok0 + r) * heads + h) * (HD / 32) + k;
-        q8_0_block_warp(qs[r * HD + k * 32 + lane], lane, oq + blk * 32, od + blk);
+        const int r = b / (HD / 32), k = b - r * (HD / 32), blk = h * (HD / 32) + k;
+        q8_0_block_warp(qs[r * HD + k * 32 + lane], lane, QuantAt{o.quad(tok0 + r, blk * 32 + (lane & ~3))}, o.scale(tok0 + r, blk));
+    }
+    if (o.tile > 0 && h == heads - 1) {         // as in prefill_swiglu_quant_kernel
+        const int nb = o.n >> 5, gap = ((nb + 31) & ~31) - nb;
+        for (int i = tid; i < n_tok * gap; i += kPrefillAttnThreads) *o.scale(tok0 + i / gap, nb + i % gap) = 0.0f;
     }
 }
 
 // act = SiLU(g) * u of every token, -> Q8_0; a thread takes four values, eight neighbouring lanes a block of 32.
-__global__ void __launch_bounds__(256) prefill_swiglu_quant_kernel(const float *gate_up, int n, PairedQuant *xq, float *xd) {
+__global__ void __launch_bounds__(256) prefill_swiglu_quant_kernel(const float *gate_up, int n, PromptAct x) {
     grid_dep_launch();
     grid_dep_wait();
     const size_t m = blockIdx.y;
@@ -527,7 +551,10 @@ __global__ void __launch_bounds__(256) prefill_swiglu_quant_kernel(const float *
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-    if (!live) return;
+    if (!live) {        // blocks behind the end of a row: prompt_tc_gemm_kernel multiplies them by a scale of zero
+        if (x.tile > 0 && (ch & 7) == 0) *x.scale(blockIdx.y, ch >> 3) = 0.0f;
+        return;
+    }
     int q[4] = {0, 0, 0, 0};
     if (amax != 0.0f) {
         const float inv = __fdiv_rn(127.0f, amax);
@@ -535,8 +562,8 @@ __global__ void __launch_bounds__(256) prefill_swiglu_quant_kernel(const float *
         for (int j = 0; j < 4; ++j) q[j] = max(-128, min(127, __float2int_rn(__fmul_rn(v[j], inv))));
     }
     const uint32_t packed = (q[0] & 0xff) | ((q[1] & 0xff) << 8) | ((q[2] & 0xff) << 16) | (static_cast<uint32_t>(q[3]) << 24);
-    *reinterpret_cast<uint32_t *>(xq + m * n + (4 * ch & ~31) + paired_place(4 * ch & 31)) = packed;
-    if ((ch & 7) == 0) xd[m * (n >> 5) + (ch >> 3)] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
+    *reinterpret_cast<uint32_t *>(x.quad(blockIdx.y, 4 * ch)) = packed;
+    if ((ch & 7) == 0) *x.scale(blockIdx.y, ch >> 3) = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
 }
 
 }  // namespace wd

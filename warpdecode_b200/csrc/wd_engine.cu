@@ -25,6 +25,7 @@
 #include "wd_dense_decoder.cuh"
 #include "wd_dense_token.cuh"
 #include "wd_dense_prefill.cuh"
+#include "wd_dense_prompt_tc.cuh"
 #include "wd_plain_moe.cuh"
 #include "wd_plain_wide.cuh"
 #include "wd_grids.h"
