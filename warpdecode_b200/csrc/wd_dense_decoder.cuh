@@ -410,38 +410,135 @@ __device__ __forceinline__ float dense_attention_core(const float *qs, const flo
     return 0.0f;
 }
 
-// The dot q . k of the one-token order - lane l runs fmaf over d = l, l + 32, ..., then the butterfly - by ONE thread, four
-// lanes at a time: quads of lanes meet in the butterfly's own pairs (16 apart, 8 apart, 4, 2, 1), so nothing is shuffled.
-template <int HD>
-__device__ __forceinline__ float lane_order_dot(const float *q, const float *k) {
-    auto quad = [&](int b, float (&a)[4]) {         // lanes 4 b .. 4 b + 3
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = 0.0f;
+// Two floats per instruction (each half rounded like the scalar operation).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// The dot q . k of the one-token order - lane l runs fmaf over d = l, l + 32, ..., then the butterfly - by ONE thread, two
+// lanes per instruction: quads of lanes meet in the butterfly's own pairs (16 apart, 8 apart, 4, 2, 1), so nothing is shuffled.
+// key(e): elements 4 e .. 4 e + 3 of the key.
+template <int HD, class Key>
+__device__ __forceinline__ float lane_order_dot(const float *q, Key key) {
+    auto quad = [&](int b, f32x2 (&a)[2]) {         // lanes 4 b .. 4 b + 3
+        a[0] = a[1] = 0ull;
 #pragma unroll
         for (int r = 0; r < HD / 32; ++r) {
-            const float4 qv = *reinterpret_cast<const float4 *>(q + r * 32 + b * 4);
-            const float4 kv = *reinterpret_cast<const float4 *>(k + r * 32 + b * 4);
-            a[0] = __fmaf_rn(qv.x, kv.x, a[0]);
-            a[1] = __fmaf_rn(qv.y, kv.y, a[1]);
-            a[2] = __fmaf_rn(qv.z, kv.z, a[2]);
-            a[3] = __fmaf_rn(qv.w, kv.w, a[3]);
+            const ulonglong2 qv = *reinterpret_cast<const ulonglong2 *>(q + r * 32 + b * 4), kv = key(r * 8 + b);
+            a[0] = fma2(qv.x, kv.x, a[0]);
+            a[1] = fma2(qv.y, kv.y, a[1]);
         }
     };
-    float s8[2][4];
+    f32x2 s8[2][2];
 #pragma unroll
     for (int p = 0; p < 2; ++p) {                   // lanes 4 p .. 4 p + 3 with those 16, 8 and 24 above
-        float a[4], b[4], c[4], d[4];
+        f32x2 a[2], b[2], c[2], d[2];
         quad(p, a);
         quad(p + 4, b);
         quad(p + 2, c);
         quad(p + 6, d);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) s8[p][i] = __fadd_rn(__fadd_rn(a[i], b[i]), __fadd_rn(c[i], d[i]));
+        for (int i = 0; i < 2; ++i) s8[p][i] = add2(add2(a[i], b[i]), add2(c[i], d[i]));
     }
-    float s4[4];
+    float e0, e1;
+    unpack2(add2(add2(s8[0][0], s8[1][0]), add2(s8[0][1], s8[1][1])), e0, e1);      // lanes (0, 1) + (2, 3)
+    return __fadd_rn(e0, e1);
+}
+// Maximum over the lanes of a warp (no NaN among them).
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Loads from shared memory, at a window address plus a constant, that keep their place among others of their kind.
+template <int OFF>
+__device__ __forceinline__ float lds_here(uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1 + %2];" : "=f"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+template <int OFF>
+__device__ __forceinline__ float4 lds4_here(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4 + %5];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a), "n"(OFF));
+    return v;
+}
+// The attention's sums over positions, one element per thread: l += p[t], acc = fmaf(p[t], v[t], acc), t ascending. p at p_at, v every ROW
+// bytes from v_at on. A step is two dependent instructions of 4.7 cycles, but a shared-memory load takes a warp's issue for about five, and the
+// compiler does not keep loads ahead of the chain by itself: eight steps run between the loads of the next eight (7 cycles a step, before 12).
+struct WeightedEight {
+    float4 w[2];
+    float x[8];
+};
+template <int ROW, int I>
+__device__ __forceinline__ void weighted_load(WeightedEight &b, uint32_t p_at, uint32_t v_at) {
+    if constexpr (I % 4 == 0) b.w[I / 4] = lds4_here<I * 4>(p_at);
+    b.x[I] = lds_here<I * ROW>(v_at);
+}
+template <int ROW, int I = 0>
+__device__ __forceinline__ void weighted_load_all(WeightedEight &b, uint32_t p_at, uint32_t v_at) {
+    weighted_load<ROW, I>(b, p_at, v_at);
+    if constexpr (I < 7) weighted_load_all<ROW, I + 1>(b, p_at, v_at);
+}
+__device__ __forceinline__ void weighted_step(float &l, float &acc, float w, float x) {       // in place among the loads
+    asm volatile("add.rn.f32 %0, %0, %1;" : "+f"(l) : "f"(w));
+    asm volatile("fma.rn.f32 %0, %1, %2, %0;" : "+f"(acc) : "f"(w), "f"(x));
+}
+template <int ROW, int I = 0>
+__device__ __forceinline__ void weighted_eight(float &l, float &acc, const WeightedEight &now, WeightedEight &next, uint32_t p_at, uint32_t v_at) {
+    weighted_load<ROW, I>(next, p_at, v_at);
+    const float4 &w = now.w[I / 4];
+    weighted_step(l, acc, I % 4 == 0 ? w.x : I % 4 == 1 ? w.y : I % 4 == 2 ? w.z : w.w, now.x[I]);
+    if constexpr (I < 7) weighted_eight<ROW, I + 1>(l, acc, now, next, p_at, v_at);
+}
+template <int ROW>
+__device__ __forceinline__ void weighted_sum(float &l, float &acc, const float *p, const float *v, int n) {
+    const uint32_t p0 = smem_u32(p), v0 = smem_u32(v);
+    const int eights = n >> 3;
+    if (eights > 0) {
+        WeightedEight a, b;
+        weighted_load_all<ROW>(a, p0, v0);
+        int k = 0;
+        auto at = [&](int i) { return i < eights ? i : 0; };      // past the end: loads that nobody uses, of what is there
+#pragma unroll 1
+        for (; k + 2 <= eights; k += 2) {
+            weighted_eight<ROW>(l, acc, a, b, p0 + (k + 1) * 32, v0 + (k + 1) * (8 * ROW));
+            weighted_eight<ROW>(l, acc, b, a, p0 + at(k + 2) * 32, v0 + at(k + 2) * (8 * ROW));
+        }
+        if (k < eights) weighted_eight<ROW>(l, acc, a, b, p0, v0);
+    }
+    const int r = eights * 8;
+    if (r < n) {            // fewer than eight are left: requested together
+        float w[7], x[7];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) s4[i] = __fadd_rn(s8[0][i], s8[1][i]);
-    return __fadd_rn(__fadd_rn(s4[0], s4[2]), __fadd_rn(s4[1], s4[3]));
+        for (int i = 0; i < 7; ++i) {
+            w[i] = lds_here<0>(p0 + min(r + i, n - 1) * 4);
+            x[i] = lds_here<0>(v0 + min(r + i, n - 1) * ROW);
+        }
+#pragma unroll
+        for (int i = 0; i < 7; ++i)
+            if (r + i < n) weighted_step(l, acc, w[i], x[i]);
+    }
 }
 
 // Asynchronous 16-byte copy global -> shared; !live fills the destination with zeros.
@@ -498,8 +595,8 @@ struct DecodeAttn {
 // keys and values must be there when they are needed: the cache below pos was written by earlier tokens, and the first
 // chunks of it (all of it up to 320 positions of 64) are copied to shared memory in a ring, keys before values,
 // requested BEFORE the wait for the QKV product; a score is one thread's work, without shuffles.
-// Measured per layer inside the step of the 16-layer model (32 heads of 64), before -> now: 6.6 -> 2.1 us at 72 positions; at 500
-// positions 74 -> 7.7 us (8.6 us by one CTA per head).
+// Measured per layer inside the step of the 16-layer model (32 heads of 64), from the end of the kernel in front: 2.2 us at 77 positions (2.8
+// before the sums' loads ran ahead of their chains), 4.6 us at 485 (5.2), of which the sums 2.3; by one CTA per head 0.9 us more there.
 //
 // C: CTAs per head, a cluster. One CTA takes in 512 bytes per position through its SM, and once a context is longer than its
 // ring holds, the last values only follow when the first keys have been scored. With C = HD / 32 each CTA scores every C-th
@@ -526,11 +623,12 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
     grid_dep_launch();
     if constexpr (C > 1) cluster_arrive();          // answered before the first store into a peer
     const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0;
-    const int h = blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     // The position comes from the finish kernel of the token before. That kernel has ended (it releases nothing early), but this is in
     // front of the wait, so its store is ordered by the fence behind it and read past L1.
     int pos;
     asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(pos) : "l"(pos_ptr) : "memory");
+    pos = __shfl_sync(0xffffffffu, pos, 0);         // the same in every lane, and known to be
     const int kv_dim = kv_heads * HD, kvh = (h * kv_heads) / heads;
     float *kc = kcache + static_cast<size_t>(kvh) * HD, *vc = vcache + static_cast<size_t>(kvh) * HD;
     // positions 0 .. pos - 1: this CTA's key chunks (every C-th), then all value chunks of its slice
@@ -636,6 +734,7 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
     }
     __syncthreads();
     if constexpr (C > 1) cluster_wait();        // the peers run
+    auto key_row = [](const float *k) { return [k](int e) { return *reinterpret_cast<const ulonglong2 *>(k + 4 * e); }; };
     float m = -INFINITY;
     const int batch = min(kNt / kChunk, slots);         // key chunks scored side by side, one position per thread
 #pragma unroll 1
@@ -648,7 +747,7 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
         if ((tid < batch * kChunk && c < n_chunks && t < pos) || newest) {
             // the last thread scores the new position, and an old one too when it has one
             if (!newest || (tid < batch * kChunk && t < pos)) {
-                const float v = __fmul_rn(lane_order_dot<HD>(qs, slot_of(c) + (tid & (kChunk - 1)) * kRow), inv_sqrt);
+                const float v = __fmul_rn(lane_order_dot<HD>(qs, key_row(slot_of(c) + (tid & (kChunk - 1)) * kRow)), inv_sqrt);
                 sc[t] = v;
                 if constexpr (C > 1) {
 #pragma unroll
@@ -657,7 +756,7 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
                 m = v > m ? v : m;          // a NaN score never becomes the maximum
             }
             if (newest) {
-                const float v = __fmul_rn(lane_order_dot<HD>(qs, kn), inv_sqrt);
+                const float v = __fmul_rn(lane_order_dot<HD>(qs, key_row(kn)), inv_sqrt);
                 sc[pos] = v;
                 m = v > m ? v : m;
             }
@@ -673,45 +772,20 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
         cluster_wait();
         for (int t = tid; t <= pos; t += kNt) m = sc[t] > m ? sc[t] : m;
     }
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+    m = warp_max(m);
     if (lane == 0) wmax[warp] = m;
     __syncthreads();
-    m = wmax[lane & (kNt / 32 - 1)];
-#pragma unroll
-    for (int s = kNt / 64; s >= 1; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+    m = warp_max(wmax[lane & (kNt / 32 - 1)]);
     for (int t = tid; t <= pos; t += kNt) sc[t] = exp_ggml(__fadd_rn(sc[t], -m));
     cp_async_wait<0>();
     __syncthreads();
     float l = 0.0f, acc = 0.0f;
+    const bool whole = n_items <= slots;        // everything is in the ring, and the value rows lie in a row: a slot is exactly its rows
+    static_assert(A::kSlot == kChunkV * kRowV, "a slot of values ends where the next begins");
 #pragma unroll 1
-    for (int c = 0; c < n_vchunks; ++c) {
-        if (tid < kSlice) {
-            const float *v = slot_of(n_chunks + c) + tid, *p = sc + c * kChunkV;
-            const int n = min(kChunkV, pos - c * kChunkV);
-            // the two chains advance four cycles a step; a whole chunk's weights and values are requested well ahead of them
-            int r = 0;
-            for (; r + 32 <= n; r += 32) {
-                float4 p4[8];
-                float x[32];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) p4[i] = *reinterpret_cast<const float4 *>(p + r + 4 * i);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) x[i] = v[(r + i) * kRowV];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    l = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(l, p4[i].x), p4[i].y), p4[i].z), p4[i].w);
-                    acc = __fmaf_rn(p4[i].x, x[4 * i], acc);
-                    acc = __fmaf_rn(p4[i].y, x[4 * i + 1], acc);
-                    acc = __fmaf_rn(p4[i].z, x[4 * i + 2], acc);
-                    acc = __fmaf_rn(p4[i].w, x[4 * i + 3], acc);
-                }
-            }
-            for (; r < n; ++r) {
-                l = __fadd_rn(l, p[r]);
-                acc = __fmaf_rn(p[r], v[r * kRowV], acc);
-            }
-        }
+    for (int c = 0; c < (whole ? 1 : n_vchunks); ++c) {
+        if (warp < kSlice / 32)
+            weighted_sum<kRowV * 4>(l, acc, sc + c * kChunkV, slot_of(n_chunks + c) + tid, whole ? pos : min(kChunkV, pos - c * kChunkV));
         if (n_vchunks > slots) {     // longer than the ring: refill the slot
             __syncthreads();
             request(n_chunks + c + slots);

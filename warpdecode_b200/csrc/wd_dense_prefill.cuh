@@ -69,30 +69,6 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src, bool live)
     const int bytes = live ? 4 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
-// Two floats per instruction (each half rounded like the scalar operation).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // The integer accumulator starts at the bit pattern of 12582912.0f = 1.5 * 2^23: for |sum| < 2^22 the result read as a float
 // is 12582912 + sum, and one exact subtraction gives (float)sum. Sums here stay below 2^20.
 constexpr int kMagicBits = 0x4b400000;
@@ -368,34 +344,6 @@ __global__ void __launch_bounds__(32 * kRopeWarps) prefill_rope_kernel(const flo
 }
 
 // ---- attention of the chunk ----------------------------------------------------------------------------------------------
-// lane_order_dot with two lanes per instruction
-template <int HD>
-__device__ __forceinline__ float lane_order_dot2(const float *q, const ulonglong2 (&k)[HD / 4]) {
-    auto quad = [&](int b, f32x2 (&a)[2]) {         // lanes 4 b .. 4 b + 3
-        a[0] = a[1] = 0ull;
-#pragma unroll
-        for (int r = 0; r < HD / 32; ++r) {
-            const ulonglong2 qv = *reinterpret_cast<const ulonglong2 *>(q + r * 32 + b * 4);
-            a[0] = fma2(qv.x, k[r * 8 + b].x, a[0]);
-            a[1] = fma2(qv.y, k[r * 8 + b].y, a[1]);
-        }
-    };
-    f32x2 s8[2][2];
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        f32x2 a[2], b[2], c[2], d[2];
-        quad(p, a);
-        quad(p + 4, b);
-        quad(p + 2, c);
-        quad(p + 6, d);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) s8[p][i] = add2(add2(a[i], b[i]), add2(c[i], d[i]));
-    }
-    float e0, e1;
-    unpack2(add2(add2(s8[0][0], s8[1][0]), add2(s8[0][1], s8[1][1])), e0, e1);      // lanes (0, 1) + (2, 3)
-    return __fadd_rn(e0, e1);
-}
-
 constexpr int kPrefillAttnThreads = 288;    // eight warps on scores and values, one on the sums of the weights
 
 // One CTA per (head, QT consecutive tokens). Scores, weights and the sums over positions keep the one-token order: maximum,
@@ -431,8 +379,8 @@ __global__ void __launch_bounds__(kPrefillAttnThreads, HD <= 64 ? 2 : 1) prefill
         for (int e = 0; e < HD / 4; ++e) k[e] = *reinterpret_cast<const ulonglong2 *>(kc + static_cast<size_t>(t) * kv_dim + e * 4);
 #pragma unroll 1
         for (int r = gidx * rows; r < (gidx + 1) * rows; r += 2) {
-            const float a = __fmul_rn(lane_order_dot2<HD>(qs + r * HD, k), inv_sqrt);
-            const float b = __fmul_rn(lane_order_dot2<HD>(qs + (r + 1) * HD, k), inv_sqrt);
+            const float a = __fmul_rn(lane_order_dot<HD>(qs + r * HD, [&](int e) { return k[e]; }), inv_sqrt);
+            const float b = __fmul_rn(lane_order_dot<HD>(qs + (r + 1) * HD, [&](int e) { return k[e]; }), inv_sqrt);
             *reinterpret_cast<float2 *>(sc + static_cast<size_t>(t) * QT + r) = make_float2(a, b);
         }
     }
