@@ -372,10 +372,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_layer_kernel(const __grid_con
         for (int w = 1; w < kWarps; w <<= 1)
 #pragma unroll
             for (int i = 0; i + w < kWarps; i += 2 * w) tot[i] = __dadd_rn(tot[i], tot[i + w]);
-        const float scale = __double2float_rn(
-            __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(P.inv_h != 0.0 ? __dmul_rn(tot[0], P.inv_h)
-                                                               : __ddiv_rn(tot[0], static_cast<double>(P.H)),
-                                                static_cast<double>(P.eps)))));
+        const float scale = inv_sqrt_to_float(__dadd_rn(P.inv_h != 0.0 ? __dmul_rn(tot[0], P.inv_h) : __ddiv_rn(tot[0], static_cast<double>(P.H)),
+                                                        static_cast<double>(P.eps)));
         if (mine) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
