@@ -158,15 +158,16 @@ __host__ __device__ inline uint32_t batch_task(const BatchList &L, int i, int T,
         d = 1u | static_cast<uint32_t>(t << 1) | static_cast<uint32_t>((t * K + pl) << 3) | static_cast<uint32_t>((v & ((1 << t3_log2) - 1)) << 9);
         aux = t * act_per_tok + (pl - L.jl0[t]) * nsb_f;
     }
+    int taken = 0;          // one gather per task: where segments are shorter than a round, a token's gathers come behind the token's before it
 #pragma unroll 1
     for (int kd = 0; kd < 2 * T; ++kd) {
         if (!(L.info[kd] & 1)) continue;
         const int td = L.info[kd] >> 1;
         int base = L.begin[kd] - kWarps - L.ng[td];
         if (base < L.gu_end[td] - kWarps) base = L.gu_end[td] - kWarps;
-        if (base < 0) base = 0;
-        // at most one per task (short segments overlap)
-        if (i >= base && i < base + L.ng[td] && (d >> 22) == 0u) d |= static_cast<uint32_t>(td * act_per_tok + (i - base) + 1) << 22;
+        if (base < taken) base = taken;
+        taken = base + L.ng[td];
+        if (i >= base && i < taken) d |= static_cast<uint32_t>(td * act_per_tok + (i - base) + 1) << 22;
     }
     return d;
 }
