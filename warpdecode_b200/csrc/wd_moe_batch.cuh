@@ -643,7 +643,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_batch_kernel(const __grid_con
             } else {
                 // the pair's activations: normally gathered a round ago; else the first warp to need a superblock does it
 #pragma unroll 1
-                for (int sk = 0; sk < P.nsb_f; ++sk) {
+                for (int k = 0; k < P.nsb_f; ++k) {
+                    const int sk = (k + i) & (P.nsb_f - 1);     // neighbouring tiles begin with different ones
                     if (!mbar_try_wait(&tbars[bar_act + aux + sk], 0)) {
                         gather(aux + sk);
                         mbar_wait(&tbars[bar_act + aux + sk], 0, err);
