@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(DecodeAttn<HD, C>::kThreads) dense_attention_k
 // ties go to the lowest row (dense_argmax_reduce_kernel, :1603-1632). Rows: R per warp, U blocks per lane and row in flight. Dynamic shared memory:
 // nb * 40 bytes.
 constexpr int kNormProductThreads = 512;
-template <bool Q8, int R, int U, int MODE, int PASSES>
+template <bool Q8, int R, int U, int MODE, int PASSES, bool AHEAD>
 __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_kernel(NormInput in, const uint8_t *wp, int rows, float *y,
                                                                                    unsigned long long *key, int8_t *oq, float *od) {
     static_assert(MODE != 1 || R == 4, "two gate rows and two up rows per warp");
@@ -839,8 +839,10 @@ __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_ker
         return (unit * kWarpsHere + warp) * R + r;
     };
     const int units = MODE == 1 ? rows >> 6 : (rows + kWarpsHere * R - 1) / (kWarpsHere * R);
-    RowBlock<Q8> w[R][U];
-    auto load = [&](int unit, int b0, bool early) {
+    // AHEAD: a long walk over rows asks for the next blocks before it multiplies the ones in hand (see dense_launch_norm_product)
+    static_assert(!AHEAD || U == 1, "one block per lane and row ahead");
+    RowBlock<Q8> w[R][U], next[AHEAD ? R : 1][U];
+    auto load = [&](RowBlock<Q8> (*to)[U], int unit, int b0, bool early) {
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -848,13 +850,13 @@ __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_ker
                 const int b = b0 + 32 * u, row = row_of(unit, r);
                 if (b < nb && (MODE == 1 || row < rows)) {
                     const size_t blk = static_cast<size_t>(row) * stride + b;
-                    if (early) w[r][u].load_early(q_all, d_all, blk);
-                    else w[r][u].load(q_all, d_all, blk);
+                    if (early) to[r][u].load_early(q_all, d_all, blk);
+                    else to[r][u].load(q_all, d_all, blk);
                 }
             }
     };
     int unit = blockIdx.x;
-    load(unit, lane, true);           // weights do not depend on the kernel before this one
+    load(w, unit, lane, true);           // weights do not depend on the kernel before this one
     dense_norm_quant_body<PASSES>(in, [] { grid_dep_wait(); }, [&](int e, uint32_t packed, float d) {
         const int b = e >> 5, j = e & 31;
         *reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>((j & 16) ? x.hi + b : x.lo + b) + (j & 15)) = packed;
@@ -871,7 +873,13 @@ __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_ker
         for (int r = 0; r < R; ++r) acc[r] = 0.0f;
 #pragma unroll 1
         for (int b0 = lane; b0 < nb; b0 += 32 * U) {
-            if (unit != static_cast<int>(blockIdx.x) || b0 != lane) load(unit, b0, false);
+            if constexpr (AHEAD) {
+                const bool wrap = b0 + 32 >= nb;
+                const int unit2 = wrap ? unit + static_cast<int>(gridDim.x) : unit;
+                if (unit2 < units) load(next, unit2, wrap ? lane : b0 + 32, true);
+            } else if (unit != static_cast<int>(blockIdx.x) || b0 != lane) {
+                load(w, unit, b0, false);
+            }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int b = b0 + 32 * u;
@@ -882,6 +890,10 @@ __global__ void __launch_bounds__(kNormProductThreads, 2) dense_norm_product_ker
                     for (int r = 0; r < R; ++r)
                         if (MODE == 1 || row_of(unit, r) < rows) acc[r] = w[r][u].term(lo, hi, d, acc[r]);
                 }
+            }
+            if constexpr (AHEAD) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) w[r][0] = next[r][0];
             }
         }
 #pragma unroll
