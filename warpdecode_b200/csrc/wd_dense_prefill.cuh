@@ -23,16 +23,14 @@ struct PromptAct {
         const int n_t = (n + 1023) >> 10, e = static_cast<int>(__brev(static_cast<unsigned>(b) & 31u) >> 27) * n_t + (b >> 5);
         return q + (static_cast<size_t>(m / tile) * 32 * n_t + e) * (tile * 36);
     }
-    // where value e (a multiple of four) of token m goes, with the three behind it
-    __device__ __forceinline__ uint8_t *quad(int m, int e) const {
-        if (tile == 0) return q + static_cast<size_t>(m) * n + (e & ~31) + paired_place(e & 31);
+    // where value e (a multiple of four) of token m goes, with the three behind it: in rows, in tiles
+    __device__ __forceinline__ uint8_t *row_quad(int m, int e) const { return q + m * n + (e & ~31) + paired_place(e & 31); }       // fewer than 2^31 bytes
+    __device__ __forceinline__ uint8_t *tile_quad(int m, int e) const {
         const int c = m % tile;
         return record(m, e >> 5) + (e >> 4 & 1) * (tile * 16) + (c >> 3) * 128 + (c & 7) * 16 + (e & 15);
     }
-    __device__ __forceinline__ float *scale(int m, int b) const {
-        if (tile == 0) return d + static_cast<size_t>(m) * (n >> 5) + b;
-        return reinterpret_cast<float *>(record(m, b) + tile * 32) + m % tile;
-    }
+    __device__ __forceinline__ float *row_scale(int m, int b) const { return d + m * (n >> 5) + b; }
+    __device__ __forceinline__ float *tile_scale(int m, int b) const { return reinterpret_cast<float *>(record(m, b) + tile * 32) + m % tile; }
 };
 
 // RMSNorm + Q8_0 of every token of the chunk, one CTA per token; the body is the one-token kernel's.
@@ -45,8 +43,8 @@ __global__ void __launch_bounds__(1024) prefill_norm_quant_kernel(float *hidden,
     const NormInput in = {h, proj != nullptr ? proj + m * n : nullptr, w, embd != nullptr || proj != nullptr ? h : nullptr, embd, tokens + m, eps,
                           n, vocab, embd_q8};
     dense_norm_quant_body<1>(in, [] { grid_dep_wait(); }, [&](int e, uint32_t packed, float d) {
-        *reinterpret_cast<uint32_t *>(x.quad(blockIdx.x, e)) = packed;
-        if ((e & 31) == 0) *x.scale(blockIdx.x, e >> 5) = d;
+        *reinterpret_cast<uint32_t *>(x.tile == 0 ? x.row_quad(blockIdx.x, e) : x.tile_quad(blockIdx.x, e)) = packed;
+        if ((e & 31) == 0) *(x.tile == 0 ? x.row_scale(blockIdx.x, e >> 5) : x.tile_scale(blockIdx.x, e >> 5)) = d;
     });
 }
 
@@ -471,11 +469,13 @@ __global__ void __launch_bounds__(kPrefillAttnThreads, HD <= 64 ? 2 : 1) prefill
     __syncthreads();
     for (int b = warp; b < n_tok * (HD / 32); b += kPrefillAttnThreads / 32) {
         const int r = b / (HD / 32), k = b - r * (HD / 32), blk = h * (HD / 32) + k;
-        q8_0_block_warp(qs[r * HD + k * 32 + lane], lane, QuantAt{o.quad(tok0 + r, blk * 32 + (lane & ~3))}, o.scale(tok0 + r, blk));
+        const float v = qs[r * HD + k * 32 + lane];
+        if (o.tile == 0) q8_0_block_warp(v, lane, QuantAt{o.row_quad(tok0 + r, blk * 32 + (lane & ~3))}, o.row_scale(tok0 + r, blk));
+        else q8_0_block_warp(v, lane, QuantAt{o.tile_quad(tok0 + r, blk * 32 + (lane & ~3))}, o.tile_scale(tok0 + r, blk));
     }
     if (o.tile > 0 && h == heads - 1) {         // as in prefill_swiglu_quant_kernel
         const int nb = o.n >> 5, gap = ((nb + 31) & ~31) - nb;
-        for (int i = tid; i < n_tok * gap; i += kPrefillAttnThreads) *o.scale(tok0 + i / gap, nb + i % gap) = 0.0f;
+        for (int i = tid; i < n_tok * gap; i += kPrefillAttnThreads) *o.tile_scale(tok0 + i / gap, nb + i % gap) = 0.0f;
     }
 }
 
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(256) prefill_swiglu_quant_kernel(const float *
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
     if (!live) {        // blocks behind the end of a row: prompt_tc_gemm_kernel multiplies them by a scale of zero
-        if (x.tile > 0 && (ch & 7) == 0) *x.scale(blockIdx.y, ch >> 3) = 0.0f;
+        if (x.tile > 0 && (ch & 7) == 0) *x.tile_scale(blockIdx.y, ch >> 3) = 0.0f;
         return;
     }
     int q[4] = {0, 0, 0, 0};
@@ -510,8 +510,9 @@ __global__ void __launch_bounds__(256) prefill_swiglu_quant_kernel(const float *
         for (int j = 0; j < 4; ++j) q[j] = max(-128, min(127, __float2int_rn(__fmul_rn(v[j], inv))));
     }
     const uint32_t packed = (q[0] & 0xff) | ((q[1] & 0xff) << 8) | ((q[2] & 0xff) << 16) | (static_cast<uint32_t>(q[3]) << 24);
-    *reinterpret_cast<uint32_t *>(x.quad(blockIdx.y, 4 * ch)) = packed;
-    if ((ch & 7) == 0) *x.scale(blockIdx.y, ch >> 3) = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
+    *reinterpret_cast<uint32_t *>(x.tile == 0 ? x.row_quad(blockIdx.y, 4 * ch) : x.tile_quad(blockIdx.y, 4 * ch)) = packed;
+    if ((ch & 7) == 0)
+        *(x.tile == 0 ? x.row_scale(blockIdx.y, ch >> 3) : x.tile_scale(blockIdx.y, ch >> 3)) = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
 }
 
 }  // namespace wd
