@@ -295,7 +295,8 @@ __device__ __forceinline__ float hsum8_lanes(float v) {
 // relative error of the estimate below 2^-21, of a third-order step its cube; the rounded expression itself is off by 2^-52 at most. Both then
 // round to the same float unless a midpoint between two floats lies within those units, which the 29 bits that the conversion drops show (64
 // units are allowed for): then, and outside 2^-100 .. 2^100 (zero, infinity and NaN among them), the expression is evaluated as it stands.
-__device__ __noinline__ float inv_sqrt_as_written(double z) { return __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn(z))); }
+__device__ __forceinline__ float inv_sqrt_as_written(double z) { return __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn(z))); }
+__device__ __noinline__ float inv_sqrt_rare(double z) { return inv_sqrt_as_written(z); }       // out of the way of the code that runs
 __device__ __forceinline__ bool rounds_alike(double v) { return (static_cast<unsigned>(__double2loint(v)) & 0x1fffffffu) - (0x10000000u - 64u) > 128u; }
 __device__ __forceinline__ float inv_sqrt_to_float(double z) {
     const float zf = __double2float_rn(z);
@@ -304,7 +305,7 @@ __device__ __forceinline__ float inv_sqrt_to_float(double z) {
     const double y = static_cast<double>(y0), e = __fma_rn(-__dmul_rn(z, y), y, 1.0);
     const double r = __fma_rn(__dmul_rn(y, e), __fma_rn(e, 0.375, 0.5), y);         // y (1 + e / 2 + 3 e^2 / 8), e = 1 - z y^2
     if (zf >= 0x1p-100f && zf <= 0x1p100f && rounds_alike(r)) return __double2float_rn(r);
-    return inv_sqrt_as_written(z);
+    return inv_sqrt_rare(z);
 }
 
 __device__ __forceinline__ float half_bits_to_float(uint16_t h) { return __half2float(__ushort_as_half(h)); }
