@@ -82,7 +82,6 @@ __global__ void __launch_bounds__(256) prompt_lay_out_kernel(const __grid_consta
 // ---- tensor memory and the tensor core -----------------------------------------------------------------------------------
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // a warp's 32 lanes x N columns, N a multiple of 4; the values are there after tc_wait_ld
 __device__ __forceinline__ void tc_ld4(uint32_t a, uint32_t *v) {
@@ -101,10 +100,11 @@ __device__ __forceinline__ void tc_ld16(uint32_t a, uint32_t *v) {
                  : "r"(a)
                  : "memory");
 }
-// tc_wait_ld, and nothing that uses v is moved in front of it
+// The wait for a read into v, and nothing that uses v is moved in front of it (there is no form without v: the read's own output does not
+// tie its uses to the wait).
 template <int N>
 __device__ __forceinline__ void tc_wait_ld(uint32_t (&v)[N]) {
-    tc_wait_ld();
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < N; ++i) asm volatile("" : "+r"(v[i])::"memory");
 }
@@ -158,6 +158,9 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, unsigned
 
 // warps 0 .. 7 compute, 8 .. 11 expand weights, 12 issues the MMAs, 13 asks for the copies (14 and 15 complete its warpgroup)
 constexpr int kTcWarps = 8, kTcThreads = 512;
+// Registers a thread: two warpgroups that compute take what the two others give back, and no more than the launch's 128 a thread.
+constexpr int kTcRegsMore = 192, kTcRegsLess = 64;
+static_assert(2 * (kTcRegsMore + kTcRegsLess) <= 4 * 128, "more than the block was launched with: the increase would wait for ever");
 template <bool Q8, int TN, int PER>
 struct PromptTc {
     static constexpr int kSub = TN / (kTcWarps / 4), kPairs = kSub / 2;                 // tokens of a warp
@@ -209,7 +212,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
     const int row_tiles = (rows + kTcRows - 1) / kTcRows, tok_tiles = (m_tokens + TN - 1) / TN, n_tiles = row_tiles * tok_tiles;
     const int mine = static_cast<int>(blockIdx.x) < n_tiles ? (n_tiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x) : 0;
     const int total = mine * per_tile;          // stages of this CTA, over all of its tiles
-    if (warp >= 12) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    if (warp >= 12) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcRegsLess));
     if (warp >= 14) {
     } else if (warp == 13) {
         if (lane == 0) {
@@ -264,7 +267,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
             }
         }
     } else if (warp >= kTcWarps) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcRegsLess));
         const int quad = warp & 3;
         const uint32_t lanes = tm + (static_cast<uint32_t>(quad * 32) << 16);
         int slot = 0;
@@ -304,22 +307,24 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
             }
         }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTcRegsMore));
         const int quad = warp & 3, sub = warp >> 2, r = quad * 32 + lane;
         const uint32_t lanes = tm + (static_cast<uint32_t>(quad * 32) << 16);
         int g = 0, slot = 0;
         // One stage: PER blocks of a lane's chain. A block's sums are read in two halves, one of them on its way from tensor memory while the
-        // other is scaled and added to the chains in A.
+        // other is scaled and added to the chains in A. A read's registers hold nothing before its wait, and a compiler may copy registers
+        // where paths meet: between a read and its wait there is no branch, and no read is under way when a stage ends.
         constexpr int kHalf = G::kSub / 2;
         uint32_t v[2][kHalf];
-        // The first half of stage g. Its MMAs were issued by a thread that had seen the stage's copies land, so their completion answers for the
-        // scales in shared memory too.
+        // The first half of stage g; behind the last stage, what nobody uses. Its MMAs were issued by a thread that had seen the stage's copies
+        // land, so their completion answers for the scales in shared memory too.
         auto begin = [&]() {
-            tc_wait(&d_full[g & 1], static_cast<uint32_t>(g >> 1) & 1u, status);
+            if (g < total) tc_wait(&d_full[g & 1], static_cast<uint32_t>(g >> 1) & 1u, status);
             tc_fence_after();
             tc_ld(lanes + G::kColD + (g & 1) * (2 * TN) + sub * G::kSub, v[0]);
         };
-        if (total > 0) begin();
+        begin();
+        tc_wait_ld(v[0]);
         auto stage = [&](auto first, f32x2 (&A)[G::kPairs]) {
             const uint8_t *st = tsm + slot * G::kStage;
             const uint8_t *dwa = st + (G::kW - kTcRows * 4) + r * 4, *dxa = st + PER * G::kW + TN * 32 + sub * G::kSub * 4;
@@ -329,7 +334,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
             for (int c = 0; c < 2 * PER; ++c) {
                 const int h = c >> 1, o = (c & 1) * (kHalf / 2);
                 uint32_t (&u)[kHalf] = v[c & 1];
-                tc_wait_ld(u);
+                if (c > 0) tc_wait_ld(u);
                 if (c + 1 < 2 * PER) {
                     tc_ld(col + ((c + 1) >> 1) * TN + ((c + 1) & 1) * kHalf, v[(c + 1) & 1]);
                 } else {
@@ -337,7 +342,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&d_free[g & 1]);
                     if (++slot == G::kStages) slot = 0;
-                    if (++g < total) begin();
+                    ++g;
+                    begin();
                 }
                 const float dw = *reinterpret_cast<const float *>(dwa + h * G::kW);
                 const ulonglong2 *dx = reinterpret_cast<const ulonglong2 *>(dxa + h * G::kX + o * 8);
@@ -357,6 +363,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
                     }
                 }
             }
+            tc_wait_ld(v[0]);
             __syncwarp();
             if (lane == 0) mbar_arrive(done);
         };
@@ -388,7 +395,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
                 for (; j >> level & 1; ++level) {       // ^4, ^2, ^1
                     tc_wait_st();
                     tc_ld<G::kSub>(lanes + G::kColStack + level * TN + sub * G::kSub, u);
-                    tc_wait_ld();
+                    tc_wait_ld(u);
 #pragma unroll
                     for (int i = 0; i < G::kPairs; ++i) A[i] = add2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), A[i]);
                 }
