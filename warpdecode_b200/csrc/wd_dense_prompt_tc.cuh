@@ -144,16 +144,23 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar) {      // the barrier t
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Bounded wait of this kernel's pipeline: by a count of polls, inline. The warps that compute carry on when one has run out: all of their
-// later waits end after 1,024 polls.
+// Bounded wait of this kernel's pipeline: by a count of polls, inline; a poll suspends the thread for 1.3 us, so that the limit is 1.4 s, or 0.3 ms
+// when another wait of the pass has run out. (These waits stand between the stages of the warps that compute: a limit by the timer takes 2 to 3 %
+// of the kernel, a flag in shared memory or a fence behind the loop 5 to 15.)
 __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, unsigned *status) {
 #pragma unroll 1
     for (unsigned i = 0; i < kSpinLimit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 1023u) == 1023u && *reinterpret_cast<volatile unsigned *>(status) != 0u) break;
+        if ((i & 255u) == 255u && *reinterpret_cast<volatile unsigned *>(status) != 0u) break;
     }
     atomicOr(status, kErrCopyTimeout);
     return false;
+}
+// What is under way ends before the CTA's memory is given back, whether a wait has run out or not.
+__device__ __forceinline__ void tc_drain(uint64_t *bar, uint32_t parity) {
+#pragma unroll 1
+    for (unsigned i = 0; i < kSpinLimit && !mbar_try_wait(bar, parity); ++i) {
+    }
 }
 
 // warps 0 .. 7 compute, 8 .. 11 expand weights, 12 issues the MMAs, 13 asks for the copies (14 and 15 complete its warpgroup)
@@ -173,13 +180,15 @@ struct PromptTc {
     static constexpr uint32_t kIdesc = 2u << 4 | 1u << 7 | 1u << 10 | (TN >> 3) << 17 | (kTcRows >> 4) << 24;
 };
 
-// status[0]: what wd_device.cuh's bounded waits raise; host_status: page-locked, written when it is not zero.
+// status[0]: what the bounded waits raise (y is then undefined); host_status: page-locked, written when it is not zero. When a wait has run out the
+// warps that ask for copies and issue MMAs stop at once, those that expand weights within 32 stages and those that compute at the end of the tile;
+// copies and MMAs under way end before the CTA does. stop_at: the tile of a CTA at which its copies stop as if their wait had run out (tests).
 template <bool Q8, int TN, int PER>
 __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uint8_t *w, int rows, int nb, const uint8_t *x, int m_tokens, float *y,
-                                                                      unsigned *status, unsigned *host_status) {
+                                                                      unsigned *status, unsigned *host_status, int stop_at) {
     using G = PromptTc<Q8, TN, PER>;
     extern __shared__ __align__(1024) uint8_t tsm[];
-    __shared__ __align__(8) uint64_t full[G::kStages], empty[G::kStages], a_full[4], a_free[4], d_full[2], d_free[2], drain;
+    __shared__ __align__(8) uint64_t full[G::kStages], empty[G::kStages], a_full[4], a_free[4], d_full[2], d_free[2];
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);     // the same in every lane, and known to be
     grid_dep_launch();
@@ -196,7 +205,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
             mbar_init(&d_full[lane], 2);        // the MMAs' completion, and the thread that issued them
             mbar_init(&d_free[lane], kTcWarps);
         }
-        if (lane == 0) mbar_init(&drain, 1);
         mbar_fence_init();
     }
     if (warp == 12) {
@@ -220,6 +228,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
             uint32_t par = 1;
             bool ok = true;
             for (int k = 0; k < mine && ok; ++k) {
+                if (k == stop_at) {
+                    atomicOr(status, kErrCopyTimeout);
+                    break;
+                }
                 const int tile = static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
                 const uint8_t *ws = w + static_cast<size_t>(tile % row_tiles) * entries * G::kW, *xs = x + static_cast<size_t>(tile / row_tiles) * entries * G::kX;
                 for (int s = 0; s < per_tile; ++s, ++g) {
@@ -236,8 +248,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
                     }
                 }
             }
-            if (!ok)            // the copies under way land before the CTA's memory is given back
-                for (int i = max(0, g - G::kStages); i < g; ++i) tc_wait(&full[i % G::kStages], static_cast<uint32_t>(i / G::kStages & 1), status);
+            for (int i = max(0, g - G::kStages); i < g; ++i) tc_drain(&full[i % G::kStages], static_cast<uint32_t>(i / G::kStages & 1));
         }
     } else if (warp == 12) {
         if (lane == 0) {
@@ -245,13 +256,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
             uint32_t par = 0;
             const uint64_t desc0 = tc_smem_desc(smem_u32(tsm + PER * G::kW), TN * 16);
             uint64_t desc = desc0;
-            for (int g = 0; g < total; ++g) {
+            int g = 0;
+            for (; g < total; ++g) {
                 if (!(tc_wait(&full[slot], par, status) && tc_wait(&a_full[g & 3], static_cast<uint32_t>(g >> 2) & 1u, status) &&
-                      tc_wait(&d_free[g & 1], (static_cast<uint32_t>(g >> 1) & 1u) ^ 1u, status))) {
-                    tc_commit(&drain);          // what is under way ends before the tensor memory is given back
-                    tc_wait(&drain, 0, status);
+                      tc_wait(&d_free[g & 1], (static_cast<uint32_t>(g >> 1) & 1u) ^ 1u, status)))
                     break;
-                }
                 tc_fence_after();
 #pragma unroll
                 for (int b = 0; b < PER; ++b)
@@ -266,6 +275,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
                     desc = desc0;
                 }
             }
+            for (int i = max(0, g - 2); i < g; ++i) tc_drain(&d_full[i & 1], static_cast<uint32_t>(i >> 1) & 1u);
+            for (int i = max(0, g - 4); i < g; ++i) tc_drain(&a_free[i & 3], static_cast<uint32_t>(i >> 2) & 1u);
         }
     } else if (warp >= kTcWarps) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcRegsLess));
@@ -275,6 +286,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
         uint32_t par = 0;
 #pragma unroll 1
         for (int g = 0; g < total; ++g) {
+            if ((g & 31) == 31 && __any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned *>(status) != 0u)) break;
             tc_wait(&full[slot], par, status);
             const uint8_t *src = tsm + slot * G::kStage + (quad * 32 + lane) * 16;
             uint32_t a[PER][8];
@@ -381,6 +393,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
 #pragma unroll 1
         for (int k = 0; k < mine; ++k) {
             const int tile = static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
+            const unsigned before = *reinterpret_cast<volatile unsigned *>(status);        // looked at behind the tile
 #pragma unroll 1
             for (int j = 0; j < 8; ++j) {
                 f32x2 A[G::kPairs], B[G::kPairs], C[G::kPairs];
@@ -422,6 +435,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prompt_tc_gemm_kernel(const uin
                     }
                 }
             }
+            if (__any_sync(0xffffffffu, before != 0u)) break;
         }
         tc_wait_st();
     }
