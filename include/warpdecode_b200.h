@@ -222,6 +222,9 @@ int wd_dense_decoder_create(const wd_dense_config *cfg, wd_dense_decoder **out);
  * (Qwen2) and q/k head norms (Qwen3) read. Files with partial or scaled rotary embeddings or 2-D tensors of other types
  * are refused by name. The file may be closed afterwards (wd_gguf is declared further down). */
 struct wd_gguf;
+/* Host only: the tokens per tile with which a prompt's product with a [rows][cols] matrix of Q4_0 or Q8_0 blocks runs on tensor cores where its
+ * workspace is there, or 0 for the other kernel (results are the same); tokens: of one pass, n_sm: SMs of the GPU. Negative on error. */
+int wd_prompt_tile(int rows, int cols, int type, int tokens, int n_sm);
 int wd_dense_decoder_load_gguf(const struct wd_gguf *g, int max_ctx, int device, wd_dense_decoder **out);
 /* The configuration a decoder was created with. */
 int wd_dense_decoder_config(const wd_dense_decoder *d, wd_dense_config *cfg);

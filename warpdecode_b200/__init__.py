@@ -561,6 +561,13 @@ def measure_tile_decoder(nsb=8, warps=16, unroll=1, device=0):
     return c.value
 
 
+def prompt_tile(rows, cols, wtype, tokens, n_sm=148):
+    """Tokens per tile of a prompt's product with a matrix on tensor cores, 0 for the other kernel (host only)."""
+    t = lib().wd_prompt_tile(rows, cols, wtype, tokens, n_sm)
+    _check(0 if t >= 0 else t)
+    return t
+
+
 def batch_tasks(hidden, expert_ffn, top_k, n_tokens, max_tokens, wide, n_cta, cta):
     """Descriptions and aux words of one CTA's tile tasks in a batch call (host only)."""
     cap = 4096
