@@ -213,7 +213,9 @@ typedef struct wd_dense_decoder wd_dense_decoder;
 #define WD_DT_Q_NORM 10      /* F32  [head_dim], optional: RMSNorm weight of every q head before the rotary embedding (Qwen3) */
 #define WD_DT_K_NORM 11      /* F32  [head_dim], optional: the same for the k heads */
 /* Allocates the tensors' buffers, the caches, and a workspace for the prompt pass: up to about 100 KB per position at ffn 8192 for up
- * to 512 positions, less or none where that would leave under 64 MiB free (prompts then take more passes, or one-token steps). */
+ * to 512 positions, less or none where that would leave under 64 MiB free (prompts then take more passes, or one-token steps). Where prompts of
+ * up to max_ctx positions can run on tensor cores (wd_prompt_tile), one layer's matrices once more in their order: 5/8 byte per Q4_0 weight, 9/8 per
+ * Q8_0 weight, 38 MB at hidden 2048 and ffn 8192; not where that would be more than a quarter of what is free. */
 int wd_dense_decoder_create(const wd_dense_config *cfg, wd_dense_decoder **out);
 /* Decoder with the geometry and every tensor of a Llama-style Q4_0 model file (architectures llama, qwen2, qwen3), read
  * the way load_model does (src/warodecode.cu:1255-1345): q/k/v and gate/up joined row-wise, an absent output.weight tied
