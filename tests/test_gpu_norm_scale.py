@@ -1,5 +1,6 @@
-"""The layer kernel's RMSNorm scale (inv_sqrt_to_float) over the sizes a residual can have: inside the range of the iteration, at both ends of it and
-outside, where the expression is evaluated as it stands. Bit for bit against the oracle."""
+"""The layer kernel's RMSNorm scale over the sizes a residual can have: inv_sqrt_to_float's step up to mean squares of 2^100 and the expression itself
+above (eps keeps the argument over 1e-6, so the lower end of the step's range is not reached). Bit for bit against the oracle. What its guard lets
+through near the middle between two floats: test_norm_scale_host.py."""
 import numpy as np
 import pytest
 
