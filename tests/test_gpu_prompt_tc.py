@@ -1,8 +1,7 @@
 """The prompt pass's tensor-core product (prompt_tc_gemm_kernel) where it can go wrong, against the oracle's one-token steps, bit for bit.
 
-Each case names the matrices that the rule (wd_prompt_tile) gives to the kernel, with the tokens per tile: token tiles of 32, 48 and 64 with a full, a nearly
-empty and a nearly full last tile, row tiles of 128 with a remainder, rows of one, two, three and more groups of 32 blocks with and without a short last
-group, Q4_0 and Q8_0, prompts of two passes, and a shorter prompt on the same workspace."""
+A model that is wide enough for the rule to pick the kernel: token tiles of 32, 48 and 64 with a full, a nearly empty and a nearly full last tile,
+row tiles of 128 with a remainder, Q4_0 and Q8_0. Which product takes which tile, and the other lengths of rows: test_gpu_prompt_tc_tiles.py."""
 import numpy as np
 import pytest
 
@@ -18,33 +17,12 @@ def wd():
     return w
 
 
-CASES = [
-    # hidden, heads, kv, head_dim, ffn, prompt, q8 (all matrices but the output product's), {matrix: tokens per tile}
-    (1024, 16, 4, 64, 5120, 65, False, {"gate_up": 32}),                    # one group of 32 blocks
-    (1024, 16, 4, 64, 5120, 65, True, {"gate_up": 32}),
-    (1024, 16, 4, 64, 9472, 449, False, {"qkv": 48, "gate_up": 64}),
-    (1024, 16, 4, 64, 9472, 512, True, {"qkv": 48, "gate_up": 64, "down": 32}),     # ten groups, the last one short
-    (1024, 16, 4, 64, 5120, 700, False, {"qkv": 48, "gate_up": 64}),                   # two passes; the second of 188 positions
-    (2048, 32, 8, 64, 2816, 300, False, {"qkv": 64, "wo": 48, "gate_up": 64, "down": 48}),       # three groups, the last one short
-    (2048, 32, 8, 64, 2816, 449, True, {"qkv": 48, "wo": 64, "gate_up": 48, "down": 64}),
-    (2048, 17, 1, 64, 6176, 319, False, {"wo": 48, "gate_up": 64}),         # 34 blocks: two groups, the last one nearly empty
-    (2048, 22, 2, 96, 6176, 300, True, {"qkv": 48, "wo": 48, "gate_up": 64}),      # 66 blocks: three; 193: seven
-    (2048, 32, 8, 64, 8192, 65, False, {"gate_up": 48}),
-    (2048, 32, 8, 64, 8192, 128, True, {"gate_up": 64}),
-    (4096, 11, 1, 96, 3104, 97, False, {"gate_up": 48}),
-]
-
-
-def tiles_of(wd, hidden, heads, kv, head_dim, ffn, prompt, q8):
-    q = wd.TYPE_Q8_0 if q8 else wd.TYPE_Q4_0
-    shapes = {"qkv": ((heads + 2 * kv) * head_dim, hidden, q), "wo": (hidden, heads * head_dim, wd.TYPE_Q4_0), "gate_up": (2 * ffn, hidden, q), "down": (hidden, ffn, q)}
-    return {k: t for k, v in shapes.items() if (t := wd.prompt_tile(*v, min(prompt, 512)))}
-
-
-@pytest.mark.parametrize("hidden,heads,kv,head_dim,ffn,prompt,q8,tiles", CASES)
-def test_prompt_on_tensor_cores(wd, oracle, hidden, heads, kv, head_dim, ffn, prompt, q8, tiles):
+# where the rule picks the kernel: gate/up everywhere
+@pytest.mark.parametrize("hidden,heads,kv,head_dim,ffn,prompt,q8", [
+    (1024, 16, 4, 64, 9472, 449, False), (1024, 16, 4, 64, 9472, 512, True), (2048, 17, 1, 64, 6176, 319, False), (2048, 22, 2, 96, 6176, 300, True),
+    (2048, 32, 8, 64, 8192, 65, False), (2048, 32, 8, 64, 8192, 128, True), (4096, 11, 1, 96, 3104, 97, False)])
+def test_prompt_on_tensor_cores(wd, oracle, hidden, heads, kv, head_dim, ffn, prompt, q8):
     from warpdecode_b200 import synth
-    assert tiles_of(wd, hidden, heads, kv, head_dim, ffn, prompt, q8) == tiles
     vocab, ctx = 96, prompt + 4
     cfg = dict(hidden=hidden, n_heads=heads, n_kv_heads=kv, head_dim=head_dim, ffn=ffn, vocab=vocab, n_layers=1, max_ctx=ctx, rms_eps=1e-5)
     dec = wd.DenseDecoder(hidden, heads, kv, head_dim, ffn, vocab, 1, ctx, 1e-5, 500000.0)
@@ -62,8 +40,4 @@ def test_prompt_on_tensor_cores(wd, oracle, hidden, heads, kv, head_dim, ffn, pr
     logits, hid = dec.read()
     assert np.array_equal(logits.view(np.uint32), ref.logits.view(np.uint32))
     assert np.array_equal(hid.view(np.uint32), ref.hidden.view(np.uint32))
-    short = tokens[:prompt // 2]                # on the caches and the workspace as they are now
-    got, _ = dec.decode(short, 1)
-    assert np.array_equal(got, ref.decode(short, 1))
-    assert np.array_equal(dec.read()[0].view(np.uint32), ref.logits.view(np.uint32))
     dec.close()

@@ -1,7 +1,7 @@
 """Which prompt products run on tensor cores (wd_prompt_tile): the choice holds for products that were measured both ways, and what the rule leaves out."""
 import pytest
 
-import test_gpu_prompt_tc as tc
+import test_gpu_prompt_tc_tiles as tc
 import warpdecode_b200 as wd
 
 Q4, Q8 = wd.TYPE_Q4_0, wd.TYPE_Q8_0
